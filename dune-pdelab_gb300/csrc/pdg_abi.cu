@@ -899,6 +899,8 @@ static void invalidate(pdg_context *ctx, bool operator_changed) {
     ctx->rec_valid = 0;
     ctx->rec64m_valid = 0;
     ctx->rec64mT_valid = 0;
+    ctx->reci_valid = 0;
+    ctx->reciT_valid = 0;
     ctx->recfp_valid = 0;
     ctx->rec32_valid = 0;
     ctx->rec32q_valid = 0;
@@ -1173,7 +1175,8 @@ int pdg_destroy(pdg_context *c) {
                   c->leg64, c->leg32, c->legw64[0], c->legw64[1], c->legw32[0], c->legw32[1],
                   c->fuse_part, c->fuse_cnt, c->Ac64, c->Aqv64, c->Aqf64, c->cq64, c->Ac32,
                   c->Aqv32, c->Aqf32, c->cq32, c->bqv64, c->bqf64, c->Kd64, c->Kd32,
-                  c->recfp, c->tabfp, c->rec32q, c->rec64m, c->rec64mT, c->tabm64};
+                  c->recfp, c->tabfp, c->rec32q, c->rec64m, c->rec64mT, c->tabm64,
+                  c->reci, c->reciT, c->reci_exp, c->reciT_exp};
   for (void *b : bufs)
     if (b) cudaFree(b);
   for (int i = 0; i < 10; i++)

@@ -154,6 +154,9 @@ struct pdg_context {
   int rec64m_valid;
   double *rec64mT;     // 3D: Mhat^-1 A'_dir^T and the transpose's line coefficients
   int rec64mT_valid;
+  int2 *reci, *reciT;  // 3D: limb records of the operator / its transpose and the
+  int *reci_exp, *reciT_exp;   // exponents of each cell's groups (k_apply_i)
+  int reci_valid, reciT_valid;
   double *tabm64;      // 3D: Mhat, Mhat^-1 e0, Mhat^-1 e_{N-1}, Mhat^-1 d0, Mhat^-1 d1, Mhat^-1
   float *rec32;        // the same records rounded to FP32 (3D FP32 operator)
   int rec32_valid;
@@ -375,6 +378,10 @@ int prepare_float_pair(pdg_context *ctx);
 // must be valid
 int launch_apply_m(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<double> &p);
 int prepare_apply_m(pdg_context *ctx, int transpose);
+// the same in 64-bit fixed point (pdg_apply_i.cu); rec64 must be valid
+bool apply_i_usable(const pdg_context *ctx);
+int launch_apply_i(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<double> &p);
+int prepare_apply_i(pdg_context *ctx, int transpose);
 
 // parameter fields beyond A = K I: true when the Gauss-point operator replaces
 // the Kronecker kernels; its launch (diffusion and reaction terms only)

@@ -1,0 +1,109 @@
+"""The 3D FP64 operator in 64-bit fixed point (pdg_apply_i.cu) against the
+oracle: sizes around the block's cell count, every degree, both forms, wide
+ranges of values and coefficients, and data its exponents cannot hold."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+import pdg  # noqa: E402
+import pdg_oracle as O  # noqa: E402
+
+
+def problem(k, n, seed=1, sigma=1.0, scale=1.0, **kw):
+    rng = np.random.default_rng(seed)
+    K = scale * np.exp(sigma * rng.standard_normal(int(np.prod(n))))
+    go = pdg.GridOperator(3, k, n, alpha=3.0, **kw)
+    go.set_permeability(K)
+    return go, O.Problem(3, k, n, alpha=3.0, K=K, **kw), rng
+
+
+def apply(go, x, transpose=False):
+    y = np.zeros(go.ndof)
+    if transpose:
+        go.jacobian_apply_transpose(x, y)
+    else:
+        pdg.OnTheFlyOperator(go).apply(x, y)
+    return y
+
+
+def rel(y, ref):
+    return np.max(np.abs(y - ref)) / np.max(np.abs(ref))
+
+
+# cells per block: 32 (k=1), 14, 8, 5 (k=4); one cell, one less, equal, one
+# more, and cells with all six neighbours
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [(1, 1, 1), (13, 1, 1), (5, 1, 3), (31, 1, 1), (3, 3, 3), (4, 3, 5)])
+def test_sizes(k, n):
+    go, P, rng = problem(k, n, method=pdg.NIPG)
+    x = rng.uniform(-1, 1, go.ndof)
+    # 57-bit operands and one rounding per stage against FP64 sums of the
+    # same length: both within a few units of 1e-15 of the largest entry
+    assert rel(apply(go, x), P.jacobian_apply(x)) <= 1e-14
+    assert rel(apply(go, x, True), P.jacobian_apply_transpose(x)) <= 1e-14
+    go.close()
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+def test_wide_ranges(k):
+    """Values over 12 decades from cell to cell, K over e^+-12: every cell is
+    as accurate as its own terms allow."""
+    go, P, rng = problem(k, (5, 4, 3), sigma=4.0)
+    x = rng.uniform(-1, 1, (go.ncell, go.nbasis)) * 10.0 ** rng.uniform(-6, 6, (go.ncell, 1))
+    y = apply(go, x.ravel()).reshape(go.ncell, -1)
+    ref = P.jacobian_apply(x.ravel()).reshape(go.ncell, -1)
+    # the sum of the magnitudes of a cell's terms: |J| |x| row sums bounded by
+    # the block's largest output for the largest input is what FP64 rounds
+    for e in range(go.ncell):
+        assert np.max(np.abs(y[e] - ref[e])) <= 1e-12 * np.max(np.abs(ref[e])), e
+    go.close()
+
+
+@pytest.mark.parametrize("factor", [1e-290, 1e-200, 1e200, 1e290])
+def test_ends_of_the_range(factor):
+    go, P, rng = problem(2, (4, 3, 2))
+    x = rng.uniform(-1, 1, go.ndof)
+    ref = P.jacobian_apply(x)
+    assert rel(apply(go, x * factor) / factor, ref) <= 1e-12
+    go.close()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_non_finite(value):
+    n = (7, 4, 3)
+    go, P, rng = problem(2, n)
+    x = rng.uniform(-1, 1, go.ndof)
+    ref = P.jacobian_apply(x).reshape(go.ncell, -1)
+    e = 2 + 7 * (1 + 4 * 1)
+    x[e * go.nbasis:(e + 1) * go.nbasis] = value
+    y = apply(go, x).reshape(go.ncell, -1)
+    hit = {e, e - 1, e + 1, e - 7, e + 7, e - 28, e + 28}
+    for c in range(go.ncell):
+        if c in hit:
+            assert not np.isfinite(y[c]).any()
+        else:
+            assert np.max(np.abs(y[c] - ref[c])) <= 1e-12 * np.max(np.abs(ref))
+    go.close()
+
+
+def test_zeros_and_one_cell():
+    """Zero vectors give zeros; a single non-zero cell reaches itself and its
+    neighbours only."""
+    n = (4, 4, 4)
+    go, P, rng = problem(3, n)
+    assert not apply(go, np.zeros(go.ndof)).any()
+    x = np.zeros((go.ncell, go.nbasis))
+    x[21] = rng.uniform(-1, 1, go.nbasis)
+    assert rel(apply(go, x.ravel()), P.jacobian_apply(x.ravel())) <= 1e-14
+    y = apply(go, x.ravel()).reshape(go.ncell, -1)
+    assert {int(c) for c in np.nonzero(np.abs(y).max(1))[0]} == {21, 20, 22, 17, 25, 5, 37}
+    go.close()
+
+
+def test_extreme_coefficients():
+    """K beyond the exponents of the limb records: the FP64 evaluation."""
+    go, P, rng = problem(2, (3, 3, 2), scale=1e60)
+    x = rng.uniform(-1, 1, go.ndof)
+    assert rel(apply(go, x), P.jacobian_apply(x)) <= 1e-12
+    go.close()
