@@ -37,8 +37,12 @@ struct ICfg {
   static constexpr int RECW = 3 * N2 + 2 * NW;       // the FP64 record (both forms)
   static constexpr int RECI = 3 * N2 + NW;           // limb pairs of one form
   static constexpr int NEXP = 16;                    // exponents per cell, see k_record_i
-  // ue, X, Y, Z, face data (12 TPC), record; 8 bytes each
-  static constexpr int PER_CELL = 4 * NB + 12 * TPC + RECI + (N == 3 ? 2 : N == 5 ? 1 : 0);
+  // ue, X, Y, Z, face data (12 TPC), record; 8 bytes each.  The padding is the
+  // one with the fewest shared-memory wavefronts of the kernel's accesses,
+  // counted on the CPU over paddings 0..15 (k = 4: 2352 per block instead of
+  // 3128 without the right one)
+  static constexpr int PER_CELL =
+      4 * NB + 12 * TPC + RECI + (N == 2 ? 6 : N == 3 ? 1 : N == 5 ? 10 : 0);
   static constexpr int LN = N == 2 ? 1 : N == 5 ? 3 : 2;              // ceil log2 N
   static constexpr int LD = N == 2 ? 0 : N == 3 ? 2 : N == 4 ? 5 : 6;  // ceil log2 max |d|
   // X, Y, Z are formed below 2^61 and shifted to 2^(61 - SHX) so that the
@@ -215,8 +219,10 @@ __device__ __noinline__ void apply_cells_fp64(const OpParams<double> &p,
   }
 }
 
+// Five and six blocks per SM at k = 4 and 3 instead of the four the register
+// count alone would give: 33x29x37 Q4 183 -> 167 us.
 template <int N>
-__global__ void __launch_bounds__(ICfg<N>::THREADS)
+__global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : 6)
     k_apply_i(const __grid_constant__ OpParams<double> p,
               const __grid_constant__ ApplyArgs<double> a, const int2 *__restrict__ rec,
               const int *__restrict__ exps, const double *__restrict__ rec64) {
@@ -323,8 +329,12 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS)
   const int ebx = Ex == kFixZero ? kFixMinBiased : Ex + 1022;
 
   // ---- own column to limbs; neighbour face data, aligned to the cell ----
+  int2 uc[N], zf[4];   // own column; the z faces' data is read by this thread only
 #pragma unroll
-  for (int z = 0; z < N; z++) ue[z * TPC + l] = fix_limbs(col[z], ebx);
+  for (int z = 0; z < N; z++) {
+    uc[z] = fix_limbs(col[z], ebx);
+    ue[z * TPC + l] = uc[z];
+  }
 #pragma unroll
   for (int f = 0; f < NF; f++) {
     const int2 *w = Am + 3 * N2 + f * (N + 1);
@@ -339,8 +349,13 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS)
     const bool on = nbr[f] >= 0;
     const long long s1 = on ? mac2_value(hh, mid, Etot - eu - ex[1 + f] - 2) : 0;
     const long long s2 = on ? mac2_value(h2, m2, Etot - eu - ex[7 + f] - 2) : 0;
-    fa[(2 * f) * TPC + l] = split32(s1);
-    fa[(2 * f + 1) * TPC + l] = split32(s2);
+    if (f < 4) {
+      fa[(2 * f) * TPC + l] = split32(s1);
+      fa[(2 * f + 1) * TPC + l] = split32(s2);
+    } else {
+      zf[2 * (f - 4)] = split32(s1);
+      zf[2 * (f - 4) + 1] = split32(s2);
+    }
   }
   if (__syncthreads_or(bad)) {
     apply_cells_fp64<N>(p, a, rec64, reinterpret_cast<double *>(ue), l, ee, nbr, active);
@@ -352,16 +367,13 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS)
   const int shu = Etot - Ex - EA - 2;
   constexpr long long kHalfX = C::SHX ? 1ll << (C::SHX > 0 ? C::SHX - 1 : 0) : 0;
   {
-    int2 Ax[N], Ay[N], uc[N];
+    int2 Ax[N], Ay[N];
 #pragma unroll
     for (int q = 0; q < N; q++) {
       Ax[q] = Am[tx * N + q];
       Ay[q] = Am[N2 + ty * N + q];
-      uc[q] = ue[q * N2 + l];
     }
     const int d0x = sd0[tx], d1x = sd1[tx], d0y = sd0[ty], d1y = sd1[ty];
-    const int2 zf0 = fa[8 * TPC + l], zf1 = fa[9 * TPC + l];
-    const int2 zf2 = fa[10 * TPC + l], zf3 = fa[11 * TPC + l];
 #pragma unroll
     for (int z = 0; z < N; z++) {
       const int lx = z * N + ty, ly = z * N + tx;
@@ -392,10 +404,10 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS)
 #pragma unroll
         for (int q = 0; q < N; q++) mac2(hh, mid, Am[2 * N2 + z * N + q], uc[q]);
         SmallSum<false> s(mac2_value(hh, mid, shu) + kHalfX);
-        if (z == 0) s.add(zf0, 1);
-        s.add(zf1, int_d0<N>(z));
-        if (z == N - 1) s.add(zf2, 1);
-        s.add(zf3, int_d1<N>(z));
+        if (z == 0) s.add(zf[0], 1);
+        s.add(zf[1], int_d0<N>(z));
+        if (z == N - 1) s.add(zf[2], 1);
+        s.add(zf[3], int_d1<N>(z));
         Zs[z * N2 + l] = split32(s.template shifted<C::SHX>());
       }
     }
