@@ -1128,6 +1128,30 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
     if (cudaMalloc(&c->tabm64, sizeof(double) * tm.size()) != cudaSuccess)
       return fail(set_error(PDG_ECUDA, "device allocation failed"));
     cudaMemcpy(c->tabm64, tm.data(), sizeof(double) * tm.size(), cudaMemcpyHostToDevice);
+    // the per-cell tensor operator's tables: M, the nodal differentiation
+    // matrix Dn, L = M^-1 Dn^T M = m_1 e_{N-1}^T - m_0 e_0^T - Dn (integration
+    // by parts), m_0, m_1 and the derivatives of the basis at the ends
+    std::vector<double> tt(3 * N * N + 4 * N);
+    const double *m0 = tm.data() + N * N, *m1 = m0 + N;
+    for (int i = 0; i < N; i++) {
+      for (int q = 0; q < N; q++) {
+        const double dn = ndlag(c, q, c->nodes[i]);
+        tt[i * N + q] = tab[i * N + q];
+        tt[N * N + i * N + q] = dn;
+        tt[2 * N * N + i * N + q] =
+            (q == N - 1 ? m1[i] : 0.0) - (q == 0 ? m0[i] : 0.0) - dn;
+      }
+      tt[3 * N * N + i] = m0[i];
+      tt[3 * N * N + N + i] = m1[i];
+      tt[3 * N * N + 2 * N + i] = t.d0[i];
+      tt[3 * N * N + 3 * N + i] = t.d1[i];
+    }
+    const std::vector<float> tt32(tt.begin(), tt.end());
+    if (cudaMalloc(&c->tabt64, sizeof(double) * tt.size()) != cudaSuccess ||
+        cudaMalloc(&c->tabt32, sizeof(float) * tt.size()) != cudaSuccess)
+      return fail(set_error(PDG_ECUDA, "device allocation failed"));
+    cudaMemcpy(c->tabt64, tt.data(), sizeof(double) * tt.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(c->tabt32, tt32.data(), sizeof(float) * tt.size(), cudaMemcpyHostToDevice);
   }
   cudaMemcpy(c->tab32, tab32.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(c->K64, ones.data(), sizeof(double) * c->ncell, cudaMemcpyHostToDevice);
@@ -1176,7 +1200,7 @@ int pdg_destroy(pdg_context *c) {
                   c->fuse_part, c->fuse_cnt, c->Ac64, c->Aqv64, c->Aqf64, c->cq64, c->Ac32,
                   c->Aqv32, c->Aqf32, c->cq32, c->bqv64, c->bqf64, c->Kd64, c->Kd32,
                   c->recfp, c->tabfp, c->rec32q, c->rec64m, c->rec64mT, c->tabm64,
-                  c->reci, c->reciT, c->reci_exp, c->reciT_exp};
+                  c->tabt64, c->tabt32, c->reci, c->reciT, c->reci_exp, c->reciT_exp};
   for (void *b : bufs)
     if (b) cudaFree(b);
   for (int i = 0; i < 10; i++)

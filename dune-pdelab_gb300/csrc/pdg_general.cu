@@ -827,6 +827,8 @@ int launch_apply_general(pdg_context *ctx, const ApplyArgs<T> &a) {
   const T *c = dbl ? (const T *)ctx->c64 : (const T *)ctx->c32;
   const T *tab = dbl ? (const T *)ctx->tab64 : (const T *)ctx->tab32;
   OpParams<T> p = make_params<T>(ctx, K, c, tab);
+  // a tensor per cell keeps every integrand polynomial: no Gauss points needed
+  if (ctx->dim == 3 && ctx->gen_A == 1 && !ctx->cq64) return launch_apply_tensor<T>(ctx, a, p);
   GenCoef<T> g{};
   if (ctx->gen_A == 1 || ctx->gen_A == 3) g.Ac = dbl ? (const T *)ctx->Ac64 : (const T *)ctx->Ac32;
   if (ctx->gen_A == 2) {

@@ -158,6 +158,8 @@ struct pdg_context {
   int *reci_exp, *reciT_exp;   // exponents of each cell's groups (k_apply_i)
   int reci_valid, reciT_valid;
   double *tabm64;      // 3D: Mhat, Mhat^-1 e0, Mhat^-1 e_{N-1}, Mhat^-1 d0, Mhat^-1 d1, Mhat^-1
+  double *tabt64;      // 3D: M, Dn, L = M^-1 Dn^T M, M^-1 e0, M^-1 e_{N-1}, d0, d1 of the
+  float *tabt32;       // per-cell tensor operator (pdg_tensor.cu)
   float *rec32;        // the same records rounded to FP32 (3D FP32 operator)
   int rec32_valid;
   float *rec32q;       // Q3: the FP32 records padded to 84 floats, couplings of
@@ -388,6 +390,10 @@ int prepare_apply_i(pdg_context *ctx, int transpose);
 bool general_coefficients(const pdg_context *ctx);
 template <typename T>
 int launch_apply_general(pdg_context *ctx, const ApplyArgs<T> &a);
+// a tensor per cell and at most a reaction per cell in 3D: evaluated on the
+// nodes (pdg_tensor.cu)
+template <typename T>
+int launch_apply_tensor(pdg_context *ctx, const ApplyArgs<T> &a, const OpParams<T> &p);
 // R(0)'s Dirichlet-data diffusion terms with the tensor (added to ctx->r0)
 int launch_rhs_general(pdg_context *ctx);
 // the face lattice (every face once: x-normal faces, then y, then z; planes
