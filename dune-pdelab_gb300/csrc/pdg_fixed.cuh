@@ -72,14 +72,15 @@ struct BlockExp {
   __device__ __forceinline__ int exponent() const { return any ? biased() - 1022 : kFixZero; }
 };
 
-// magnitude of x in units of 2^(E - 57), E = eb - 1022, truncated (x finite,
+// magnitude of x in units of 2^(E - F), E = eb - 1022, truncated (x finite,
 // biased exponent at most eb; zeros and subnormals give 0, since eb >= 64)
+template <int F = kFixBits>
 __device__ __forceinline__ unsigned long long fix_mag(double x, int eb) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const int sh = min(eb - (int)((hi >> 20) & 0x7ffu), 63);
   const unsigned mh = (hi & 0xfffffu) | 0x100000u;
   const unsigned long long t =
-      ((unsigned long long)__funnelshift_l(lo, mh, 4) << 32) | (unsigned)(lo << 4);
+      ((unsigned long long)__funnelshift_l(lo, mh, F - 53) << 32) | (unsigned)(lo << (F - 53));
   return t >> sh;
 }
 __device__ __forceinline__ long long fix_signed(double x, int eb) {
@@ -91,8 +92,9 @@ __device__ __forceinline__ int2 limbs(long long X) {
   const int h = (int)((X + (1ll << 28)) >> 29);
   return make_int2(h, (int)((unsigned)X - ((unsigned)h << 29)));
 }
+template <int F = kFixBits>
 __device__ __forceinline__ int2 fix_limbs(double x, int eb) {
-  const int2 r = limbs((long long)fix_mag(x, eb));
+  const int2 r = limbs((long long)fix_mag<F>(x, eb));
   const int s = __double2hiint(x) >> 31;
   return make_int2((r.x ^ s) - s, (r.y ^ s) - s);
 }
@@ -103,10 +105,18 @@ __device__ __forceinline__ void mac2(long long &hh, long long &mid, int2 a, int2
   mid += (long long)a.x * b.y;
   mid += (long long)a.y * b.x;
 }
-// the contraction in units of 2^(Ea + Eb - 59), shifted right by sh
+// One of the operands may have kFixWide = 59 bits (|h| <= 2^30): the sums of
+// five such products stay below 2^62.
+constexpr int kFixWide = 59;
+// the contraction of 57-bit operands in units of 2^(Ea + Eb - 59), shifted right by sh
 // (at most 63)
 __device__ __forceinline__ long long mac2_value(long long hh, long long mid, int sh) {
   return ((hh << 3) + (mid >> 26)) >> (int)min((unsigned)sh, 63u);
+}
+
+// the contraction of a 59-bit with a 57-bit operand in units of 2^(Ea + Eb - 59)
+__device__ __forceinline__ long long mac2_value_wide(long long hh, long long mid) {
+  return (hh << 1) + (mid >> 28);
 }
 
 // a 64-bit integer as v = y 2^32 + x with signed 32-bit x and y

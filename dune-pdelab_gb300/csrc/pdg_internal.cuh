@@ -121,6 +121,8 @@ struct PrecData {
   void *inv16;     // FP16 dense inverses (dense_fp16), scaled by invscale [ncell]
   float *invscale;
   double *Lsum_inv;  // FP64 FDM: 1 / (sum of the directions' eigenvalues) per DOF [ncell][N^d]
+  int2 *Qi;        // 3D FP64 FDM: limbs of the scaled Q [ncell][3 N*N] and the exponents of
+  int *Qi_exp;     // each cell (pdg_fdm_i.cu, which also scales Lsum_inv)
 };
 
 }  // namespace pdg
@@ -310,6 +312,11 @@ void prec_free(pdg_context *ctx, int precision);
 template <typename T>
 int block_solve(pdg_context *ctx, const T *d, T *v, int transpose, const int *skip,
                 const int *cells, int ncells, T scale);
+// FP64 FDM block Jacobi on 3D grids in 64-bit fixed point (pdg_fdm_i.cu): its
+// records from Q and Lsum_inv, and v = scale D^-1 d on a cell list (or all)
+int fdm_record_i(pdg_context *ctx);
+int fdm_apply_i(pdg_context *ctx, const double *d, double *v, const int *skip, const int *cells,
+                int ncells, double scale);
 int diag_blocks(pdg_context *ctx, double **D);   // row-major FP64 diagonal blocks
 int bj_iterative_setup(pdg_context *ctx, int precision);
 template <typename T>

@@ -1066,6 +1066,13 @@ static int fdm_setup(pdg_context *ctx, int precision) {
     k_fdm_lsum_inv<<<b2, 256, 0, ctx->stream>>>(ctx->ndof, dim, N, (const double *)pd.L,
                                                    pd.Lsum_inv);
     PDG_CUDA_TRY(cudaGetLastError());
+    if (dim == 3) {
+      const int st = fdm_record_i(ctx);
+      if (st != PDG_OK) {
+        cudaFree(dLi);
+        return st;
+      }
+    }
   }
   PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   cudaFree(dLi);
@@ -1161,6 +1168,8 @@ void prec_free(pdg_context *ctx, int precision) {
   if (pd.inv16) cudaFree(pd.inv16);
   if (pd.invscale) cudaFree(pd.invscale);
   if (pd.Lsum_inv) cudaFree(pd.Lsum_inv);
+  if (pd.Qi) cudaFree(pd.Qi);
+  if (pd.Qi_exp) cudaFree(pd.Qi_exp);
   pd = PrecData{0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
 }
 
@@ -1285,12 +1294,20 @@ static int fdm_dispatch(pdg_context *ctx, const T *d, T *v, const int *skip, con
     case 22: return fdm_apply_dn<T, 2, 3>(ctx, d, v, skip, cells, ncells, scale);
     case 23: return fdm_apply_dn<T, 2, 4>(ctx, d, v, skip, cells, ncells, scale);
     case 24: return fdm_apply_dn<T, 2, 5>(ctx, d, v, skip, cells, ncells, scale);
-    case 31: return fdm_apply_dn<T, 3, 2>(ctx, d, v, skip, cells, ncells, scale);
-    case 32: return fdm_apply_dn<T, 3, 3>(ctx, d, v, skip, cells, ncells, scale);
-    case 33: return fdm_apply_dn<T, 3, 4>(ctx, d, v, skip, cells, ncells, scale);
-    case 34: return fdm_apply_dn<T, 3, 5>(ctx, d, v, skip, cells, ncells, scale);
-    default: return set_error(PDG_EUNSUPPORTED, "dim/degree not compiled in");
+    default: break;
   }
+  if constexpr (std::is_same<T, double>::value) {
+    if (ctx->dim == 3) return fdm_apply_i(ctx, d, v, skip, cells, ncells, scale);
+  } else {
+    switch (ctx->dim * 10 + ctx->k) {
+      case 31: return fdm_apply_dn<T, 3, 2>(ctx, d, v, skip, cells, ncells, scale);
+      case 32: return fdm_apply_dn<T, 3, 3>(ctx, d, v, skip, cells, ncells, scale);
+      case 33: return fdm_apply_dn<T, 3, 4>(ctx, d, v, skip, cells, ncells, scale);
+      case 34: return fdm_apply_dn<T, 3, 5>(ctx, d, v, skip, cells, ncells, scale);
+      default: break;
+    }
+  }
+  return set_error(PDG_EUNSUPPORTED, "dim/degree not compiled in");
 }
 
 template <typename T>

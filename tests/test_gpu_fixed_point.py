@@ -107,3 +107,52 @@ def test_extreme_coefficients():
     x = rng.uniform(-1, 1, go.ndof)
     assert rel(apply(go, x), P.jacobian_apply(x)) <= 1e-12
     go.close()
+
+
+def block_residual(P, nb, e, v, d):
+    """|D_e v_e - d_e| / |d_e| with the oracle's operator on one cell."""
+    s = slice(e * nb, (e + 1) * nb)
+    one = np.zeros(v.size)
+    one[s] = v[s]
+    return rel(P.jacobian_apply(one)[s], d[s])
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [(1, 1, 1), (13, 1, 1), (5, 1, 3), (31, 1, 1), (4, 3, 5)])
+def test_fdm_sizes(k, n):
+    go, P, rng = problem(k, n, sigma=2.0)
+    d = rng.uniform(-1, 1, (go.ncell, go.nbasis)) * 10.0 ** rng.uniform(-6, 6, (go.ncell, 1))
+    d = d.ravel()
+    v = np.zeros(go.ndof)
+    pr = pdg.GridOperatorPreconditioner(go)
+    pr.pre()
+    pr.apply(v, d)
+    # the blocks' condition numbers reach 1e3 (k = 4): 1e3 roundings of 1e-16
+    for e in range(go.ncell):
+        assert block_residual(P, go.nbasis, e, v, d) <= 1e-11
+    go.close()
+
+
+def test_fdm_extremes():
+    """Infinities stay in their cell; zeros give zeros; values near the ends
+    of the range."""
+    go, P, rng = problem(2, (7, 4, 3))
+    pr = pdg.GridOperatorPreconditioner(go)
+    pr.pre()
+    d = rng.uniform(-1, 1, go.ndof)
+    ref = np.zeros(go.ndof)
+    pr.apply(ref, d)
+    v = np.zeros(go.ndof)
+    pr.apply(v, np.zeros(go.ndof))
+    assert not v.any()
+    for f in (1e-280, 1e270):
+        pr.apply(v, d * f)
+        assert rel(v / f, ref) <= 1e-13
+    bad = d.copy()
+    bad[9 * go.nbasis:10 * go.nbasis] = np.nan
+    pr.apply(v, bad)
+    hit = np.zeros(go.ndof, bool)
+    hit[9 * go.nbasis:10 * go.nbasis] = True
+    assert np.isnan(v[hit]).all()
+    assert np.max(np.abs(v[~hit] - ref[~hit])) <= 1e-13 * np.max(np.abs(ref))
+    go.close()
