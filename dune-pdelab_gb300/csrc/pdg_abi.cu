@@ -904,6 +904,7 @@ static void invalidate(pdg_context *ctx, bool operator_changed) {
     ctx->recfp_valid = 0;
     ctx->rec32_valid = 0;
     ctx->rec32q_valid = 0;
+    ctx->rec32c_valid = 0;
     ctx->A_valid = 0;
     ctx->prec[0].ready = 0;
     ctx->prec[1].ready = 0;
@@ -1068,6 +1069,7 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
     tab[2 * N * N + a] = t.d0[a];
     tab[2 * N * N + N + a] = t.d1[a];
   }
+  std::copy(tab.begin(), tab.end(), c->tab_host);
   std::vector<float> tab32(tab.begin(), tab.end());
   std::vector<double> ones(c->ncell, 1.0);
   std::vector<float> ones32(c->ncell, 1.0f);
@@ -1199,7 +1201,7 @@ int pdg_destroy(pdg_context *c) {
                   c->leg64, c->leg32, c->legw64[0], c->legw64[1], c->legw32[0], c->legw32[1],
                   c->fuse_part, c->fuse_cnt, c->Ac64, c->Aqv64, c->Aqf64, c->cq64, c->Ac32,
                   c->Aqv32, c->Aqf32, c->cq32, c->bqv64, c->bqf64, c->Kd64, c->Kd32,
-                  c->recfp, c->tabfp, c->rec32q, c->rec64m, c->rec64mT, c->tabm64,
+                  c->recfp, c->tabfp, c->rec32q, c->rec32c, c->rec64m, c->rec64mT, c->tabm64,
                   c->tabt64, c->tabt32, c->reci, c->reciT, c->reci_exp, c->reciT_exp};
   for (void *b : bufs)
     if (b) cudaFree(b);

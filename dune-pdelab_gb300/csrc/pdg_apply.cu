@@ -642,11 +642,10 @@ int launch_apply(pdg_context *ctx, const ApplyArgs<T> &a, const T *K, const T *c
   }
   OpParams<T> p = make_params<T>(ctx, K, c, tab);
   if constexpr (std::is_same<T, float>::value) {
-    // the staged kernels (plane per thread) win for N <= 4: Q1, Q2 (78 vs
-    // 126 us at 64^3 Q2) and the Q3 variant with swizzled 16-byte rows; at
-    // N = 5 the generic kernel is used
+    // degrees 1 and 2: one cell per thread; degree 3: the staged kernel with
+    // swizzled 16-byte rows; degree 4: the generic kernel
     if (ctx->dim == 3 && ctx->N <= 4 && !a.cells && a.ncells == 0 && K == ctx->K32) {
-      PDG_TRY(ensure_record32(ctx));
+      if (ctx->N == 4) PDG_TRY(ensure_record32(ctx));
       PDG_TRY(launch_apply32_3d(ctx, a, p, ctx->rec32));
       if (convection_on(ctx)) PDG_TRY(launch_convection<T>(ctx, a));
       return nl_apply<T>(ctx, a);

@@ -144,6 +144,7 @@ struct pdg_context {
   float *c32;
   double *tab64;
   float *tab32;
+  double tab_host[2 * pdg::kMaxN1 * pdg::kMaxN1 + 2 * pdg::kMaxN1];   // tab64 on the host
   pdg::Velocity vel;
 
   // source and boundary data on the device
@@ -164,6 +165,8 @@ struct pdg_context {
   float *tabt32;       // per-cell tensor operator (pdg_tensor.cu)
   float *rec32;        // the same records rounded to FP32 (3D FP32 operator)
   int rec32_valid;
+  float *rec32c;       // degrees 1, 2: face coefficients per cell (k_apply32_cell)
+  int rec32c_valid;
   float *rec32q;       // Q3: the FP32 records padded to 84 floats, couplings of
   int rec32q_valid;    // faces without a neighbour zeroed (k_apply32_q3t)
   // parameter fields beyond A = K I (pdg_set_permeability_tensor / _points,
@@ -295,6 +298,10 @@ int basis_change(pdg_context *ctx, int which, int transpose, const T *in, T *out
 // 3D FP32 operator with staged neighbour runs (all cells, coupled or diag_only)
 int launch_apply32_3d(pdg_context *ctx, const ApplyArgs<float> &a, const OpParams<float> &p,
                       const float *rec);
+// the same for degrees 1 and 2, one cell per thread (pdg_cell32.cu), and the
+// FP32 FDM block Jacobi of these degrees on all cells
+int launch_apply32_cell(pdg_context *ctx, const ApplyArgs<float> &a, const OpParams<float> &p);
+int fdm32_cell(pdg_context *ctx, const float *d, float *v, const int *skip, float scale);
 int launch_grad_logK(pdg_context *ctx, const double *u, const double *lam, double *g);
 int launch_grad_source(pdg_context *ctx, const double *lam, double *g);
 

@@ -1252,6 +1252,8 @@ static int fdm_apply_dn(pdg_context *ctx, const T *d, T *v, const int *skip, con
       return PDG_OK;
     }
   }
+  if constexpr (std::is_same<T, float>::value && D == 3 && N <= 3)
+    if (!cells) return fdm32_cell(ctx, d, v, skip, scale);
   using C = PCfg<D, N>;
   const size_t smem = sizeof(T) * C::CPB * (C::PER_CELL + fdm_pad<T, D, N>());
   const long work = cells ? ncells : ctx->ncell;

@@ -199,13 +199,12 @@ __device__ __forceinline__ void block_sum2_sel(double &a, double &b, double *scr
 // group, zero between launches (each group's last block resets its own).
 constexpr int kFuseGroup = 256;
 
+// (s0, s1): the block's sums, in thread 0
 template <int MAXT, bool kScratch = false>
-__device__ __forceinline__ void reduce_tail_grouped(double *part, long max_blocks, int *cnt,
-                                                    const RedCtx &rc, double s0, double s1,
-                                                    int fin, int slot0, int slot1,
-                                                    double *scratch = nullptr) {
+__device__ __forceinline__ void grouped_finish(double *part, long max_blocks, int *cnt,
+                                               const RedCtx &rc, double s0, double s1, int fin,
+                                               int slot0, int slot1, double *scratch = nullptr) {
   __shared__ bool last;
-  block_sum2_sel<MAXT, kScratch>(s0, s1, scratch);
   const int b = (int)blockIdx.x, g = b / kFuseGroup;
   const int ngroups = (int)((gridDim.x + kFuseGroup - 1) / kFuseGroup);
   const int gsize = min(kFuseGroup, (int)gridDim.x - g * kFuseGroup);
@@ -246,6 +245,64 @@ __device__ __forceinline__ void reduce_tail_grouped(double *part, long max_block
     run_finisher(rc, fin, slot0, slot1, a, c);
     rc.flags[F_COUNTER] = 0;
   }
+}
+
+template <int MAXT, bool kScratch = false>
+__device__ __forceinline__ void reduce_tail_grouped(double *part, long max_blocks, int *cnt,
+                                                    const RedCtx &rc, double s0, double s1,
+                                                    int fin, int slot0, int slot1,
+                                                    double *scratch = nullptr) {
+  block_sum2_sel<MAXT, kScratch>(s0, s1, scratch);
+  grouped_finish<MAXT, kScratch>(part, max_blocks, cnt, rc, s0, s1, fin, slot0, slot1, scratch);
+}
+
+// A sum carried as an unevaluated pair of floats (48 bits): block sums of FP32
+// kernels on the FP32 pipe.  GB300's FP64 pipe takes 17 cycles for one
+// warp-wide addition, a block sum in FP64 about 18 of them.
+struct TwoFloat {
+  float h, l;
+};
+__device__ __forceinline__ TwoFloat two_add(TwoFloat a, TwoFloat b) {
+  const float s = __fadd_rn(a.h, b.h), t = __fsub_rn(s, a.h);
+  const float e = __fadd_rn(__fadd_rn(__fsub_rn(a.h, __fsub_rn(s, t)), __fsub_rn(b.h, t)),
+                            __fadd_rn(a.l, b.l));
+  const float h = __fadd_rn(s, e);
+  // a sum that is not finite stays what it is
+  return TwoFloat{h, isfinite(h) ? __fsub_rn(e, __fsub_rn(h, s)) : 0.f};
+}
+__device__ __forceinline__ TwoFloat warp_sum_two(TwoFloat v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const TwoFloat w{__shfl_down_sync(0xffffffffu, v.h, o), __shfl_down_sync(0xffffffffu, v.l, o)};
+    v = two_add(v, w);
+  }
+  return v;
+}
+// reduce_tail_grouped with two-float sums of each thread (blocks of T threads,
+// T a multiple of 32)
+template <int T>
+__device__ __forceinline__ void reduce_tail_two_float(double *part, long max_blocks, int *cnt,
+                                                      const RedCtx &rc, TwoFloat s0, TwoFloat s1,
+                                                      int fin) {
+  __shared__ TwoFloat w0[T / 32], w1[T / 32];
+  s0 = warp_sum_two(s0);
+  s1 = warp_sum_two(s1);
+  if ((threadIdx.x & 31) == 0) {
+    w0[threadIdx.x >> 5] = s0;
+    w1[threadIdx.x >> 5] = s1;
+  }
+  __syncthreads();
+  double a = 0.0, c = 0.0;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 1; i < T / 32; i++) {
+      s0 = two_add(s0, w0[i]);
+      s1 = two_add(s1, w1[i]);
+    }
+    a = (double)s0.h + (double)s0.l;
+    c = (double)s1.h + (double)s1.l;
+  }
+  grouped_finish<T>(part, max_blocks, cnt, rc, a, c, fin, -1, -1);
 }
 
 int red_dot(pdg_context *ctx, const RedCtx &rc, long n, const double *a, const double *b,
