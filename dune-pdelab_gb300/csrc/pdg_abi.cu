@@ -370,7 +370,6 @@ static int cg_device(pdg_context *ctx, T *x, T *b, T *p, T *q, double reduction,
   if (fuse) PDG_TRY(ensure_fuse(ctx));
   // one iteration's launches (the iteration count advances on the device)
   auto body = [&]() -> int {
-    PDG_TRY(inc_iter(ctx, rc, 1.0));
     if (fuse) {
       // q = A p with lambda = rholast / <p, q> in the same launch
       ctx->fuse_fin = FIN_CG_LAMBDA;

@@ -16,8 +16,12 @@
 // term, and {kappa_e, kappa_o, penalty} of each face) instead of the assembled
 // 1D matrices A'_dir (57 at degree 2): with the shape matrices as constants
 // the self terms of a face share the jump and the normal derivatives with its
-// neighbour terms.  What bounds them is HBM: 64^3 Q2, 7.1M DOF, 57 MB of
-// vectors and 24 MB of coefficients are 12 us.
+// neighbour terms.  64^3 Q2 (7.1M DOF) takes 47 us for the operator and 38 us for
+// the block Jacobi with the residual update (plane-per-thread kernels with
+// exchanges: 81 and 68 us); the bytes need 12 and 22 us.  What is left is the
+// latency of load, compute and store within a block at 10 and 18 warps per SM.
+// 64 threads per block: 32 and 128 are slower on large or small grids (64^3
+// mixed CG 252, 252 and 281 ms, 32^3 gradient 69, 80 and 69 ms).
 //
 // Block sums of the fused dot products are formed in two-float arithmetic
 // (the FP64 pipe takes 17 cycles for one warp-wide addition, and a block sum
@@ -26,6 +30,7 @@
 #include <cstdint>
 
 #include "pdg_ops.cuh"
+#include "pdg_tma.cuh"
 #include "pdg_vec.cuh"
 
 namespace pdg {
@@ -83,37 +88,52 @@ __global__ void k_record_c32(const OpParams<double> p, float *__restrict__ rec) 
   r[22] = 0.f;
 }
 
-// asynchronous copy of the source elements [g0, g0 + count) to dst[ph + i],
-// ph = g0 mod 4 (16-byte chunks of a common phase; chunks that reach outside
-// [0, lim) element-wise, zeros there).  Returns dst + ph.
-template <int THREADS>
-__device__ __forceinline__ float *stage_run(float *dst, const float *src, long g0, long lim,
-                                            int count) {
-  const int ph = (int)(((g0 % 4) + 4) % 4);
-  const long ga = g0 - ph;
-  const int nch = (ph + count + 3) / 4;
-  const bool vec_ok = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  for (int c = threadIdx.x; c < nch; c += THREADS) {
-    const long gc = ga + 4L * c;
-    if (vec_ok && gc >= 0 && gc + 4 <= lim) {
-      const unsigned sa = (unsigned)__cvta_generic_to_shared(dst + 4 * c);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src + gc)
-                   : "memory");
+// Staging of a block's input runs.  A run of source elements [g0, g0 + count)
+// lands at dst[ph + i], ph = g0 mod 4, so that source and destination share
+// their 16-byte phase.  Runs inside [0, lim) of an aligned source are one bulk
+// copy by thread 0, completing on `bar` (per-thread copies of all runs cost the
+// operator about 900 of its 3800 instructions per warp); runs that straddle an
+// end are copied element-wise with zeros outside, runs outside are left out
+// (an absent neighbour is read from a zero block).  All threads call it, then
+// wait().
+template <int T>
+struct Stager {
+  unsigned bar, bytes;
+  __device__ __forceinline__ explicit Stager(unsigned long long *b) : bar(smem_u32(b)), bytes(0) {
+    if (threadIdx.x == 0) mbar_init(bar, 1);
+    __syncthreads();
+  }
+  __device__ __forceinline__ float *run(float *dst, const float *src, long g0, long lim,
+                                        int count) {
+    const int ph = (int)(((g0 % 4) + 4) % 4);
+    const long ga = g0 - ph;
+    const int len = (ph + count + 3) & ~3;
+    if (ga + len <= 0 || ga >= lim) return dst + ph;
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && ga >= 0 && ga + len <= lim) {
+      if (threadIdx.x == 0) {
+        // every copy is announced before it is issued; the phase completes
+        // with the arrival in wait()
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar),
+                     "r"(4u * len)
+                     : "memory");
+        bulk_load(smem_u32(dst), src + ga, 4u * len, bar);
+      }
     } else {
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const long g = gc + j;
-        dst[4 * c + j] = (g >= 0 && g < lim) ? src[g] : 0.f;
+      for (int c = threadIdx.x; c < len; c += T) {
+        const long g = ga + c;
+        dst[c] = (g >= 0 && g < lim) ? src[g] : 0.f;
       }
     }
+    return dst + ph;
   }
-  return dst + ph;
-}
-__device__ __forceinline__ void stage_wait() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
-}
+  // false: the copies did not arrive within the poll limit
+  __device__ __forceinline__ bool wait() {
+    if (threadIdx.x == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+    const bool ok = mbar_wait(bar, 0, kTmaPolls);
+    return __syncthreads_and(ok);
+  }
+};
 
 // coefficients of a face in the form of this launch: {a1 kappa_e, a1 kappa_o,
 // penalty, a2 kappa_e} with (a1, a2) = (1, -theta), transposed (-theta, 1)
@@ -148,47 +168,61 @@ __device__ __forceinline__ void cell_line(const C32Tab<N> &tb, float k, const fl
   res[N - 1] += hi.pen * jh - hi.ke * duh - hi.ko * dh;
 }
 
-// write-back of a block's run staged in shared memory (16-byte aligned)
+// write-back of a block's run staged in shared memory: element f(O[i], index)
 template <int N, class F>
 __device__ __forceinline__ void write_run(const float *O, float *y, long g0, long ndof, F f) {
   using C = C32Cfg<N>;
   const int count = (int)min((long)C::RUN, ndof - g0);
-  if ((reinterpret_cast<uintptr_t>(y) & 15) == 0 && count == C::RUN) {
-    // g0 is a multiple of 64 N^3
-    for (int i = 4 * threadIdx.x; i < C::RUN; i += 4 * C::T) {
-      float4 v = *reinterpret_cast<const float4 *>(O + i);
-      v.x = f(v.x, g0 + i);
-      v.y = f(v.y, g0 + i + 1);
-      v.z = f(v.z, g0 + i + 2);
-      v.w = f(v.w, g0 + i + 3);
-      *reinterpret_cast<float4 *>(y + g0 + i) = v;
-    }
-  } else {
-    for (int i = threadIdx.x; i < count; i += C::T) y[g0 + i] = f(O[i], g0 + i);
-  }
+  for (int i = threadIdx.x; i < count; i += C::T) y[g0 + i] = f(O[i], g0 + i);
+}
+// the same unchanged, as one bulk store by thread 0 (full block, 16-byte
+// aligned y; g0 is a multiple of 64 N^3).  The caller has fenced the writes of
+// O for the async proxy before its barrier, and calls bulk_store_wait before
+// the block ends.
+template <int N>
+__device__ __forceinline__ bool bulk_store_ok(const float *y, long g0, long ndof) {
+  return (reinterpret_cast<uintptr_t>(y) & 15) == 0 && g0 + C32Cfg<N>::RUN <= ndof;
+}
+__device__ __forceinline__ void bulk_store(float *y, const float *O, unsigned bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(y),
+               "r"(smem_u32(O)), "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_store_wait() {
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+__device__ __forceinline__ void fence_async() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
 template <int N>
 __global__ void __launch_bounds__(C32Cfg<N>::T)
     k_apply32_cell(const OpParams<float> p, const ApplyArgs<float> a,
-                   const float *__restrict__ rec, const C32Tab<N> tb) {
+                   const float *__restrict__ rec,
+                   const __grid_constant__ C32Tab<N> tb, int *tma_err) {
   using C = C32Cfg<N>;
   constexpr int N2 = C::N2, NB = C::NB, T = C::T;
   extern __shared__ __align__(16) float sm[];
   if (a.skip && *a.skip) return;
   const long e0 = (long)blockIdx.x * T, ndof = p.ncell * NB;
   const long sx = p.nc[0], sxy = (long)p.nc[0] * p.nc[1];
+  __shared__ __align__(8) unsigned long long bar;
+  Stager<T> st(&bar);
   float *Y0 = sm + C::OWNP;
-  const float *OWN = stage_run<T>(sm, a.x, (e0 - 1) * NB, ndof, C::OWN);
-  const float *YL = stage_run<T>(Y0, a.x, (e0 - sx) * NB, ndof, C::RUN);
-  const float *YH = stage_run<T>(Y0 + C::RUNP, a.x, (e0 + sx) * NB, ndof, C::RUN);
-  const float *ZL = stage_run<T>(Y0 + 2 * C::RUNP, a.x, (e0 - sxy) * NB, ndof, C::RUN);
-  const float *ZH = stage_run<T>(Y0 + 3 * C::RUNP, a.x, (e0 + sxy) * NB, ndof, C::RUN);
   float *R0 = Y0 + 4 * C::RUNP;
-  const float *RS = stage_run<T>(R0, rec, e0 * C::REC, p.ncell * C::REC, C::RECS);
+  const float *RS = st.run(R0, rec, e0 * C::REC, p.ncell * C::REC, C::RECS);
+  const float *OWN = st.run(sm, a.x, (e0 - 1) * NB, ndof, C::OWN);
+  const float *YL = st.run(Y0, a.x, (e0 - sx) * NB, ndof, C::RUN);
+  const float *YH = st.run(Y0 + C::RUNP, a.x, (e0 + sx) * NB, ndof, C::RUN);
+  const float *ZL = st.run(Y0 + 2 * C::RUNP, a.x, (e0 - sxy) * NB, ndof, C::RUN);
+  const float *ZH = st.run(Y0 + 3 * C::RUNP, a.x, (e0 + sxy) * NB, ndof, C::RUN);
   float *zero = R0 + C::RECP;   // stands in for an absent neighbour
   if (threadIdx.x < NB) zero[threadIdx.x] = 0.f;
-  stage_wait();
+  if (!st.wait()) {
+    if (threadIdx.x == 0) atomicExch(tma_err, 1);
+    return;
+  }
 
   const int cs = threadIdx.x;
   const long e = e0 + cs;
@@ -264,7 +298,8 @@ __global__ void __launch_bounds__(C32Cfg<N>::T)
   {
     const Face32 xlo(R + 4, a1, a2), xhi(R + 7, a1, a2), ylo(R + 10, a1, a2), yhi(R + 13, a1, a2);
     const float kx = R[0], ky = R[1], kc = R[3];
-#pragma unroll
+    // not unrolled: the instruction cache holds one plane's code
+#pragma unroll 1
     for (int z = 0; z < N; z++) {
       float u[N][N], P[N][N];
 #pragma unroll
@@ -355,13 +390,21 @@ __global__ void __launch_bounds__(C32Cfg<N>::T)
   for (int z = 0; z < N; z++)
 #pragma unroll
     for (int i = 0; i < N2; i++) Y0[cs * NB + z * N2 + i] = out[z][i / N][i % N];
+  const bool plain = !a.accumulate && !a.add && a.alpha == 1.f &&
+                     bulk_store_ok<N>(a.y, e0 * NB, ndof);
+  if (plain) fence_async();
   __syncthreads();
-  write_run<N>(Y0, a.y, e0 * NB, ndof, [&](float v, long g) {
-    float r = a.alpha * v;
-    if (a.accumulate) r += a.y[g];
-    if (a.add) r += a.add[g];
-    return r;
-  });
+  if (plain) {
+    if (threadIdx.x == 0) bulk_store(a.y + e0 * NB, Y0, 4u * C::RUN);
+  } else {
+    write_run<N>(Y0, a.y, e0 * NB, ndof, [&](float v, long g) {
+      float r = a.alpha * v;
+      if (a.accumulate) r += a.y[g];
+      if (a.add) r += a.add[g];
+      return r;
+    });
+  }
+  if (plain && threadIdx.x == 0) bulk_store_wait();
   if (a.dot_part)
     reduce_tail_two_float<T>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
                              RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, TwoFloat{0.f, 0.f},
@@ -372,23 +415,28 @@ __global__ void __launch_bounds__(C32Cfg<N>::T)
 // rq (fused CG): first d -= lambda rq, written back, and the fused sums carry
 // |d|^2 and <d, v>
 template <int N>
-__global__ void __launch_bounds__(C32Cfg<N>::T)
+__global__ void __launch_bounds__(C32Cfg<N>::T, 9)
     k_fdm32_cell(long ncell, const float *__restrict__ Q, const float *__restrict__ L, float *d,
                  float *v, const int *__restrict__ skip, float scale, double *dot_part,
                  long dot_max_blocks, int *dot_cnt, double *dot_scal, int *dot_flags, int dot_fin,
-                 const float *rq) {
+                 const float *rq, int *tma_err) {
   using C = C32Cfg<N>;
   constexpr int N2 = C::N2, NB = C::NB, T = C::T;
   if (skip && *skip) return;
   extern __shared__ __align__(16) float sm[];
   const long e0 = (long)blockIdx.x * T, ndof = ncell * NB;
   float *Q0 = sm + 2 * C::RUNP, *L0 = Q0 + (T * 3 * N2 + 7) / 4 * 4;
-  // runs start at multiples of 64 N^3: no phase
-  stage_run<T>(sm, d, e0 * NB, ndof, C::RUN);
-  if (rq) stage_run<T>(sm + C::RUNP, rq, e0 * NB, ndof, C::RUN);
-  stage_run<T>(Q0, Q, e0 * 3 * N2, ncell * 3 * N2, T * 3 * N2);
-  stage_run<T>(L0, L, e0 * 3 * N, ncell * 3 * N, T * 3 * N);
-  stage_wait();
+  __shared__ __align__(8) unsigned long long bar;
+  Stager<T> st(&bar);
+  // runs start at multiples of 64: no phase
+  st.run(sm, d, e0 * NB, ndof, C::RUN);
+  if (rq) st.run(sm + C::RUNP, rq, e0 * NB, ndof, C::RUN);
+  st.run(Q0, Q, e0 * 3 * N2, ncell * 3 * N2, T * 3 * N2);
+  st.run(L0, L, e0 * 3 * N, ncell * 3 * N, T * 3 * N);
+  if (!st.wait()) {
+    if (threadIdx.x == 0) atomicExch(tma_err, 1);
+    return;
+  }
   const int cs = threadIdx.x;
   const bool active = e0 + cs < ncell;
   float *D = sm + cs * NB, *V = sm + C::RUNP + cs * NB;
@@ -476,10 +524,20 @@ __global__ void __launch_bounds__(C32Cfg<N>::T)
     s1 = two_add(s1, TwoFloat{s, 0.f});
   }
   if (!active) s0 = s1 = TwoFloat{0.f, 0.f};
+  const bool bulk = bulk_store_ok<N>(v, e0 * NB, ndof) && bulk_store_ok<N>(d, e0 * NB, ndof);
+  if (bulk) fence_async();
   __syncthreads();
-  const auto same = [](float x, long) { return x; };
-  if (rq) write_run<N>(sm, d, e0 * NB, ndof, same);
-  write_run<N>(sm + C::RUNP, v, e0 * NB, ndof, same);
+  if (bulk) {
+    if (threadIdx.x == 0) {
+      if (rq) bulk_store(d + e0 * NB, sm, 4u * C::RUN);
+      bulk_store(v + e0 * NB, sm + C::RUNP, 4u * C::RUN);
+    }
+  } else {
+    const auto same = [](float x, long) { return x; };
+    if (rq) write_run<N>(sm, d, e0 * NB, ndof, same);
+    write_run<N>(sm + C::RUNP, v, e0 * NB, ndof, same);
+  }
+  if (bulk && threadIdx.x == 0) bulk_store_wait();
   if (dot_part)
     reduce_tail_two_float<T>(dot_part, dot_max_blocks, dot_cnt,
                              RedCtx{nullptr, dot_scal, dot_flags}, rq ? s0 : s1,
@@ -514,7 +572,8 @@ static int launch_apply32_cell_n(pdg_context *ctx, const ApplyArgs<float> &a,
     tb.d1[i] = (float)ctx->tab_host[2 * C::N2 + N + i];
   }
   const unsigned blocks = (unsigned)((ctx->ncell + C::T - 1) / C::T);
-  k_apply32_cell<N><<<blocks, C::T, smem, ctx->stream>>>(p, a, ctx->rec32c, tb);
+  k_apply32_cell<N><<<blocks, C::T, smem, ctx->stream>>>(p, a, ctx->rec32c, tb,
+                                                          ctx->d_flag + F_TMA);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }
@@ -537,7 +596,8 @@ static int fdm32_cell_n(pdg_context *ctx, const float *d, float *v, const int *s
       ctx->ncell, (const float *)ctx->prec[PDG_F32].Q, (const float *)ctx->prec[PDG_F32].L,
       const_cast<float *>(d), v, skip, scale, fuse ? ctx->fuse_part : nullptr,
       ctx->fuse_max_blocks, ctx->fuse_cnt, ctx->red_out, ctx->d_flag, ctx->fuse_fin,
-      (fuse && ctx->fuse_fin == FIN_CG_DEF_BETA) ? (const float *)ctx->fuse_q : nullptr);
+      (fuse && ctx->fuse_fin == FIN_CG_DEF_BETA) ? (const float *)ctx->fuse_q : nullptr,
+      ctx->d_flag + F_TMA);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }

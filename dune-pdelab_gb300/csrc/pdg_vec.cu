@@ -238,11 +238,6 @@ __global__ void k_set_iter(RedCtx rc, double it) {
   if (rc.flags[F_STATE]) return;
   rc.scal[S_ITER] = it;
 }
-// the same, counting on the device (launches replayed from a graph)
-__global__ void k_inc_iter(RedCtx rc, double step) {
-  if (rc.flags[F_STATE]) return;
-  rc.scal[S_ITER] += step;
-}
 
 static unsigned ew_grid(long n) {
   long g = (n + 255) / 256;
@@ -328,12 +323,6 @@ int set_iter(pdg_context *ctx, const RedCtx &rc, double it) {
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }
-int inc_iter(pdg_context *ctx, const RedCtx &rc, double step) {
-  k_inc_iter<<<1, 1, 0, ctx->stream>>>(rc, step);
-  PDG_CUDA_TRY(cudaGetLastError());
-  return PDG_OK;
-}
-
 #define PDG_INST_UPD(T)                                                                     \
   template int cg_update_xr<T>(pdg_context *, const RedCtx &, long, T *, T *, const T *,    \
                                const T *);                                                  \

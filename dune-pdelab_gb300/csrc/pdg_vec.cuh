@@ -96,6 +96,8 @@ __device__ inline void run_finisher(const RedCtx &rc, int fin, int slot0, int sl
       break;
     }
     case FIN_CG_LAMBDA:
+      // once per iteration of a running solve: the iteration count advances here
+      s[S_ITER] += 1.0;
       s[S_ALPHA] = s[S_RHO] / d0;
       break;
     case FIN_CG_BETA:
@@ -198,6 +200,7 @@ __device__ __forceinline__ void block_sum2_sel(double &a, double &b, double *scr
 // block, then 2 per group from offset 2 * max_blocks; `cnt`: one int per
 // group, zero between launches (each group's last block resets its own).
 constexpr int kFuseGroup = 256;
+constexpr unsigned kFuseOne = 1024;
 
 // (s0, s1): the block's sums, in thread 0
 template <int MAXT, bool kScratch = false>
@@ -205,9 +208,11 @@ __device__ __forceinline__ void grouped_finish(double *part, long max_blocks, in
                                                const RedCtx &rc, double s0, double s1, int fin,
                                                int slot0, int slot1, double *scratch = nullptr) {
   __shared__ bool last;
-  const int b = (int)blockIdx.x, g = b / kFuseGroup;
-  const int ngroups = (int)((gridDim.x + kFuseGroup - 1) / kFuseGroup);
-  const int gsize = min(kFuseGroup, (int)gridDim.x - g * kFuseGroup);
+  // up to kFuseOne blocks: one group, one level
+  const int group = gridDim.x <= kFuseOne ? (int)gridDim.x : kFuseGroup;
+  const int b = (int)blockIdx.x, g = b / group;
+  const int ngroups = (int)((gridDim.x + group - 1) / group);
+  const int gsize = min(group, (int)gridDim.x - g * group);
   if (threadIdx.x == 0) {
     part[2 * b] = s0;
     part[2 * b + 1] = s1;
@@ -219,10 +224,17 @@ __device__ __forceinline__ void grouped_finish(double *part, long max_blocks, in
   __threadfence();
   double a = 0.0, c = 0.0;
   for (int i = threadIdx.x; i < gsize; i += blockDim.x) {
-    a += __ldcg(part + 2 * (g * kFuseGroup + i));
-    c += __ldcg(part + 2 * (g * kFuseGroup + i) + 1);
+    a += __ldcg(part + 2 * (g * group + i));
+    c += __ldcg(part + 2 * (g * group + i) + 1);
   }
   block_sum2_sel<MAXT, kScratch>(a, c, scratch);
+  if (ngroups == 1) {
+    if (threadIdx.x == 0) {
+      cnt[0] = 0;
+      run_finisher(rc, fin, slot0, slot1, a, c);
+    }
+    return;
+  }
   double *gpart = part + 2 * max_blocks;
   if (threadIdx.x == 0) {
     gpart[2 * g] = a;
@@ -334,7 +346,6 @@ template <typename T>
 int bi_update_full(pdg_context *ctx, const RedCtx &rc, long n, T *x, T *r, const T *y,
                    const T *t);   // x += omega y; r -= omega t; def check; rho = rho_new
 int set_iter(pdg_context *ctx, const RedCtx &rc, double it);
-int inc_iter(pdg_context *ctx, const RedCtx &rc, double step);
 
 // plain vector kernels
 template <typename T>
