@@ -25,6 +25,7 @@
 
 #include "pdg_fixed.cuh"
 #include "pdg_ops.cuh"
+#include "pdg_vec.cuh"
 
 namespace pdg {
 
@@ -142,9 +143,10 @@ __global__ void k_record_i(long ncell, const double *__restrict__ rec, int2 *__r
 
 // The block's cells in plain FP64 (weak form, from the FP64 record): not a
 // fast path, it keeps what FP64 gives for infinities, NaN and values near the
-// ends of the range.  Called by every thread of the block.
+// ends of the range.  Called by every thread of the block; returns the sum of
+// x * y_out over the thread's column.
 template <int N>
-__device__ __noinline__ void apply_cells_fp64(const OpParams<double> &p,
+__device__ __noinline__ double apply_cells_fp64(const OpParams<double> &p,
                                               const ApplyArgs<double> &a,
                                               const double *__restrict__ rec, double *cell,
                                               int l, int ee, const int *nbr, bool active) {
@@ -206,7 +208,8 @@ __device__ __noinline__ void apply_cells_fp64(const OpParams<double> &p,
     ue[z * N2 + l] = t1;
   }
   __syncthreads();
-  if (!active) return;
+  double part = 0.0;
+  if (!active) return part;
   for (int z = 0; z < N; z++) {
     double s = 0.0;
     for (int q = 0; q < N; q++)
@@ -215,8 +218,10 @@ __device__ __noinline__ void apply_cells_fp64(const OpParams<double> &p,
     const size_t idx = (size_t)ee * NB + z * TPC + l;
     if (a.accumulate) s += a.y[idx];
     if (a.add) s += a.add[idx];
+    part += a.x[idx] * s;
     a.y[idx] = s;
   }
+  return part;
 }
 
 // Five and six blocks per SM at k = 4 and 3 instead of the four the register
@@ -357,8 +362,18 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : 6)
       zf[2 * (f - 4) + 1] = split32(s2);
     }
   }
+  // <x, y_out> of the fused CG: block sums in the cell memory, once it is free
+  const auto finish = [&](double part) {
+    __syncthreads();
+    reduce_tail_grouped<C::THREADS, true>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
+                                          RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, 0.0,
+                                          a.dot_fin, -1, -1,
+                                          reinterpret_cast<double *>(smem_raw));
+  };
   if (__syncthreads_or(bad)) {
-    apply_cells_fp64<N>(p, a, rec64, reinterpret_cast<double *>(ue), l, ee, nbr, active);
+    const double part =
+        apply_cells_fp64<N>(p, a, rec64, reinterpret_cast<double *>(ue), l, ee, nbr, active);
+    if (a.dot_part) finish(part);
     return;
   }
 
@@ -436,6 +451,7 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : 6)
   }
   __syncthreads();
   // ---- out = M_z W + M_y T1 ----
+  double part = 0.0;
   if (active) {
     // one unit of the integers below as an FP64 factor (0: all of the cell's
     // data is zero)
@@ -457,9 +473,11 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : 6)
       const int idx = z * TPC + l;
       if (a.accumulate) r += ye[idx];
       if (ad) r += ad[idx];
+      if (a.dot_part) part += xe[idx] * r;
       ye[idx] = r;
     }
   }
+  if (a.dot_part) finish(part);
 }
 
 template <int N>
@@ -517,8 +535,18 @@ static int launch_i_n(pdg_context *ctx, const ApplyArgs<double> &a, const OpPara
   const long work = a.ncells > 0 ? a.ncells : ctx->ncell;
   if (work <= 0) return PDG_OK;
   const unsigned blocks = (unsigned)((work + C::CPB - 1) / C::CPB);
+  ApplyArgs<double> af = a;
+  if (ctx->fuse_fin && a.ncells == 0) {
+    // the fused CG: <p, A p> -> lambda in the same launch
+    af.dot_part = ctx->fuse_part;
+    af.dot_max_blocks = ctx->fuse_max_blocks;
+    af.dot_cnt = ctx->fuse_cnt;
+    af.dot_scal = ctx->red_out;
+    af.dot_flags = ctx->d_flag;
+    af.dot_fin = ctx->fuse_fin;
+  }
   k_apply_i<N><<<blocks, C::THREADS, smem, ctx->stream>>>(
-      p, a, a.transpose ? ctx->reciT : ctx->reci, a.transpose ? ctx->reciT_exp : ctx->reci_exp,
+      p, af, a.transpose ? ctx->reciT : ctx->reci, a.transpose ? ctx->reciT_exp : ctx->reci_exp,
       ctx->rec64);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;

@@ -25,6 +25,7 @@
 // their block to a plain FP64 evaluation.
 #include "pdg_fixed.cuh"
 #include "pdg_ops.cuh"
+#include "pdg_vec.cuh"
 
 namespace pdg {
 
@@ -103,9 +104,10 @@ __global__ void k_fdm_record_i(long ncell, const double *__restrict__ Q, double 
 }
 
 // The block's cells in plain FP64: not a fast path (see apply_cells_fp64 in
-// pdg_apply_i.cu).  Called by every thread of the block.
+// pdg_apply_i.cu).  Called by every thread of the block; returns the sum of
+// d * v over the thread's column.
 template <int N>
-__device__ __noinline__ void fdm_cells_fp64(const double *__restrict__ Q,
+__device__ __noinline__ double fdm_cells_fp64(const double *__restrict__ Q,
                                             const double *__restrict__ L, const double *d,
                                             double *v, double *S0, int l, long e, bool active,
                                             double scale) {
@@ -144,12 +146,16 @@ __device__ __noinline__ void fdm_cells_fp64(const double *__restrict__ Q,
     for (int y = 0; y < N; y++) s += Qy[ty * N + y] * S1[z * N2 + y * N + tx];
     S0[z * N2 + l] = s;
   }
-  if (!active) return;
+  double part = 0.0;
+  if (!active) return part;
   for (int z = 0; z < N; z++) {
     double s = 0.0;
     for (int zp = 0; zp < N; zp++) s += Qz[z * N + zp] * S0[zp * N2 + l];
+    const double dz = d[e * NB + z * N2 + l];
     v[e * NB + z * N2 + l] = scale * s;
+    part += dz * (scale * s);
   }
+  return part;
 }
 
 // contraction of N limb pairs (fb: 59 bits), shifted right by s >= 0, rounded
@@ -170,13 +176,26 @@ __device__ __forceinline__ long long shift_by(long long v, int s) {
   return s >= 0 ? (long long)((unsigned long long)v << s) : (v + ((1ll << r) >> 1)) >> r;
 }
 
-// d and v may be the same vector: a cell is read before it is written
-template <int N>
+// One launch: the operands of the fused CG, or part null.  rq != null: first
+// d -= lambda rq (lambda = scal[S_ALPHA]), written back; the sums then carry
+// |d|^2 and <d, v>.  d, v and rq may alias element-wise: every entry is read
+// and written by one thread, read before it is written.
+struct FdmFuse {
+  double *part;
+  long max_blocks;
+  int *cnt;
+  double *scal;
+  int *flags;
+  int fin;
+  const double *rq;
+};
+
+template <int N, bool kFuse>
 __global__ void __launch_bounds__(FICfg<N>::THREADS)
     k_fdm_i(long ncell, const int2 *__restrict__ Qi, const int *__restrict__ exps,
             const double *__restrict__ Linv, const double *__restrict__ Q64,
-            const double *__restrict__ L64, const double *d, double *v, const int *__restrict__ skip, const int *__restrict__ cells, int ncells,
-            double scale) {
+            const double *__restrict__ L64, double *d, double *v, const int *__restrict__ skip,
+            const int *__restrict__ cells, int ncells, double scale, const FdmFuse fuse) {
   using C = FICfg<N>;
   constexpr int N2 = C::N2, NB = C::NB, TPC = C::TPC, CPB = C::CPB;
   if (skip && *skip) return;
@@ -200,6 +219,19 @@ __global__ void __launch_bounds__(FICfg<N>::THREADS)
     lin[z] = Linv[e * NB + z * TPC + l];
   }
   for (int i = l; i < 3 * N2; i += TPC) Qs[i] = Qi[e * 3 * N2 + i];
+  double part2 = 0.0;
+  if (kFuse && fuse.rq) {
+    const double lambda = fuse.scal[S_ALPHA];
+#pragma unroll
+    for (int z = 0; z < N; z++) {
+      const size_t i = e * NB + z * TPC + l;
+      col[z] -= lambda * fuse.rq[i];
+      if (active) {
+        d[i] = col[z];
+        part2 += col[z] * col[z];
+      }
+    }
+  }
   const int *ex = exps + e * C::NEXP;
   BlockExp b;
 #pragma unroll
@@ -225,8 +257,17 @@ __global__ void __launch_bounds__(FICfg<N>::THREADS)
       S0[zp * N2 + l] = limbs(contract<N>([&](int q) { return Qz[q * N + zp]; },
                                           [&](int q) { return u[q]; }, 0));
   }
+  const auto finish = [&](double part) {
+    __syncthreads();
+    reduce_tail_grouped<C::THREADS, true>(
+        fuse.part, fuse.max_blocks, fuse.cnt, RedCtx{nullptr, fuse.scal, fuse.flags},
+        fuse.rq ? part2 : part, fuse.rq ? part : 0.0, fuse.fin, -1, -1,
+        reinterpret_cast<double *>(smem_raw));
+  };
   if (__syncthreads_or(bad)) {
-    fdm_cells_fp64<N>(Q64, L64, d, v, reinterpret_cast<double *>(S0), l, e, active, scale);
+    const double part = fdm_cells_fp64<N>(Q64, L64, d, v, reinterpret_cast<double *>(S0), l, e,
+                                          active, scale);
+    if (kFuse) finish(part);
     return;
   }
   // y
@@ -290,6 +331,7 @@ __global__ void __launch_bounds__(FICfg<N>::THREADS)
     for (int z = 0; z < N; z++)
       u[z] = limbs(contract<N>([&](int q) { return c[q]; },
                                [&](int q) { return S1[z * N2 + q * N + tx]; }, s));
+    double part = 0.0;
     if (active) {
       // one unit of the last contraction
       const int E = Ed + top - 1140 + ex[0] + ex[1];
@@ -300,9 +342,13 @@ __global__ void __launch_bounds__(FICfg<N>::THREADS)
         long long hh = 0, mid = 0;
 #pragma unroll
         for (int q = 0; q < N; q++) mac2(hh, mid, Qz[z * N + q], u[q]);
-        v[e * NB + z * N2 + l] = scale * ((double)mac2_value_wide(hh, mid) * unit);
+        const double r = scale * ((double)mac2_value_wide(hh, mid) * unit);
+        const size_t i = e * NB + z * N2 + l;
+        if (kFuse) part += d[i] * r;
+        v[i] = r;
       }
     }
+    if (kFuse) finish(part);
   }
 }
 
@@ -337,9 +383,16 @@ static int fdm_apply_i_n(pdg_context *ctx, const double *d, double *v, const int
   if (work <= 0) return PDG_OK;
   const size_t smem = sizeof(int2) * C::CPB * C::PER_CELL;
   const unsigned blocks = (unsigned)((work + C::CPB - 1) / C::CPB);
-  k_fdm_i<N><<<blocks, C::THREADS, smem, ctx->stream>>>(
-      ctx->ncell, pd.Qi, pd.Qi_exp, pd.Lsum_inv, (const double *)pd.Q, (const double *)pd.L, d, v,
-      skip, cells, ncells, scale);
+  FdmFuse fuse{};
+  if (ctx->fuse_fin && !cells)
+    fuse = FdmFuse{ctx->fuse_part, ctx->fuse_max_blocks, ctx->fuse_cnt, ctx->red_out, ctx->d_flag,
+                   ctx->fuse_fin,
+                   ctx->fuse_fin == FIN_CG_DEF_BETA ? (const double *)ctx->fuse_q : nullptr};
+  // the fused form is its own instance: its code in the plain one cost 4 %
+  auto *kernel = fuse.part ? k_fdm_i<N, true> : k_fdm_i<N, false>;
+  kernel<<<blocks, C::THREADS, smem, ctx->stream>>>(
+      ctx->ncell, pd.Qi, pd.Qi_exp, pd.Lsum_inv, (const double *)pd.Q, (const double *)pd.L,
+      const_cast<double *>(d), v, skip, cells, ncells, scale, fuse);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }
