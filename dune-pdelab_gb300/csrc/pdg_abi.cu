@@ -277,7 +277,25 @@ static int fetch_state(pdg_context *ctx, double *scal, int *flags) {
   PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (scal) std::memcpy(scal, ctx->h_red, sizeof(double) * S_COUNT);
   if (flags) std::memcpy(flags, hf, sizeof(int) * F_COUNT);
-  if (hf[F_TMA]) return set_error(PDG_ETIMEOUT, "TMA staging of the FP32 operator timed out");
+  if (hf[F_TMA]) return set_error(PDG_ETIMEOUT, "a bounded device wait ran out");
+  return PDG_OK;
+}
+
+// after batch k of CG iterations: copy the flags behind it, and look at those
+// of batch k - 1, whose copy the host waits for while batch k runs
+static int poll_batch(pdg_context *ctx, int k, bool *done) {
+  for (int j = 0; j < 2; j++)
+    if (!ctx->ev_poll[j])
+      PDG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ev_poll[j], cudaEventDisableTiming));
+  int *slots = reinterpret_cast<int *>(ctx->h_red + S_COUNT) + F_COUNT;
+  PDG_CUDA_TRY(cudaMemcpyAsync(slots + F_COUNT * (k & 1), ctx->d_flag, sizeof(int) * F_COUNT,
+                               cudaMemcpyDeviceToHost, ctx->stream));
+  PDG_CUDA_TRY(cudaEventRecord(ctx->ev_poll[k & 1], ctx->stream));
+  if (k == 0) return PDG_OK;
+  PDG_CUDA_TRY(cudaEventSynchronize(ctx->ev_poll[(k - 1) & 1]));
+  const int *f = slots + F_COUNT * ((k - 1) & 1);
+  if (f[F_TMA]) return set_error(PDG_ETIMEOUT, "a bounded device wait ran out");
+  if (f[F_STATE]) *done = true;
   return PDG_OK;
 }
 
@@ -348,10 +366,11 @@ static int ensure_fuse(pdg_context *ctx) {
 }
 
 // dune-istl CGSolver::apply restated on the device.  x: initial guess and
-// result; b: right-hand side, overwritten by the defect.  w0, w1: work.
+// result; b: right-hand side, overwritten by the defect.  w[0..2]: work.
 template <typename T>
-static int cg_device(pdg_context *ctx, T *x, T *b, T *p, T *q, double reduction, int maxit,
+static int cg_device(pdg_context *ctx, T *x, T *b, T **w, double reduction, int maxit,
                      int transpose, KrylovOut *out) {
+  T *p = w[0], *q = w[1];
   const RedCtx rc = red_ctx(ctx);
   const int *skip = ctx->d_flag + F_STATE;
   k_init_solve<<<1, 1, 0, ctx->stream>>>(rc.scal, rc.flags, reduction);
@@ -368,6 +387,19 @@ static int cg_device(pdg_context *ctx, T *x, T *b, T *p, T *q, double reduction,
   bool done = false;
   const bool fuse = std::is_same<T, float>::value ? cg_fusable(ctx)
                                                   : cg_fusable64(ctx, transpose);
+  if constexpr (std::is_same<T, double>::value) {
+    // a small 2D grid: all iterations in one launch
+    bool ran = false;
+    if (fuse && ctx->dim == 2) PDG_TRY(cg2d_solve(ctx, x, b, p, q, w[2], maxit, &ran));
+    if (ran) {
+      PDG_TRY(fetch_state(ctx, scal, flags));
+      out->state = flags[F_STATE];
+      out->def0 = scal[S_DEF0];
+      out->def = scal[S_DEF];
+      out->iterations = (int)scal[S_ITER];
+      return PDG_OK;
+    }
+  }
   if (fuse) PDG_TRY(ensure_fuse(ctx));
   // one iteration's launches (the iteration count advances on the device)
   auto body = [&]() -> int {
@@ -399,8 +431,10 @@ static int cg_device(pdg_context *ctx, T *x, T *b, T *p, T *q, double reduction,
   // After two batches run one by one (lazy set-up done, the solve not yet
   // converged), a batch of iterations is captured once into a CUDA graph and
   // replayed: one launch per batch instead of one per kernel, which is what
-  // small grids are bound by.  Launches after convergence skip their work.
+  // small grids are bound by.  Launches after convergence skip their work, so
+  // the state of a batch is looked at while the next one runs.
   cudaGraphExec_t gexec = nullptr;
+  int nbatch = 0;
   const bool graphs = ctx->stream != nullptr && ctx->stream != cudaStreamLegacy &&
                       ctx->stream != cudaStreamPerThread && !ctx->use_matrix;
   int st = PDG_OK;
@@ -425,6 +459,9 @@ static int cg_device(pdg_context *ctx, T *x, T *b, T *p, T *q, double reduction,
         return set_error(PDG_ECUDA, "CUDA graph launch failed");
       }
       i += batch;
+      st = poll_batch(ctx, nbatch++, &done);
+      if (st != PDG_OK) break;
+      continue;
     } else {
       st = body();
       if (st != PDG_OK) break;
@@ -505,7 +542,7 @@ template <typename T>
 static int krylov_device(pdg_context *ctx, int method, T *x, T *b, T **w, double reduction,
                          int maxit, int transpose, KrylovOut *out, double guard = 0.0,
                          int restart = 30, int replace = 0) {
-  if (method == PDG_CG) return cg_device<T>(ctx, x, b, w[0], w[1], reduction, maxit, transpose, out);
+  if (method == PDG_CG) return cg_device<T>(ctx, x, b, w, reduction, maxit, transpose, out);
   if (method == PDG_BICGSTAB)
     return bicgstab_device<T>(ctx, x, b, w, reduction, maxit, transpose, out, guard, replace);
   if (method == PDG_GMRES) {
@@ -1081,7 +1118,7 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
       cudaMalloc(&c->red_partials, sizeof(double) * 2 * kRedBlocks) != cudaSuccess ||
       cudaMalloc(&c->red_out, sizeof(double) * S_COUNT) != cudaSuccess ||
       cudaMalloc(&c->d_flag, sizeof(int) * F_COUNT) != cudaSuccess ||
-      cudaMallocHost(&c->h_red, sizeof(double) * S_COUNT + sizeof(int) * F_COUNT) != cudaSuccess)
+      cudaMallocHost(&c->h_red, sizeof(double) * S_COUNT + sizeof(int) * 3 * F_COUNT) != cudaSuccess)
     return fail(set_error(PDG_ECUDA, "device allocation failed"));
   cudaMemcpy(c->tab64, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice);
   if (c->dim == 3) {
@@ -1202,7 +1239,7 @@ int pdg_destroy(pdg_context *c) {
                   c->fuse_part, c->fuse_cnt, c->Ac64, c->Aqv64, c->Aqf64, c->cq64, c->Ac32,
                   c->Aqv32, c->Aqf32, c->cq32, c->bqv64, c->bqf64, c->Kd64, c->Kd32,
                   c->recfp, c->tabfp, c->rec32q, c->rec32c, c->rec64m, c->rec64mT, c->tabm64,
-                  c->tabt64, c->tabt32, c->reci, c->reciT, c->reci_exp, c->reciT_exp};
+                  c->tabt64, c->tabt32, c->cg2_slots, c->reci, c->reciT, c->reci_exp, c->reciT_exp};
   for (void *b : bufs)
     if (b) cudaFree(b);
   for (int i = 0; i < 10; i++)
@@ -1210,6 +1247,8 @@ int pdg_destroy(pdg_context *c) {
   for (int i = 0; i < 8; i++)
     if (c->w32[i]) cudaFree(c->w32[i]);
   if (c->h_red) cudaFreeHost(c->h_red);
+  for (cudaEvent_t ev : c->ev_poll)
+    if (ev) cudaEventDestroy(ev);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);

@@ -1,0 +1,400 @@
+// pdg_cg2d.cu -- a whole FP64 CG solve with the FDM cell-block Jacobi on a
+// small 2D grid in one cooperative launch.
+//
+// Reference: dune-istl's CGSolver over OnTheFlyOperator and
+// GridOperatorPreconditioner (backend/istl/matrixfree/backends.hh:116-126),
+// the recurrence of cg_device (pdg_abi.cu) with the arithmetic of
+// k_apply<double, 2, N> and k_fdm_apply<double, 2, N>.
+//
+// A 2D grid of a few thousand cells gives a launch microseconds of work: with
+// three launches per iteration the 2D Q1 64^2 solve took 24 us per iteration,
+// nearly all of it launches and reduction tails.  Here every SM owns a run of
+// cells for the whole solve.  Their records, factors and vectors stay in shared
+// memory; only the search direction and the preconditioned residual are
+// written to global memory, for the neighbours' face terms.  An iteration is
+// two grid-wide sums:
+//
+//   p = z + beta p (own cells; a neighbour's p is formed from its z and its
+//   previous p), q = A p                                 -- sum <p, q>
+//   x += lambda p, r -= lambda q, z = M^-1 r              -- sums <r, r>, <z, r>
+//
+// A grid-wide sum is one exchange: each block publishes its partial sums in its
+// slot and all blocks read all slots, adding them in block order (the same
+// result everywhere, and the same in every run).  Reading a slot of block j
+// also orders the reader after everything block j wrote before, so it is the
+// barrier as well.  Waits are bounded.
+#include <algorithm>
+
+#include "pdg_ops.cuh"
+#include "pdg_vec.cuh"
+
+namespace pdg {
+
+template <int N>
+struct CG2Cfg {
+  static constexpr int N2 = N * N;
+  static constexpr int REC = 2 * N2 + 20;              // k_cell_record<double, 2, N>
+  // per cell in shared memory: record, Q, 1/(lx+ly), and x, r, p, q, z
+  static constexpr int PER_CELL = REC + 2 * N2 + N2 + 5 * N2;
+  static constexpr int TAB = N2 + 2 * N;
+};
+
+constexpr int kCg2Sets = 4;              // slot sets in use in turn
+// threads per block: one for each of the 2 x 152 slots a block polls, so that
+// an exchange is one L2 round trip; cells go to the first threads
+constexpr int kCg2Threads = 320;
+constexpr int kCg2Polls = 1 << 21;       // bound of one wait (seconds)
+// an empty slot: a NaN no arithmetic produces
+constexpr unsigned long long kCg2Empty = 0xffffffffffffffffull;
+
+struct Cg2Args {
+  const double *rec, *Q, *Linv;
+  double *x, *b;          // solution and defect (both updated)
+  double *p[2], *z;       // exchanged vectors
+  unsigned long long *slots;   // [kCg2Sets][2][grid], all empty
+  double *scal;
+  int *flags;
+  int maxit, cells_per_block;
+};
+
+__device__ __forceinline__ unsigned long long ld_slot(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_slot(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// The sums of v0 (and v1, nv = 2) over the first nw warps of all blocks, in
+// every thread; the round number picks the slot set.  false: a block did not
+// publish in time.  red: shared scratch of 2 * 32 + 2 * gridDim doubles.
+__device__ __forceinline__ bool grid_sum(const Cg2Args &g, unsigned round, int nv, int nw,
+                                         double &v0, double &v1, double *red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nb = gridDim.x;
+  double *all = red + 64;
+  if (w < nw) {
+    v0 = warp_sum_d(v0);
+    if (nv > 1) v1 = warp_sum_d(v1);
+    if (lane == 0) {
+      red[2 * w] = v0;
+      red[2 * w + 1] = v1;
+    }
+  }
+  __syncthreads();   // every thread's global writes come before the fence below
+  const unsigned set = round % kCg2Sets;
+  if (threadIdx.x < nv) {
+    const int k = threadIdx.x;
+    double v = red[k];
+    for (int i = 1; i < nw; i++) v += red[2 * i + k];
+    // free the own slots of the set after next: all blocks have read them (they
+    // published the previous round after that)
+    unsigned long long *old = g.slots + 2 * (size_t)((set + 2) % kCg2Sets) * nb + blockIdx.x;
+    st_slot(old + k * nb, kCg2Empty);
+    if (nv == 1) st_slot(old + nb, kCg2Empty);
+    __threadfence();
+    const unsigned long long a = __double_as_longlong(v);
+    st_slot(g.slots + (2 * (size_t)set + k) * nb + blockIdx.x,
+            a == kCg2Empty ? 0x7ff8000000000000ull : a);
+  }
+  bool ok = true;
+  for (int i = threadIdx.x; i < nv * nb; i += kCg2Threads) {
+    const unsigned long long *s = g.slots + 2 * (size_t)set * nb + i;
+    unsigned long long v = ld_slot(s);
+    for (int it = 0; v == kCg2Empty && it < kCg2Polls; it++) v = ld_slot(s);
+    ok = ok && v != kCg2Empty;
+    all[i] = __longlong_as_double(v);
+  }
+  __threadfence();
+  ok = __syncthreads_and(ok);
+  if (w < nv) {
+    double a = 0.0;
+    for (int i = lane; i < nb; i += 32) a += all[w * nb + i];
+    a = warp_sum_d(a);
+    if (lane == 0) red[62 + w] = a;
+  }
+  __syncthreads();
+  v0 = red[62];
+  if (nv > 1) v1 = red[63];
+  return ok;
+}
+
+template <int N>
+__global__ void __launch_bounds__(kCg2Threads)
+    k_cg2d(const OpParams<double> pr, const Cg2Args g) {
+  using C = CG2Cfg<N>;
+  constexpr int N2 = C::N2;
+  extern __shared__ __align__(16) double sh[];
+  __shared__ double sc[2];
+  const int t = threadIdx.x;
+  const int c0 = blockIdx.x * g.cells_per_block;
+  const int c1 = min((int)pr.ncell, c0 + g.cells_per_block);
+  const int nc = max(0, c1 - c0), cap = g.cells_per_block;
+  const int nw = (min(cap, kCg2Threads) + 31) / 32;
+  // arrays [entry][cell] in shared memory: one cell per thread, no conflicts
+  double *rec = sh, *Q = rec + C::REC * cap, *Li = Q + 2 * N2 * cap, *X = Li + N2 * cap,
+         *R = X + N2 * cap, *P = R + N2 * cap, *W = P + N2 * cap, *Z = W + N2 * cap,
+         *tM = Z + N2 * cap, *red = tM + C::TAB;
+  const double *td0 = tM + N2, *td1 = td0 + N;
+  if (g.flags[F_STATE]) return;   // converged before the first iteration
+  for (int i = t; i < nc * C::REC; i += kCg2Threads)
+    rec[(i % C::REC) * cap + i / C::REC] = g.rec[(size_t)c0 * C::REC + i];
+  for (int i = t; i < nc * 2 * N2; i += kCg2Threads)
+    Q[(i % (2 * N2)) * cap + i / (2 * N2)] = g.Q[(size_t)c0 * 2 * N2 + i];
+  for (int i = t; i < nc * N2; i += kCg2Threads) {
+    const int k = (i % N2) * cap + i / N2;
+    const size_t o = (size_t)c0 * N2 + i;
+    Li[k] = g.Linv[o];
+    X[k] = g.x[o];
+    R[k] = g.b[o];
+    // the first direction p = M^-1 b is given in p[0]; z = 0 and beta = 1
+    // reproduce it in the first iteration
+    P[k] = g.p[0][o];
+  }
+  for (int i = t; i < N2; i += kCg2Threads) tM[i] = pr.tab[i];
+  for (int i = t; i < 2 * N; i += kCg2Threads) tM[N2 + i] = pr.tab[2 * N2 + i];
+  double rho = g.scal[S_RHO], beta = 0.0, def = g.scal[S_DEF];
+  const double stop = g.scal[S_DEF0] * g.scal[S_RED];
+  __syncthreads();
+
+  int state = 0, it = 0;
+  unsigned round = 0;
+  double lambda = 0.0;
+  while (it < g.maxit && state == 0) {
+    // ---- p = z + beta p, q = A p ----
+    const double *pold = g.p[it & 1];
+    double *pnew = g.p[(it + 1) & 1];
+    const bool first = it == 0;
+    double s0 = 0.0, s1 = 0.0;
+    for (int c = t; c < nc; c += kCg2Threads) {
+      const int e = c0 + c;
+      const int iy = e / pr.nc[0], ix = e - iy * pr.nc[0];
+      const double *rc = rec + c;   // entry k of the record: rc[k * cap]
+      double u[N][N];
+#pragma unroll
+      for (int k = 0; k < N2; k++) {
+        const double v = first ? P[k * cap + c] : fma(beta, P[k * cap + c], Z[k * cap + c]);
+        u[k / N][k % N] = v;
+        P[k * cap + c] = v;
+        __stcg(pnew + (size_t)e * N2 + k, v);
+      }
+      // neighbour lines: (s1, s2) per face point, as in k_apply
+      double f1[4][N], f2[4][N];
+#pragma unroll
+      for (int f = 0; f < 4; f++) {
+        const int hi = f & 1;
+        const bool on = f == 0 ? ix > 0 : f == 1 ? ix + 1 < pr.nc[0] : f == 2 ? iy > 0
+                                                                              : iy + 1 < pr.nc[1];
+        const int nb = f == 0 ? e - 1 : f == 1 ? e + 1 : f == 2 ? e - pr.nc[0] : e + pr.nc[0];
+        double v[N2];
+#pragma unroll
+        for (int k = 0; k < N2; k++) {
+          const size_t o = (size_t)(on ? nb : e) * N2 + k;
+          const double po = __ldcg(pold + o);
+          v[k] = first ? po : fma(beta, po, __ldcg(g.z + o));
+        }
+        // {hp ke, hp ko, hp pen, th hp ke, th hp ko} of the face
+        const double ko = rc[(2 * N2 + 5 * f + 1) * cap], pen = rc[(2 * N2 + 5 * f + 2) * cap],
+                     tke = rc[(2 * N2 + 5 * f + 3) * cap];
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          double dv = 0.0;
+#pragma unroll
+          for (int q = 0; q < N; q++)
+            dv += (hi ? td0[q] : td1[q]) * (f < 2 ? v[a * N + q] : v[q * N + a]);
+          const int qv = hi ? 0 : N - 1;
+          const double val = f < 2 ? v[a * N + qv] : v[qv * N + a];
+          f1[f][a] = on ? (hi ? -ko * dv : ko * dv) - pen * val : 0.0;
+          f2[f][a] = on ? (hi ? -tke : tke) * val : 0.0;
+        }
+      }
+      double Xp[N][N], Yp[N][N];
+#pragma unroll
+      for (int y = 0; y < N; y++)
+#pragma unroll
+        for (int x = 0; x < N; x++) {
+          double sx = 0.0, sy = 0.0;
+#pragma unroll
+          for (int q = 0; q < N; q++) {
+            sx += rc[(x * N + q) * cap] * u[y][q];
+            sy += rc[(N2 + y * N + q) * cap] * u[q][x];
+          }
+          if (x == 0) sx += f1[0][y];
+          sx += td0[x] * f2[0][y];
+          if (x == N - 1) sx += f1[1][y];
+          sx += td1[x] * f2[1][y];
+          if (y == 0) sy += f1[2][x];
+          sy += td0[y] * f2[2][x];
+          if (y == N - 1) sy += f1[3][x];
+          sy += td1[y] * f2[3][x];
+          Xp[y][x] = sx;
+          Yp[y][x] = sy;
+        }
+#pragma unroll
+      for (int y = 0; y < N; y++)
+#pragma unroll
+        for (int x = 0; x < N; x++) {
+          double s = 0.0;
+#pragma unroll
+          for (int q = 0; q < N; q++) {
+            s += tM[y * N + q] * Xp[q][x];
+            s += tM[x * N + q] * Yp[y][q];
+          }
+          W[(y * N + x) * cap + c] = s;
+          s0 += u[y][x] * s;
+        }
+    }
+    if (!grid_sum(g, round++, 1, nw, s0, s1, red)) {
+      state = -1;
+      break;
+    }
+    if (t == 0) sc[0] = rho / s0;
+    __syncthreads();
+    lambda = sc[0];
+    it++;
+    // ---- x += lambda p, r -= lambda q, z = M^-1 r ----
+    s0 = s1 = 0.0;
+    for (int c = t; c < nc; c += kCg2Threads) {
+      const int e = c0 + c;
+      double r[N][N], a[N][N];
+#pragma unroll
+      for (int k = 0; k < N2; k++) {
+        const int i = k * cap + c;
+        X[i] += lambda * P[i];
+        const double v = R[i] - lambda * W[i];
+        R[i] = v;
+        r[k / N][k % N] = v;
+        s0 += v * v;
+      }
+      const double *Qx = Q + c, *Qy = Qx + N2 * cap;   // entry [i][j]: Qx[(i N + j) cap]
+      double w[N][N];
+#pragma unroll
+      for (int yp = 0; yp < N; yp++)
+#pragma unroll
+        for (int x = 0; x < N; x++) {
+          double s = 0.0;
+#pragma unroll
+          for (int y = 0; y < N; y++) s += Qy[(y * N + yp) * cap] * r[y][x];
+          w[yp][x] = s;
+        }
+#pragma unroll
+      for (int y = 0; y < N; y++)
+#pragma unroll
+        for (int xp = 0; xp < N; xp++) {
+          double s = 0.0;
+#pragma unroll
+          for (int x = 0; x < N; x++) s += Qx[(x * N + xp) * cap] * w[y][x];
+          a[y][xp] = s * Li[(y * N + xp) * cap + c];
+        }
+#pragma unroll
+      for (int y = 0; y < N; y++)
+#pragma unroll
+        for (int x = 0; x < N; x++) {
+          double s = 0.0;
+#pragma unroll
+          for (int xp = 0; xp < N; xp++) s += Qx[(x * N + xp) * cap] * a[y][xp];
+          w[y][x] = s;
+        }
+#pragma unroll
+      for (int y = 0; y < N; y++)
+#pragma unroll
+        for (int x = 0; x < N; x++) {
+          double s = 0.0;
+#pragma unroll
+          for (int yp = 0; yp < N; yp++) s += Qy[(y * N + yp) * cap] * w[yp][x];
+          Z[(y * N + x) * cap + c] = s;
+          __stcg(g.z + (size_t)e * N2 + y * N + x, s);
+          s1 += r[y][x] * s;
+        }
+    }
+    if (!grid_sum(g, round++, 2, nw, s0, s1, red)) {
+      state = -1;
+      break;
+    }
+    if (t == 0) {
+      sc[0] = sqrt(s0);
+      sc[1] = s1 / rho;
+    }
+    __syncthreads();
+    def = sc[0];
+    beta = sc[1];
+    rho = s1;
+    if (!isfinite(def)) state = 2;
+    else if (def < stop || def < 1e-30) state = 1;
+  }
+  for (int i = t; i < nc * N2; i += kCg2Threads) {
+    const int k = (i % N2) * cap + i / N2;
+    const size_t o = (size_t)c0 * N2 + i;
+    g.x[o] = X[k];
+    g.b[o] = R[k];
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    g.scal[S_DEF] = def;
+    g.scal[S_RHO] = rho;
+    g.scal[S_ALPHA] = lambda;
+    g.scal[S_BETA] = beta;
+    g.scal[S_ITER] = it;
+    if (state > 0) g.flags[F_STATE] = state;
+  }
+  if (state < 0 && t == 0) atomicExch(&g.flags[F_TMA], 1);
+}
+
+__global__ void k_cg2d_slots(unsigned long long *s, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) s[i] = kCg2Empty;
+}
+
+template <int N>
+static int cg2d_n(pdg_context *ctx, double *x, double *b, double *p, double *p2, double *z,
+                  int maxit, bool *ran) {
+  using C = CG2Cfg<N>;
+  *ran = false;
+  static int dev = -1, sms = 0, coop = 0, smem_max = 0;
+  if (dev != ctx->device) {
+    PDG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    PDG_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+    PDG_CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                        ctx->device));
+    cudaFuncAttributes fa;
+    PDG_CUDA_TRY(cudaFuncGetAttributes(&fa, k_cg2d<N>));
+    smem_max -= (int)fa.sharedSizeBytes;
+    PDG_CUDA_TRY(cudaFuncSetAttribute(k_cg2d<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      smem_max));
+    dev = ctx->device;
+  }
+  if (!coop || sms < 1) return PDG_OK;
+  const int grid = (int)std::min<long>(sms, ctx->ncell);
+  const int cap = (int)((ctx->ncell + grid - 1) / grid);
+  const size_t smem =
+      sizeof(double) * ((size_t)C::PER_CELL * cap + C::TAB + 64 + 2 * (size_t)grid);
+  if (smem > (size_t)smem_max) return PDG_OK;   // the cells do not fit on the SMs
+  const int nslots = kCg2Sets * grid * 2;
+  if (!ctx->cg2_slots) PDG_CUDA_TRY(cudaMalloc(&ctx->cg2_slots, sizeof(double) * kCg2Sets * sms * 2));
+  k_cg2d_slots<<<(nslots + 255) / 256, 256, 0, ctx->stream>>>(ctx->cg2_slots, nslots);
+  PDG_CUDA_TRY(cudaGetLastError());
+  OpParams<double> pr = make_params<double>(ctx, ctx->K64, ctx->c64, ctx->tab64);
+  const PrecData &pd = ctx->prec[PDG_F64];
+  Cg2Args g{ctx->rec64, (const double *)pd.Q, pd.Lsum_inv, x, b, {p, p2}, z, ctx->cg2_slots,
+            ctx->red_out, ctx->d_flag, maxit, cap};
+  void *args[] = {&pr, &g};
+  PDG_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_cg2d<N>, dim3(grid), dim3(kCg2Threads), args, smem,
+                                           ctx->stream));
+  *ran = true;
+  return PDG_OK;
+}
+
+// The iterations of a CG solve whose scalars are set up (first defect, rho,
+// p = M^-1 b); *ran false: not a grid for this kernel, nothing was launched.
+int cg2d_solve(pdg_context *ctx, double *x, double *b, double *p, double *p2, double *z, int maxit,
+               bool *ran) {
+  switch (ctx->N) {
+    case 2: return cg2d_n<2>(ctx, x, b, p, p2, z, maxit, ran);
+    case 3: return cg2d_n<3>(ctx, x, b, p, p2, z, maxit, ran);
+    case 4: return cg2d_n<4>(ctx, x, b, p, p2, z, maxit, ran);
+    case 5: return cg2d_n<5>(ctx, x, b, p, p2, z, maxit, ran);
+    default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
+  }
+}
+
+}  // namespace pdg

@@ -266,6 +266,9 @@ struct pdg_context {
   int fuse_fin;
   void *fuse_q;            // FIN_CG_DEF_BETA: the FDM launch first does b -= lambda q
 
+  unsigned long long *cg2_slots;   // partial sums of the one-launch 2D CG (pdg_cg2d.cu)
+  cudaEvent_t ev_poll[2];          // state copies of the CG batches in flight
+
   // staging buffers for host pointers
   double *stage_a, *stage_b;
   // host-buffer applies pipelined over slabs: copy streams and their events
@@ -398,6 +401,11 @@ int prepare_apply_m(pdg_context *ctx, int transpose);
 bool apply_i_usable(const pdg_context *ctx);
 int launch_apply_i(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<double> &p);
 int prepare_apply_i(pdg_context *ctx, int transpose);
+
+// the iterations of a small 2D FP64 CG solve in one launch (pdg_cg2d.cu); *ran
+// false: the grid does not fit, nothing was launched
+int cg2d_solve(pdg_context *ctx, double *x, double *b, double *p, double *p2, double *z, int maxit,
+               bool *ran);
 
 // parameter fields beyond A = K I: true when the Gauss-point operator replaces
 // the Kronecker kernels; its launch (diffusion and reaction terms only)
