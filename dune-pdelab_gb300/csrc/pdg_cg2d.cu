@@ -23,6 +23,12 @@
 // result everywhere, and the same in every run).  Reading a slot of block j
 // also orders the reader after everything block j wrote before, so it is the
 // barrier as well.  Waits are bounded.
+//
+// One DOF per thread: a warp-wide FP64 operation occupies its quarter of the SM
+// for 64 cycles (measured, dependent or not), so the FP64 operations of a
+// thread, not their number per cell, set the time of the two phases, and the
+// threads of a block must cover all four quarters.  With one cell per thread
+// the 2D Q1 64^2 iteration took 19.5 us.
 #include <algorithm>
 
 #include "pdg_ops.cuh"
@@ -34,8 +40,9 @@ template <int N>
 struct CG2Cfg {
   static constexpr int N2 = N * N;
   static constexpr int REC = 2 * N2 + 20;              // k_cell_record<double, 2, N>
-  // per cell in shared memory: record, Q, 1/(lx+ly), and x, r, p, q, z
-  static constexpr int PER_CELL = REC + 2 * N2 + N2 + 5 * N2;
+  // per cell in shared memory: record, Q, 1/(lx+ly); x, r, p, q, z; two
+  // exchange arrays and the face data (s1, s2 of N points of 4 faces)
+  static constexpr int PER_CELL = REC + 2 * N2 + N2 + 5 * N2 + 2 * N2 + 8 * N;
   static constexpr int TAB = N2 + 2 * N;
 };
 
@@ -59,11 +66,15 @@ struct Cg2Args {
 
 __device__ __forceinline__ unsigned long long ld_slot(const unsigned long long *p) {
   unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void st_slot(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ void st_slot_release(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // The sums of v0 (and v1, nv = 2) over the first nw warps of all blocks, in
@@ -93,10 +104,9 @@ __device__ __forceinline__ bool grid_sum(const Cg2Args &g, unsigned round, int n
     unsigned long long *old = g.slots + 2 * (size_t)((set + 2) % kCg2Sets) * nb + blockIdx.x;
     st_slot(old + k * nb, kCg2Empty);
     if (nv == 1) st_slot(old + nb, kCg2Empty);
-    __threadfence();
     const unsigned long long a = __double_as_longlong(v);
-    st_slot(g.slots + (2 * (size_t)set + k) * nb + blockIdx.x,
-            a == kCg2Empty ? 0x7ff8000000000000ull : a);
+    st_slot_release(g.slots + (2 * (size_t)set + k) * nb + blockIdx.x,
+                    a == kCg2Empty ? 0x7ff8000000000000ull : a);
   }
   bool ok = true;
   for (int i = threadIdx.x; i < nv * nb; i += kCg2Threads) {
@@ -106,7 +116,6 @@ __device__ __forceinline__ bool grid_sum(const Cg2Args &g, unsigned round, int n
     ok = ok && v != kCg2Empty;
     all[i] = __longlong_as_double(v);
   }
-  __threadfence();
   ok = __syncthreads_and(ok);
   if (w < nv) {
     double a = 0.0;
@@ -124,33 +133,29 @@ template <int N>
 __global__ void __launch_bounds__(kCg2Threads)
     k_cg2d(const OpParams<double> pr, const Cg2Args g) {
   using C = CG2Cfg<N>;
-  constexpr int N2 = C::N2;
+  constexpr int N2 = C::N2, CPP = kCg2Threads / N2;   // cells per pass
   extern __shared__ __align__(16) double sh[];
   __shared__ double sc[2];
   const int t = threadIdx.x;
   const int c0 = blockIdx.x * g.cells_per_block;
   const int c1 = min((int)pr.ncell, c0 + g.cells_per_block);
   const int nc = max(0, c1 - c0), cap = g.cells_per_block;
-  const int nw = (min(cap, kCg2Threads) + 31) / 32;
-  // arrays [entry][cell] in shared memory: one cell per thread, no conflicts
+  const int nw = (min(cap, CPP) * N2 + 31) / 32;      // warps with DOFs
+  // records and factors [cell][entry], vectors [cell][N2]
   double *rec = sh, *Q = rec + C::REC * cap, *Li = Q + 2 * N2 * cap, *X = Li + N2 * cap,
          *R = X + N2 * cap, *P = R + N2 * cap, *W = P + N2 * cap, *Z = W + N2 * cap,
-         *tM = Z + N2 * cap, *red = tM + C::TAB;
+         *T0 = Z + N2 * cap, *T1 = T0 + N2 * cap, *F = T1 + N2 * cap, *tM = F + 8 * N * cap,
+         *red = tM + C::TAB;
   const double *td0 = tM + N2, *td1 = td0 + N;
   if (g.flags[F_STATE]) return;   // converged before the first iteration
-  for (int i = t; i < nc * C::REC; i += kCg2Threads)
-    rec[(i % C::REC) * cap + i / C::REC] = g.rec[(size_t)c0 * C::REC + i];
-  for (int i = t; i < nc * 2 * N2; i += kCg2Threads)
-    Q[(i % (2 * N2)) * cap + i / (2 * N2)] = g.Q[(size_t)c0 * 2 * N2 + i];
+  for (int i = t; i < nc * C::REC; i += kCg2Threads) rec[i] = g.rec[(size_t)c0 * C::REC + i];
+  for (int i = t; i < nc * 2 * N2; i += kCg2Threads) Q[i] = g.Q[(size_t)c0 * 2 * N2 + i];
   for (int i = t; i < nc * N2; i += kCg2Threads) {
-    const int k = (i % N2) * cap + i / N2;
     const size_t o = (size_t)c0 * N2 + i;
-    Li[k] = g.Linv[o];
-    X[k] = g.x[o];
-    R[k] = g.b[o];
-    // the first direction p = M^-1 b is given in p[0]; z = 0 and beta = 1
-    // reproduce it in the first iteration
-    P[k] = g.p[0][o];
+    Li[i] = g.Linv[o];
+    X[i] = g.x[o];
+    R[i] = g.b[o];
+    P[i] = g.p[0][o];   // the first direction p = M^-1 b
   }
   for (int i = t; i < N2; i += kCg2Threads) tM[i] = pr.tab[i];
   for (int i = t; i < 2 * N; i += kCg2Threads) tM[N2 + i] = pr.tab[2 * N2 + i];
@@ -158,6 +163,7 @@ __global__ void __launch_bounds__(kCg2Threads)
   const double stop = g.scal[S_DEF0] * g.scal[S_RED];
   __syncthreads();
 
+  const int cl = t / N2, d = t - cl * N2, y = d / N, x = d - y * N;
   int state = 0, it = 0;
   unsigned round = 0;
   double lambda = 0.0;
@@ -167,83 +173,85 @@ __global__ void __launch_bounds__(kCg2Threads)
     double *pnew = g.p[(it + 1) & 1];
     const bool first = it == 0;
     double s0 = 0.0, s1 = 0.0;
-    for (int c = t; c < nc; c += kCg2Threads) {
+    for (int b = 0; b < nc; b += CPP) {
+      const int c = b + cl;
+      const bool on = cl < CPP && c < nc;
       const int e = c0 + c;
-      const int iy = e / pr.nc[0], ix = e - iy * pr.nc[0];
-      const double *rc = rec + c;   // entry k of the record: rc[k * cap]
-      double u[N][N];
+      double u = 0.0;
+      if (on) {
+        // neighbour lines: (s1, s2) of the face points, as in k_apply; one or
+        // two of the cell's 4 N lines per thread
+        const unsigned iy = pr.div0.div((unsigned)e), ix = (unsigned)e - iy * (unsigned)pr.nc[0];
 #pragma unroll
-      for (int k = 0; k < N2; k++) {
-        const double v = first ? P[k * cap + c] : fma(beta, P[k * cap + c], Z[k * cap + c]);
-        u[k / N][k % N] = v;
-        P[k * cap + c] = v;
-        __stcg(pnew + (size_t)e * N2 + k, v);
-      }
-      // neighbour lines: (s1, s2) per face point, as in k_apply
-      double f1[4][N], f2[4][N];
+        for (int l0 = 0; l0 < 4 * N; l0 += N2) {
+          const int l = l0 + d;
+          if (l < 4 * N) {
+            const int f = l / N, a = l - f * N, hi = f & 1;
+            const bool has = f == 0 ? ix > 0 : f == 1 ? (int)ix + 1 < pr.nc[0]
+                                             : f == 2 ? iy > 0 : (int)iy + 1 < pr.nc[1];
+            double f1 = 0.0, f2 = 0.0;
+            if (has) {
+              const int st = f < 2 ? 1 : pr.nc[0];
+              const size_t o = (size_t)(hi ? e + st : e - st) * N2 + (f < 2 ? a * N : a);
+              const int inc = f < 2 ? 1 : N;
+              double v[N];
 #pragma unroll
-      for (int f = 0; f < 4; f++) {
-        const int hi = f & 1;
-        const bool on = f == 0 ? ix > 0 : f == 1 ? ix + 1 < pr.nc[0] : f == 2 ? iy > 0
-                                                                              : iy + 1 < pr.nc[1];
-        const int nb = f == 0 ? e - 1 : f == 1 ? e + 1 : f == 2 ? e - pr.nc[0] : e + pr.nc[0];
-        double v[N2];
+              for (int q = 0; q < N; q++) {
+                const double po = __ldcg(pold + o + q * inc);
+                v[q] = first ? po : fma(beta, po, __ldcg(g.z + o + q * inc));
+              }
+              const double *td = hi ? td0 : td1;
+              double dv = 0.0;
 #pragma unroll
-        for (int k = 0; k < N2; k++) {
-          const size_t o = (size_t)(on ? nb : e) * N2 + k;
-          const double po = __ldcg(pold + o);
-          v[k] = first ? po : fma(beta, po, __ldcg(g.z + o));
-        }
-        // {hp ke, hp ko, hp pen, th hp ke, th hp ko} of the face
-        const double ko = rc[(2 * N2 + 5 * f + 1) * cap], pen = rc[(2 * N2 + 5 * f + 2) * cap],
-                     tke = rc[(2 * N2 + 5 * f + 3) * cap];
-#pragma unroll
-        for (int a = 0; a < N; a++) {
-          double dv = 0.0;
-#pragma unroll
-          for (int q = 0; q < N; q++)
-            dv += (hi ? td0[q] : td1[q]) * (f < 2 ? v[a * N + q] : v[q * N + a]);
-          const int qv = hi ? 0 : N - 1;
-          const double val = f < 2 ? v[a * N + qv] : v[qv * N + a];
-          f1[f][a] = on ? (hi ? -ko * dv : ko * dv) - pen * val : 0.0;
-          f2[f][a] = on ? (hi ? -tke : tke) * val : 0.0;
-        }
-      }
-      double Xp[N][N], Yp[N][N];
-#pragma unroll
-      for (int y = 0; y < N; y++)
-#pragma unroll
-        for (int x = 0; x < N; x++) {
-          double sx = 0.0, sy = 0.0;
-#pragma unroll
-          for (int q = 0; q < N; q++) {
-            sx += rc[(x * N + q) * cap] * u[y][q];
-            sy += rc[(N2 + y * N + q) * cap] * u[q][x];
+              for (int q = 0; q < N; q++) dv += td[q] * v[q];
+              const double val = hi ? v[0] : v[N - 1];
+              // {hp ke, hp ko, hp pen, th hp ke, th hp ko} of the face
+              const double *k5 = rec + c * C::REC + 2 * N2 + 5 * f;
+              const double kd = k5[1] * dv, kv = k5[3] * val;
+              f1 = (hi ? -kd : kd) - k5[2] * val;
+              f2 = hi ? -kv : kv;
+            }
+            F[c * 8 * N + l] = f1;
+            F[c * 8 * N + 4 * N + l] = f2;
           }
-          if (x == 0) sx += f1[0][y];
-          sx += td0[x] * f2[0][y];
-          if (x == N - 1) sx += f1[1][y];
-          sx += td1[x] * f2[1][y];
-          if (y == 0) sy += f1[2][x];
-          sy += td0[y] * f2[2][x];
-          if (y == N - 1) sy += f1[3][x];
-          sy += td1[y] * f2[3][x];
-          Xp[y][x] = sx;
-          Yp[y][x] = sy;
         }
+        const int i = c * N2 + d;
+        u = first ? P[i] : fma(beta, P[i], Z[i]);
+        P[i] = u;
+        __stcg(pnew + (size_t)c0 * N2 + i, u);
+      }
+      __syncthreads();
+      if (on) {
+        const double *Ax = rec + c * C::REC + x * N, *Ay = rec + c * C::REC + N2 + y * N;
+        const double *pc = P + c * N2, *f1 = F + c * 8 * N, *f2 = f1 + 4 * N;
+        double sx = 0.0, sy = 0.0;
 #pragma unroll
-      for (int y = 0; y < N; y++)
-#pragma unroll
-        for (int x = 0; x < N; x++) {
-          double s = 0.0;
-#pragma unroll
-          for (int q = 0; q < N; q++) {
-            s += tM[y * N + q] * Xp[q][x];
-            s += tM[x * N + q] * Yp[y][q];
-          }
-          W[(y * N + x) * cap + c] = s;
-          s0 += u[y][x] * s;
+        for (int q = 0; q < N; q++) {
+          sx += Ax[q] * pc[y * N + q];
+          sy += Ay[q] * pc[q * N + x];
         }
+        if (x == 0) sx += f1[y];
+        sx += td0[x] * f2[y];
+        if (x == N - 1) sx += f1[N + y];
+        sx += td1[x] * f2[N + y];
+        if (y == 0) sy += f1[2 * N + x];
+        sy += td0[y] * f2[2 * N + x];
+        if (y == N - 1) sy += f1[3 * N + x];
+        sy += td1[y] * f2[3 * N + x];
+        T0[c * N2 + d] = sx;
+        T1[c * N2 + d] = sy;
+      }
+      __syncthreads();
+      if (on) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+          s += tM[y * N + q] * T0[c * N2 + q * N + x];
+          s += tM[x * N + q] * T1[c * N2 + y * N + q];
+        }
+        W[c * N2 + d] = s;
+        s0 += u * s;
+      }
     }
     if (!grid_sum(g, round++, 1, nw, s0, s1, red)) {
       state = -1;
@@ -255,67 +263,55 @@ __global__ void __launch_bounds__(kCg2Threads)
     it++;
     // ---- x += lambda p, r -= lambda q, z = M^-1 r ----
     s0 = s1 = 0.0;
-    for (int c = t; c < nc; c += kCg2Threads) {
-      const int e = c0 + c;
-      double r[N][N], a[N][N];
-#pragma unroll
-      for (int k = 0; k < N2; k++) {
-        const int i = k * cap + c;
+    for (int b = 0; b < nc; b += CPP) {
+      const int c = b + cl, i = c * N2 + d;
+      const bool on = cl < CPP && c < nc;
+      const double *Qx = Q + c * 2 * N2, *Qy = Qx + N2, *t0 = T0 + c * N2, *t1 = T1 + c * N2;
+      double r = 0.0;
+      if (on) {
+        r = R[i] - lambda * W[i];
+        R[i] = r;
         X[i] += lambda * P[i];
-        const double v = R[i] - lambda * W[i];
-        R[i] = v;
-        r[k / N][k % N] = v;
-        s0 += v * v;
+        s0 += r * r;
       }
-      const double *Qx = Q + c, *Qy = Qx + N2 * cap;   // entry [i][j]: Qx[(i N + j) cap]
-      double w[N][N];
+      __syncthreads();
+      if (on) {
+        double s = 0.0;
 #pragma unroll
-      for (int yp = 0; yp < N; yp++)
+        for (int k = 0; k < N; k++) s += Qy[k * N + y] * R[c * N2 + k * N + x];
+        T0[i] = s;
+      }
+      __syncthreads();
+      if (on) {
+        double s = 0.0;
 #pragma unroll
-        for (int x = 0; x < N; x++) {
-          double s = 0.0;
+        for (int k = 0; k < N; k++) s += Qx[k * N + x] * t0[y * N + k];
+        T1[i] = s * Li[i];
+      }
+      __syncthreads();
+      if (on) {
+        double s = 0.0;
 #pragma unroll
-          for (int y = 0; y < N; y++) s += Qy[(y * N + yp) * cap] * r[y][x];
-          w[yp][x] = s;
-        }
+        for (int k = 0; k < N; k++) s += Qx[x * N + k] * t1[y * N + k];
+        T0[i] = s;
+      }
+      __syncthreads();
+      if (on) {
+        double s = 0.0;
 #pragma unroll
-      for (int y = 0; y < N; y++)
-#pragma unroll
-        for (int xp = 0; xp < N; xp++) {
-          double s = 0.0;
-#pragma unroll
-          for (int x = 0; x < N; x++) s += Qx[(x * N + xp) * cap] * w[y][x];
-          a[y][xp] = s * Li[(y * N + xp) * cap + c];
-        }
-#pragma unroll
-      for (int y = 0; y < N; y++)
-#pragma unroll
-        for (int x = 0; x < N; x++) {
-          double s = 0.0;
-#pragma unroll
-          for (int xp = 0; xp < N; xp++) s += Qx[(x * N + xp) * cap] * a[y][xp];
-          w[y][x] = s;
-        }
-#pragma unroll
-      for (int y = 0; y < N; y++)
-#pragma unroll
-        for (int x = 0; x < N; x++) {
-          double s = 0.0;
-#pragma unroll
-          for (int yp = 0; yp < N; yp++) s += Qy[(y * N + yp) * cap] * w[yp][x];
-          Z[(y * N + x) * cap + c] = s;
-          __stcg(g.z + (size_t)e * N2 + y * N + x, s);
-          s1 += r[y][x] * s;
-        }
+        for (int k = 0; k < N; k++) s += Qy[y * N + k] * t0[k * N + x];
+        Z[i] = s;
+        __stcg(g.z + (size_t)c0 * N2 + i, s);
+        s1 += r * s;
+      }
     }
     if (!grid_sum(g, round++, 2, nw, s0, s1, red)) {
       state = -1;
       break;
     }
-    if (t == 0) {
-      sc[0] = sqrt(s0);
-      sc[1] = s1 / rho;
-    }
+    // two warps: the square root and the quotient at the same time
+    if (t == 0) sc[0] = sqrt(s0);
+    if (t == 32) sc[1] = s1 / rho;
     __syncthreads();
     def = sc[0];
     beta = sc[1];
@@ -324,10 +320,9 @@ __global__ void __launch_bounds__(kCg2Threads)
     else if (def < stop || def < 1e-30) state = 1;
   }
   for (int i = t; i < nc * N2; i += kCg2Threads) {
-    const int k = (i % N2) * cap + i / N2;
     const size_t o = (size_t)c0 * N2 + i;
-    g.x[o] = X[k];
-    g.b[o] = R[k];
+    g.x[o] = X[i];
+    g.b[o] = R[i];
   }
   if (blockIdx.x == 0 && t == 0) {
     g.scal[S_DEF] = def;
