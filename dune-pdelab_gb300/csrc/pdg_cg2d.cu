@@ -18,11 +18,13 @@
 //   previous p), q = A p                                 -- sum <p, q>
 //   x += lambda p, r -= lambda q, z = M^-1 r              -- sums <r, r>, <z, r>
 //
-// A grid-wide sum is one exchange: each block publishes its partial sums in its
-// slot and all blocks read all slots, adding them in block order (the same
-// result everywhere, and the same in every run).  Reading a slot of block j
-// also orders the reader after everything block j wrote before, so it is the
-// barrier as well.  Waits are bounded.
+// A grid-wide sum is two hops: each block publishes its partial sums in its
+// slot; block 0 reads the slots, adds them in block order (the same result in
+// every run), forms the scalars of the recurrence and publishes those.  Slots
+// are released and acquired, so having read the scalars a block is also ordered
+// after everything the other blocks wrote before: it is the barrier as well.
+// (With every block reading every slot the polling itself took 4 to 5 us.)
+// Waits are bounded.
 //
 // One DOF per thread: a warp-wide FP64 operation occupies its quarter of the SM
 // for 64 cycles (measured, dependent or not), so the FP64 operations of a
@@ -47,9 +49,10 @@ struct CG2Cfg {
 };
 
 constexpr int kCg2Sets = 4;              // slot sets in use in turn
-// threads per block: one for each of the 2 x 152 slots a block polls, so that
-// an exchange is one L2 round trip; cells go to the first threads
+// threads per block: one for each of the 2 x 152 slots block 0 polls, so that
+// a hop is one L2 round trip; cells go to the first threads
 constexpr int kCg2Threads = 320;
+constexpr int kCg2Copies = 8;            // copies of the scalars, 128 bytes apart
 constexpr int kCg2Polls = 1 << 21;       // bound of one wait (seconds)
 // an empty slot: a NaN no arithmetic produces
 constexpr unsigned long long kCg2Empty = 0xffffffffffffffffull;
@@ -58,7 +61,8 @@ struct Cg2Args {
   const double *rec, *Q, *Linv;
   double *x, *b;          // solution and defect (both updated)
   double *p[2], *z;       // exchanged vectors
-  unsigned long long *slots;   // [kCg2Sets][2][grid], all empty
+  unsigned long long *slots;   // [kCg2Sets][2][grid] partial sums, all empty,
+  unsigned long long *result;  // [kCg2Sets][kCg2Copies][16] scalars, all empty
   double *scal;
   int *flags;
   int maxit, cells_per_block;
@@ -77,14 +81,30 @@ __device__ __forceinline__ void st_slot_release(unsigned long long *p, unsigned 
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// The sums of v0 (and v1, nv = 2) over the first nw warps of all blocks, in
-// every thread; the round number picks the slot set.  false: a block did not
-// publish in time.  red: shared scratch of 2 * 32 + 2 * gridDim doubles.
-__device__ __forceinline__ bool grid_sum(const Cg2Args &g, unsigned round, int nv, int nw,
-                                         double &v0, double &v1, double *red) {
+// One value read from / written to a slot; an empty slot is never written
+__device__ __forceinline__ bool take_slot(const unsigned long long *s, double *v) {
+  unsigned long long x = ld_slot(s);
+  for (int it = 0; x == kCg2Empty && it < kCg2Polls; it++) x = ld_slot(s);
+  *v = __longlong_as_double(x);
+  return x != kCg2Empty;
+}
+__device__ __forceinline__ void put_slot(unsigned long long *s, double v) {
+  const unsigned long long x = __double_as_longlong(v);
+  st_slot_release(s, x == kCg2Empty ? 0x7ff8000000000000ull : x);
+}
+
+// The exchange of one round: sums v0 (and v1, nv = 2) over the first nw warps of
+// all blocks; block 0 turns them into nr scalars with `scalars(s, out)`, called
+// by its threads 0, 32, .. 32 (nr - 1) (scalar k by thread 32 k); every thread
+// gets them in res[0 .. nr).  false: a block or block 0 did not publish in time.
+// red: shared scratch of 64 + 2 * gridDim doubles.
+template <class F>
+__device__ __forceinline__ bool exchange(const Cg2Args &g, unsigned round, int nv, int nr, int nw,
+                                         double v0, double v1, double *red, double *res,
+                                         F scalars) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nb = gridDim.x;
-  double *all = red + 64;
+  const unsigned set = round % kCg2Sets, old = (set + 2) % kCg2Sets;
   if (w < nw) {
     v0 = warp_sum_d(v0);
     if (nv > 1) v1 = warp_sum_d(v1);
@@ -93,40 +113,47 @@ __device__ __forceinline__ bool grid_sum(const Cg2Args &g, unsigned round, int n
       red[2 * w + 1] = v1;
     }
   }
-  __syncthreads();   // every thread's global writes come before the fence below
-  const unsigned set = round % kCg2Sets;
-  if (threadIdx.x < nv) {
+  __syncthreads();   // every thread's global writes come before the release below
+  if (threadIdx.x < 2) {
     const int k = threadIdx.x;
-    double v = red[k];
-    for (int i = 1; i < nw; i++) v += red[2 * i + k];
-    // free the own slots of the set after next: all blocks have read them (they
-    // published the previous round after that)
-    unsigned long long *old = g.slots + 2 * (size_t)((set + 2) % kCg2Sets) * nb + blockIdx.x;
-    st_slot(old + k * nb, kCg2Empty);
-    if (nv == 1) st_slot(old + nb, kCg2Empty);
-    const unsigned long long a = __double_as_longlong(v);
-    st_slot_release(g.slots + (2 * (size_t)set + k) * nb + blockIdx.x,
-                    a == kCg2Empty ? 0x7ff8000000000000ull : a);
+    // free the own slots of the set after next: block 0 has read them (it
+    // published the previous round's scalars after that)
+    st_slot(g.slots + (2 * (size_t)old + k) * nb + blockIdx.x, kCg2Empty);
+    if (k < nv) {
+      double v = red[k];
+      for (int i = 1; i < nw; i++) v += red[2 * i + k];
+      put_slot(g.slots + (2 * (size_t)set + k) * nb + blockIdx.x, v);
+    }
   }
   bool ok = true;
-  for (int i = threadIdx.x; i < nv * nb; i += kCg2Threads) {
-    const unsigned long long *s = g.slots + 2 * (size_t)set * nb + i;
-    unsigned long long v = ld_slot(s);
-    for (int it = 0; v == kCg2Empty && it < kCg2Polls; it++) v = ld_slot(s);
-    ok = ok && v != kCg2Empty;
-    all[i] = __longlong_as_double(v);
+  if (blockIdx.x == 0) {
+    double *all = red + 64;
+    for (int i = threadIdx.x; i < nv * nb; i += kCg2Threads)
+      ok = take_slot(g.slots + 2 * (size_t)set * nb + i, all + i) && ok;
+    ok = __syncthreads_and(ok);
+    if (w < nv) {
+      double a = 0.0;
+      for (int i = lane; i < nb; i += 32) a += all[w * nb + i];
+      a = warp_sum_d(a);
+      if (lane == 0) red[60 + w] = a;
+    }
+    __syncthreads();
+    if (lane == 0 && w < nr) res[w] = scalars(w, red[60], red[61]);
+    __syncthreads();
+    if (threadIdx.x < nr * kCg2Copies) {
+      const int k = threadIdx.x % nr, c = threadIdx.x / nr;
+      // all blocks have read the scalars of the round before last
+      for (int j = k; j < 4; j += nr)
+        st_slot(g.result + 16 * ((size_t)old * kCg2Copies + c) + j, kCg2Empty);
+      // a failed wait is not published: every block then runs out as well
+      if (ok) put_slot(g.result + 16 * ((size_t)set * kCg2Copies + c) + k, res[k]);
+    }
+  } else if (threadIdx.x < nr) {
+    ok = take_slot(g.result + 16 * ((size_t)set * kCg2Copies + blockIdx.x % kCg2Copies) +
+                       threadIdx.x,
+                   res + threadIdx.x);
   }
-  ok = __syncthreads_and(ok);
-  if (w < nv) {
-    double a = 0.0;
-    for (int i = lane; i < nb; i += 32) a += all[w * nb + i];
-    a = warp_sum_d(a);
-    if (lane == 0) red[62 + w] = a;
-  }
-  __syncthreads();
-  v0 = red[62];
-  if (nv > 1) v1 = red[63];
-  return ok;
+  return __syncthreads_and(ok);
 }
 
 template <int N>
@@ -135,7 +162,7 @@ __global__ void __launch_bounds__(kCg2Threads)
   using C = CG2Cfg<N>;
   constexpr int N2 = C::N2, CPP = kCg2Threads / N2;   // cells per pass
   extern __shared__ __align__(16) double sh[];
-  __shared__ double sc[2];
+  __shared__ double sc[4];
   const int t = threadIdx.x;
   const int c0 = blockIdx.x * g.cells_per_block;
   const int c1 = min((int)pr.ncell, c0 + g.cells_per_block);
@@ -253,12 +280,11 @@ __global__ void __launch_bounds__(kCg2Threads)
         s0 += u * s;
       }
     }
-    if (!grid_sum(g, round++, 1, nw, s0, s1, red)) {
+    if (!exchange(g, round++, 1, 1, nw, s0, 0.0, red, sc,
+                  [&](int, double a, double) { return rho / a; })) {
       state = -1;
       break;
     }
-    if (t == 0) sc[0] = rho / s0;
-    __syncthreads();
     lambda = sc[0];
     it++;
     // ---- x += lambda p, r -= lambda q, z = M^-1 r ----
@@ -305,17 +331,16 @@ __global__ void __launch_bounds__(kCg2Threads)
         s1 += r * s;
       }
     }
-    if (!grid_sum(g, round++, 2, nw, s0, s1, red)) {
+    // def = |r|, beta = <z, r> / rho, rho = <z, r>
+    if (!exchange(g, round++, 2, 3, nw, s0, s1, red, sc, [&](int k, double a, double c) {
+          return k == 0 ? sqrt(a) : k == 1 ? c / rho : c;
+        })) {
       state = -1;
       break;
     }
-    // two warps: the square root and the quotient at the same time
-    if (t == 0) sc[0] = sqrt(s0);
-    if (t == 32) sc[1] = s1 / rho;
-    __syncthreads();
     def = sc[0];
     beta = sc[1];
-    rho = s1;
+    rho = sc[2];
     if (!isfinite(def)) state = 2;
     else if (def < stop || def < 1e-30) state = 1;
   }
@@ -364,14 +389,16 @@ static int cg2d_n(pdg_context *ctx, double *x, double *b, double *p, double *p2,
   const size_t smem =
       sizeof(double) * ((size_t)C::PER_CELL * cap + C::TAB + 64 + 2 * (size_t)grid);
   if (smem > (size_t)smem_max) return PDG_OK;   // the cells do not fit on the SMs
-  const int nslots = kCg2Sets * grid * 2;
-  if (!ctx->cg2_slots) PDG_CUDA_TRY(cudaMalloc(&ctx->cg2_slots, sizeof(double) * kCg2Sets * sms * 2));
+  const int npart = kCg2Sets * grid * 2, nslots = npart + kCg2Sets * kCg2Copies * 16;
+  if (!ctx->cg2_slots)
+    PDG_CUDA_TRY(cudaMalloc(&ctx->cg2_slots,
+                            sizeof(double) * kCg2Sets * (sms * 2 + kCg2Copies * 16)));
   k_cg2d_slots<<<(nslots + 255) / 256, 256, 0, ctx->stream>>>(ctx->cg2_slots, nslots);
   PDG_CUDA_TRY(cudaGetLastError());
   OpParams<double> pr = make_params<double>(ctx, ctx->K64, ctx->c64, ctx->tab64);
   const PrecData &pd = ctx->prec[PDG_F64];
   Cg2Args g{ctx->rec64, (const double *)pd.Q, pd.Lsum_inv, x, b, {p, p2}, z, ctx->cg2_slots,
-            ctx->red_out, ctx->d_flag, maxit, cap};
+            ctx->cg2_slots + npart, ctx->red_out, ctx->d_flag, maxit, cap};
   void *args[] = {&pr, &g};
   PDG_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_cg2d<N>, dim3(grid), dim3(kCg2Threads), args, smem,
                                            ctx->stream));
