@@ -956,7 +956,18 @@ using namespace pdg;
   do {                                                                         \
     if (!(ctx)) return set_error(PDG_EINVAL, "null context");                 \
     PDG_CUDA_TRY(cudaSetDevice((ctx)->device));                                \
+    if (!(ctx)->run_active) PDG_TRY(own_stream_entry(ctx));                    \
   } while (0)
+
+// a call on the context's own (or bound) stream follows the calls that ran on
+// callers' streams
+static int own_stream_entry(pdg_context *ctx) {
+  ctx->own_dirty = 1;
+  if (!ctx->own_must_wait) return PDG_OK;
+  ctx->own_must_wait = 0;
+  PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->ev_run, 0));
+  return PDG_OK;
+}
 
 extern "C" {
 
@@ -1111,7 +1122,7 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
   std::vector<double> ones(c->ncell, 1.0);
   std::vector<float> ones32(c->ncell, 1.0f);
   if (cudaMalloc(&c->tab64, sizeof(double) * tab.size()) != cudaSuccess ||
-      cudaMalloc(&c->tab32, sizeof(float) * tab.size()) != cudaSuccess ||
+      cudaMalloc(&c->tab32, sizeof(float) * (tab.size() + 3 * N * N + 4 * N)) != cudaSuccess ||
       cudaMalloc(&c->K64, sizeof(double) * c->ncell) != cudaSuccess ||
       cudaMalloc(&c->K32, sizeof(float) * c->ncell) != cudaSuccess ||
       cudaMalloc(&c->r0, sizeof(double) * c->ndof) != cudaSuccess ||
@@ -1164,9 +1175,6 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
       tm[N * N + 2 * N + i] = md0;
       tm[N * N + 3 * N + i] = md1;
     }
-    if (cudaMalloc(&c->tabm64, sizeof(double) * tm.size()) != cudaSuccess)
-      return fail(set_error(PDG_ECUDA, "device allocation failed"));
-    cudaMemcpy(c->tabm64, tm.data(), sizeof(double) * tm.size(), cudaMemcpyHostToDevice);
     // the per-cell tensor operator's tables: M, the nodal differentiation
     // matrix Dn, L = M^-1 Dn^T M = m_1 e_{N-1}^T - m_0 e_0^T - Dn (integration
     // by parts), m_0, m_1 and the derivatives of the basis at the ends
@@ -1185,14 +1193,17 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
       tt[3 * N * N + 2 * N + i] = t.d0[i];
       tt[3 * N * N + 3 * N + i] = t.d1[i];
     }
-    const std::vector<float> tt32(tt.begin(), tt.end());
-    if (cudaMalloc(&c->tabt64, sizeof(double) * tt.size()) != cudaSuccess ||
-        cudaMalloc(&c->tabt32, sizeof(float) * tt.size()) != cudaSuccess)
+    // both table sets in one allocation (FP32: behind tab32)
+    const size_t nm = tm.size();
+    tm.insert(tm.end(), tt.begin(), tt.end());
+    if (cudaMalloc(&c->tabm64, sizeof(double) * tm.size()) != cudaSuccess)
       return fail(set_error(PDG_ECUDA, "device allocation failed"));
-    cudaMemcpy(c->tabt64, tt.data(), sizeof(double) * tt.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(c->tabt32, tt32.data(), sizeof(float) * tt.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(c->tabm64, tm.data(), sizeof(double) * tm.size(), cudaMemcpyHostToDevice);
+    c->tabt64 = c->tabm64 + nm;
+    tab32.insert(tab32.end(), tt.begin(), tt.end());
+    c->tabt32 = c->tab32 + tab.size();
   }
-  cudaMemcpy(c->tab32, tab32.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(c->tab32, tab32.data(), sizeof(float) * tab32.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(c->K64, ones.data(), sizeof(double) * c->ncell, cudaMemcpyHostToDevice);
   cudaMemcpy(c->K32, ones32.data(), sizeof(float) * c->ncell, cudaMemcpyHostToDevice);
   cudaMemset(c->d_flag, 0, sizeof(int) * F_COUNT);
@@ -1221,6 +1232,9 @@ int pdg_destroy(pdg_context *c) {
   if (!c) return PDG_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
+  if (c->run_pending) cudaEventSynchronize(c->ev_run);
+  if (c->ev_run) cudaEventDestroy(c->ev_run);
+  if (c->ev_own) cudaEventDestroy(c->ev_own);
   if (c->pipe_h2d) {
     cudaStreamSynchronize(c->pipe_h2d);
     cudaStreamSynchronize(c->pipe_d2h);
@@ -1239,7 +1253,7 @@ int pdg_destroy(pdg_context *c) {
                   c->fuse_part, c->fuse_cnt, c->Ac64, c->Aqv64, c->Aqf64, c->cq64, c->Ac32,
                   c->Aqv32, c->Aqf32, c->cq32, c->bqv64, c->bqf64, c->Kd64, c->Kd32,
                   c->recfp, c->tabfp, c->rec32q, c->rec32c, c->rec64m, c->rec64mT, c->tabm64,
-                  c->tabt64, c->tabt32, c->cg2_slots, c->reci, c->reciT, c->reci_exp, c->reciT_exp};
+                  c->cg2_slots, c->reci, c->reciT, c->reci_exp, c->reciT_exp};
   for (void *b : bufs)
     if (b) cudaFree(b);
   for (int i = 0; i < 10; i++)
@@ -1265,10 +1279,52 @@ int pdg_destroy(pdg_context *c) {
 
 int pdg_set_stream(pdg_context *ctx, void *stream) {
   PDG_CHECK_CTX(ctx);
+  if (ctx->run_active) return set_error(PDG_ESTATE, "pdg_set_stream inside pdg_run_on");
   ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;
   return PDG_OK;
 }
 
+int pdg_run_on(pdg_context *ctx, void *stream) {
+  if (!ctx) return set_error(PDG_EINVAL, "null context");
+  if (ctx->run_active || ctx->stream != ctx->own_stream)
+    return set_error(PDG_ESTATE, "pdg_run_on needs the context on its own stream");
+  PDG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    cs = cudaStreamCaptureStatusNone;
+  }
+  // a capture cannot wait for work outside it (nor record its end for it): the
+  // graph's launches are ordered by the caller
+  ctx->run_capturing = cs != cudaStreamCaptureStatusNone;
+  if (!ctx->run_capturing) {
+    if (!ctx->ev_run) {
+      PDG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ev_run, cudaEventDisableTiming));
+      PDG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ev_own, cudaEventDisableTiming));
+    }
+    if (ctx->own_dirty) {
+      PDG_CUDA_TRY(cudaEventRecord(ctx->ev_own, ctx->own_stream));
+      PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_own, 0));
+      ctx->own_dirty = 0;
+    }
+    if (ctx->run_pending) PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_run, 0));
+  }
+  ctx->stream = s;
+  ctx->run_active = 1;
+  return PDG_OK;
+}
+int pdg_run_done(pdg_context *ctx) {
+  if (!ctx) return set_error(PDG_EINVAL, "null context");
+  if (!ctx->run_active) return set_error(PDG_ESTATE, "pdg_run_done without pdg_run_on");
+  const cudaStream_t s = ctx->stream;
+  ctx->stream = ctx->own_stream;
+  ctx->run_active = 0;
+  if (ctx->run_capturing) return PDG_OK;
+  PDG_CUDA_TRY(cudaEventRecord(ctx->ev_run, s));
+  ctx->run_pending = ctx->own_must_wait = 1;
+  return PDG_OK;
+}
 int pdg_get_stream(const pdg_context *ctx, void **stream) {
   if (!ctx || !stream) return set_error(PDG_EINVAL, "null argument");
   *stream = (void *)ctx->stream;

@@ -135,6 +135,10 @@ struct pdg_context {
   double theta, pen_fac;
   cudaStream_t stream;
   cudaStream_t own_stream;
+  // calls run on a caller's stream (pdg_run_on): ev_run marks the end of the
+  // last such call, ev_own the own stream's work before it
+  cudaEvent_t ev_run, ev_own;
+  int run_active, run_capturing, run_pending, own_must_wait, own_dirty;
   int device;
 
   // coefficients on the device

@@ -127,6 +127,8 @@ _SIGS = {
     "pdg_default_solver_options": (None, [C.POINTER(SolverOptions)]),
     "pdg_set_stream": (C.c_int, [_vp, _vp]),
     "pdg_get_stream": (C.c_int, [_vp, C.POINTER(_vp)]),
+    "pdg_run_on": (C.c_int, [_vp, _vp]),
+    "pdg_run_done": (C.c_int, [_vp]),
     "pdg_sizes": (C.c_int, [_vp, C.POINTER(C.c_long), C.POINTER(C.c_int), C.POINTER(C.c_long),
                             C.POINTER(C.c_int), C.POINTER(C.c_long)]),
     "pdg_volume_points": (C.c_int, [_vp, _vp]),
@@ -243,6 +245,33 @@ def _stream_ordered(method):
     return wrapper
 
 
+def _on_current_stream(method):
+    """Run a single operation on torch's current stream itself: its work stands
+    between torch's own there, and the library orders it against the context's
+    other work (pdg_run_on).  Host vectors take the events of
+    ``_stream_ordered``; so does everything that replays CUDA graphs."""
+    ordered = _stream_ordered(method)
+
+    @functools.wraps(method)
+    def wrapper(self, *args, **kw):
+        go = getattr(self, "go", self)
+        torch = sys.modules.get("torch")
+        if (torch is None or go._explicit_stream or not go._h or go._running
+                or not torch.cuda.is_initialized()):
+            return method(self, *args, **kw)
+        if kw or any(isinstance(a, np.ndarray) for a in args):
+            return ordered(self, *args, **kw)
+        lib = load()
+        _check(lib.pdg_run_on(go._h, torch.cuda.current_stream(go.cfg.device).cuda_stream))
+        go._running = True
+        try:
+            return method(self, *args)
+        finally:
+            go._running = False
+            _check(lib.pdg_run_done(go._h))
+    return wrapper
+
+
 def _ptr(v, dtype=np.float64):
     """Raw address of a numpy array or torch tensor (contiguous, right dtype)."""
     if v is None:
@@ -326,6 +355,7 @@ class GridOperator:
         self.cfg = cfg
         self.dim, self.degree, self.basis = dim, degree, basis
         self._explicit_stream = False
+        self._running = False        # inside a call on torch's current stream
         self._lib_stream = None
         self._h = _vp()
         _check(load().pdg_create(C.byref(cfg), C.byref(self._h)))
@@ -448,38 +478,38 @@ class GridOperator:
         _check(load().pdg_set_boundary_data(self._h, *[_ptr(a) for a in arrs]))
 
     # -- GridOperator -----------------------------------------------------
-    @_stream_ordered
+    @_on_current_stream
     def residual(self, x, r):
         """r += R(x)"""
         _check(load().pdg_residual(self._h, _ptr(x), _ptr(r)))
         return r
 
-    @_stream_ordered
+    @_on_current_stream
     def jacobian_apply(self, z, y):
         """y += J z"""
         _check(load().pdg_jacobian_apply(self._h, _ptr(z), _ptr(y)))
         return y
 
-    @_stream_ordered
+    @_on_current_stream
     def jacobian_apply_f32(self, z, y):
         """y += J z in FP32 (device tensors)"""
         _check(load().pdg_jacobian_apply_f32(self._h, _ptr(z, np.float32), _ptr(y, np.float32)))
         return y
 
-    @_stream_ordered
+    @_on_current_stream
     def apply_f32(self, x, y):
         """y = J x in FP32 (device tensors)"""
         _check(load().pdg_apply_f32(self._h, _ptr(x, np.float32), _ptr(y, np.float32)))
         return y
 
-    @_stream_ordered
+    @_on_current_stream
     def jacobian_apply_transpose_f32(self, z, y):
         """y += J^T z in FP32 (device tensors)"""
         _check(load().pdg_jacobian_apply_transpose_f32(self._h, _ptr(z, np.float32),
                                                        _ptr(y, np.float32)))
         return y
 
-    @_stream_ordered
+    @_on_current_stream
     def jacobian_apply_transpose(self, z, y):
         """y += J^T z"""
         _check(load().pdg_jacobian_apply_transpose(self._h, _ptr(z), _ptr(y)))
@@ -558,7 +588,7 @@ class GridOperator:
         _check(load().pdg_matrix_apply(self._h, _ptr(x), _ptr(y)))
         return y
 
-    @_stream_ordered
+    @_on_current_stream
     def mass_apply(self, x, y):
         """y = M x (DG mass matrix)"""
         _check(load().pdg_mass_apply(self._h, _ptr(x), _ptr(y)))
@@ -587,12 +617,12 @@ class OnTheFlyOperator:
     def __init__(self, go: GridOperator):
         self.go = go
 
-    @_stream_ordered
+    @_on_current_stream
     def apply(self, x, y):
         """y = J x"""
         _check(load().pdg_apply(self.go.handle, _ptr(x), _ptr(y)))
 
-    @_stream_ordered
+    @_on_current_stream
     def applyscaleadd(self, alpha, x, y):
         """y += alpha J x"""
         _check(load().pdg_applyscaleadd(self.go.handle, float(alpha), _ptr(x), _ptr(y)))
@@ -615,8 +645,19 @@ class GridOperatorPreconditioner:
             _check(load().pdg_prec_setup(self.go.handle, self.kind, self.precision))
             self._ready = True
 
-    @_stream_ordered
     def apply(self, v, d):
+        # a SOR sweep replays a CUDA graph
+        (self._apply_own if self.kind & PREC_SOR else self._apply_current)(v, d)
+
+    @_stream_ordered
+    def _apply_own(self, v, d):
+        self._apply(v, d)
+
+    @_on_current_stream
+    def _apply_current(self, v, d):
+        self._apply(v, d)
+
+    def _apply(self, v, d):
         if self.precision == F64:
             _check(load().pdg_prec_apply(self.go.handle, _ptr(d), _ptr(v)))
         else:

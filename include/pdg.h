@@ -205,6 +205,17 @@ void pdg_default_solver_options(pdg_solver_options *opt);
    reference runs on the host). */
 int pdg_set_stream(pdg_context *ctx, void *stream);
 
+/* The calls from pdg_run_on to pdg_run_done run on `stream` (cudaStream_t as
+   void*; NULL = the legacy default stream) instead of the context's own stream:
+   ordered after the context's earlier work, and before its later work, on
+   whatever stream that runs.  For single operations between a caller's own
+   work on that stream; a solve replays CUDA graphs on the context's stream and
+   should run there.  PDG_ESTATE while a stream is bound by pdg_set_stream, or
+   nested.  A stream in capture is not ordered against work outside the
+   capture.  No reference counterpart. */
+int pdg_run_on(pdg_context *ctx, void *stream);
+int pdg_run_done(pdg_context *ctx);
+
 /* The stream the context currently works on (the one set by pdg_set_stream,
    else its own).  No reference counterpart: a caller on another stream
    (a framework's current stream) orders its own work against this one with
