@@ -196,6 +196,9 @@ struct pdg_context {
   double *bqv64, *bqf64;
   double *conv64;      // per-cell weighted velocity at volume and face points (FP64)
   float *conv32;       // the same in FP32
+  // limb tables of B and D, their exponents and the cells' (pdg_conv_i.cu)
+  int2 *convtabi;
+  int *convexps, conv_exp[5];
   double *convtab64;   // B and D (basis values / derivatives at Gauss points)
   float *convtab32;
   // GMRES Krylov bases (m+1 vectors), the FP64 flexible-GMRES basis of the
@@ -435,5 +438,9 @@ inline bool convection_on(const pdg_context *ctx) {
 int conv_setup(pdg_context *ctx);
 template <typename T>
 int launch_convection(pdg_context *ctx, const ApplyArgs<T> &a);
+// the FP64 convection apply (not transposed, all cells or a range) in 64-bit
+// fixed point, and its set-up from the FP64 tables (B, D) and records
+int conv_setup_i(pdg_context *ctx, const double *tab);
+int launch_conv_i(pdg_context *ctx, const ApplyArgs<double> &a);
 
 }  // namespace pdg

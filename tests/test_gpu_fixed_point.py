@@ -156,3 +156,56 @@ def test_fdm_extremes():
     assert np.isnan(v[hit]).all()
     assert np.max(np.abs(v[~hit] - ref[~hit])) <= 1e-13 * np.max(np.abs(ref))
     go.close()
+
+
+def convection(k, n, seed=9, sigma=1.0, **kw):
+    go, P, rng = problem(k, n, seed=seed, sigma=sigma, **kw)
+    modes = pdg.fourier_velocity_modes(seed)
+    go.set_velocity_modes(modes)
+    P.set_modes(modes)
+    return go, P, rng
+
+
+# cells per block: 32 (k=1), 14, 8, 5 (k=4)
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [(1, 1, 1), (15, 1, 1), (3, 11, 1), (4, 3, 5)])
+@pytest.mark.parametrize("basis", [0, 2])
+def test_convection_sizes(k, n, basis):
+    """Equidistant and Gauss-Lobatto nodes: the 1D tables' scaling differs."""
+    kw = dict(basis=basis) if basis else {}
+    go, P, rng = convection(k, n, **kw)
+    x = rng.uniform(-1, 1, go.ndof)
+    assert rel(apply(go, x), P.jacobian_apply(x)) <= 1e-12
+    go.close()
+
+
+@pytest.mark.parametrize("k", [1, 2, 4])
+def test_convection_wide_ranges(k):
+    """K of 1e-12 leaves convection alone: a cell's result follows its own
+    values and its upwind neighbours', however large the others are."""
+    go, P, rng = convection(k, (5, 4, 3), scale=1e-12, sigma=0.1)
+    x = rng.uniform(-1, 1, (go.ncell, go.nbasis)) * 10.0 ** rng.uniform(-3, 3, (go.ncell, 1))
+    y = apply(go, x.ravel()).reshape(go.ncell, -1)
+    ref = P.jacobian_apply(x.ravel()).reshape(go.ncell, -1)
+    for e in range(go.ncell):
+        assert np.max(np.abs(y[e] - ref[e])) <= 1e-12 * np.max(np.abs(ref[e])), e
+    for f in (1e-280, 1e270):
+        assert rel(apply(go, x.ravel() * f) / f, ref.ravel()) <= 1e-12
+    go.close()
+
+
+def test_convection_non_finite():
+    n = (7, 4, 3)
+    go, P, rng = convection(2, n)
+    x = rng.uniform(-1, 1, go.ndof)
+    ref = P.jacobian_apply(x).reshape(go.ncell, -1)
+    e = 2 + 7 * (1 + 4 * 1)
+    x[e * go.nbasis:(e + 1) * go.nbasis] = np.nan
+    y = apply(go, x).reshape(go.ncell, -1)
+    hit = {e, e - 1, e + 1, e - 7, e + 7, e - 28, e + 28}
+    for c in range(go.ncell):
+        if c in hit:
+            assert not np.isfinite(y[c]).any()
+        else:
+            assert np.max(np.abs(y[c] - ref[c])) <= 1e-12 * np.max(np.abs(ref))
+    go.close()
