@@ -355,8 +355,8 @@ static bool cg_fusable64(const pdg_context *ctx, int transpose) {
 
 static int ensure_fuse(pdg_context *ctx) {
   if (ctx->fuse_part) return PDG_OK;
-  // the fused kernels run at least 5 cells per block
-  const long maxb = ctx->ncell / 5 + 2;
+  // the fused kernels run at least 4 cells per block
+  const long maxb = ctx->ncell / 4 + 2;
   const long ngroups = (maxb + kFuseGroup - 1) / kFuseGroup;
   PDG_CUDA_TRY(cudaMalloc(&ctx->fuse_part, sizeof(double) * 2 * (maxb + ngroups)));
   PDG_CUDA_TRY(cudaMalloc(&ctx->fuse_cnt, sizeof(int) * ngroups));

@@ -32,7 +32,7 @@ namespace pdg {
 template <int N>
 struct ICfg {
   static constexpr int N2 = N * N, NB = N * N * N, TPC = N * N, NF = 6;
-  static constexpr int CPB = (128 / TPC) > 0 ? (128 / TPC) : 1;
+  static constexpr int CPB = (N == 4 ? 64 : 128) / TPC;   // 32, 14, 4, 5 cells
   static constexpr int THREADS = CPB * TPC;
   static constexpr int NW = NF * (N + 1);
   static constexpr int RECW = 3 * N2 + 2 * NW;       // the FP64 record (both forms)
@@ -224,10 +224,12 @@ __device__ __noinline__ double apply_cells_fp64(const OpParams<double> &p,
   return part;
 }
 
-// Five and six blocks per SM at k = 4 and 3 instead of the four the register
-// count alone would give: 33x29x37 Q4 183 -> 167 us.
+// 24 or 20 warps per SM.  64^3 Q2: 197 us with 64 threads per block, 204 with
+// 128, 222 with 256; 128 is kept at k = 2 because the fused sums of a small CG
+// pay for every block (24^3 Q2 CG 28.2 against 29.3 ms).  33x29x37 Q4 183 ->
+// 167 us with five blocks instead of the four the register count alone gives.
 template <int N>
-__global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : 6)
+__global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6)
     k_apply_i(const __grid_constant__ OpParams<double> p,
               const __grid_constant__ ApplyArgs<double> a, const int2 *__restrict__ rec,
               const int *__restrict__ exps, const double *__restrict__ rec64) {

@@ -32,7 +32,7 @@ namespace pdg {
 template <int N>
 struct FICfg {
   static constexpr int N2 = N * N, NB = N * N * N, TPC = N * N;
-  static constexpr int CPB = (128 / TPC) > 0 ? (128 / TPC) : 1;
+  static constexpr int CPB = (N == 4 ? 64 : 128) / TPC;   // 32, 14, 4, 5 cells
   static constexpr int THREADS = CPB * TPC;
   static constexpr int NEXP = 8;   // EB[3], EL, usable
   // two exchange arrays and the factors; padding with the fewest shared-memory

@@ -223,9 +223,11 @@ __device__ __forceinline__ void grouped_finish(double *part, long max_blocks, in
   if (!last) return;
   __threadfence();
   double a = 0.0, c = 0.0;
+  // (a warp-wide FP64 addition takes 64 cycles: the second sum only where used)
+  const bool two = fin == FIN_CG_DEF_BETA || slot1 >= 0;
   for (int i = threadIdx.x; i < gsize; i += blockDim.x) {
     a += __ldcg(part + 2 * (g * group + i));
-    c += __ldcg(part + 2 * (g * group + i) + 1);
+    if (two) c += __ldcg(part + 2 * (g * group + i) + 1);
   }
   block_sum2_sel<MAXT, kScratch>(a, c, scratch);
   if (ngroups == 1) {
