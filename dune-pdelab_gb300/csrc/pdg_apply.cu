@@ -462,12 +462,9 @@ __global__ void __launch_bounds__(Cfg<D, N>::THREADS)
   }
   // (compiled for the 2D FP64 operator only, the one fused CG that uses it)
   if constexpr (D == 2 && sizeof(T) == 8) if (a.dot_part) {
-    // block sums in the cell memory, free once every thread is past its reads
-    __syncthreads();
-    reduce_tail_grouped<C::THREADS, true>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
-                                          RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, 0.0,
-                                          a.dot_fin, -1, -1,
-                                          reinterpret_cast<double *>(smem_raw));
+    reduce_tail_grouped<C::THREADS>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
+                                    RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, 0.0,
+                                    a.dot_fin);
   }
 }
 

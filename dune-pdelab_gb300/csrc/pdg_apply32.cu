@@ -476,12 +476,10 @@ __global__ void __launch_bounds__(Q3Cfg::THREADS, 5)
     }
     part += pin.x * v.x + pin.y * v.y + pin.z * v.z + pin.w * v.w;
   }
-  // block sums in the YH run (its z-face terms were consumed in stage 2): no
-  // static shared arrays, six blocks per SM
   if (a.dot_part)
-    reduce_tail_grouped<Q3Cfg::THREADS, true>(
+    reduce_tail_grouped<Q3Cfg::THREADS>(
         a.dot_part, a.dot_max_blocks, a.dot_cnt, RedCtx{nullptr, a.dot_scal, a.dot_flags},
-        (double)part, 0.0, a.dot_fin, -1, -1, reinterpret_cast<double *>(YH));
+        (double)part, 0.0, a.dot_fin);
 }
 
 // ---------------------------------------------------------------------------
@@ -525,8 +523,7 @@ struct Q3T {
   static constexpr int SMEM = 1024 + P1_END;
   static constexpr int LINES_OWN = (CPB + 2) * 2, LINES_RUN = CPB * 2;
   static_assert((CPB + 2) * 256 <= YL_B, "own run overlaps the y runs");
-  static_assert(P2_END + 2 * THREADS * 8 <= P1_END,
-                "phase-2 arrays and the block-sum scratch must fit the phase-1 space");
+  static_assert(P2_END <= P1_END, "phase-2 arrays must fit the phase-1 space");
   static_assert(LINES_OWN == Q3Cfg::LINES_OWN && LINES_RUN == Q3Cfg::LINES_RUN &&
                     LINES_OWN == (int)kLinesOwn && LINES_RUN == (int)kLinesRun,
                 "tensor maps are shared with k_apply32_q3");
@@ -947,12 +944,10 @@ __global__ void __launch_bounds__(Q3T::THREADS, 5)
   }
 
   const float part = q3_run<kTr>(p, a, tb, base, e0, zl, zh);
-  // block sums in the phase-1 space past the phase-2 arrays (record space,
-  // dead since stage 1; other warps may still read the arrays)
   if (a.dot_part)
-    reduce_tail_grouped<Q3T::THREADS, true>(
+    reduce_tail_grouped<Q3T::THREADS>(
         a.dot_part, a.dot_max_blocks, a.dot_cnt, RedCtx{nullptr, a.dot_scal, a.dot_flags},
-        (double)part, 0.0, a.dot_fin, -1, -1, reinterpret_cast<double *>(base + C::P2_END));
+        (double)part, 0.0, a.dot_fin);
 }
 
 // Persistent form: a block runs the runs blockIdx.x, + gridDim.x, ... with
@@ -1047,12 +1042,10 @@ __global__ void __launch_bounds__(Q3T::THREADS, 3)
       zh[q] = nzh[q];
     }
   }
-  // block sums in region 0's scratch space (free: the last sync above, or
-  // no run at all)
   if (a.dot_part)
-    reduce_tail_grouped<Q3T::THREADS, true>(
+    reduce_tail_grouped<Q3T::THREADS>(
         a.dot_part, a.dot_max_blocks, a.dot_cnt, RedCtx{nullptr, a.dot_scal, a.dot_flags},
-        part, 0.0, a.dot_fin, -1, -1, reinterpret_cast<double *>(base + C::P2_END));
+        part, 0.0, a.dot_fin);
 }
 
 static EdgeTab make_edge_tab_uncached(const pdg_context *ctx) {

@@ -364,13 +364,11 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
       zf[2 * (f - 4) + 1] = split32(s2);
     }
   }
-  // <x, y_out> of the fused CG: block sums in the cell memory, once it is free
+  // <x, y_out> of the fused CG
   const auto finish = [&](double part) {
-    __syncthreads();
-    reduce_tail_grouped<C::THREADS, true>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
-                                          RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, 0.0,
-                                          a.dot_fin, -1, -1,
-                                          reinterpret_cast<double *>(smem_raw));
+    reduce_tail_grouped<C::THREADS>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
+                                    RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, 0.0,
+                                    a.dot_fin);
   };
   if (__syncthreads_or(bad)) {
     const double part =

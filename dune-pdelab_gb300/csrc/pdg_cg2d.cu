@@ -106,8 +106,8 @@ __device__ __forceinline__ bool exchange(const Cg2Args &g, unsigned round, int n
   const int nb = gridDim.x;
   const unsigned set = round % kCg2Sets, old = (set + 2) % kCg2Sets;
   if (w < nw) {
-    v0 = warp_sum_d(v0);
-    if (nv > 1) v1 = warp_sum_d(v1);
+    v0 = warp_sum_fixed(v0, 32);
+    if (nv > 1) v1 = warp_sum_fixed(v1, 32);
     if (lane == 0) {
       red[2 * w] = v0;
       red[2 * w + 1] = v1;
@@ -134,7 +134,7 @@ __device__ __forceinline__ bool exchange(const Cg2Args &g, unsigned round, int n
     if (w < nv) {
       double a = 0.0;
       for (int i = lane; i < nb; i += 32) a += all[w * nb + i];
-      a = warp_sum_d(a);
+      a = warp_sum_fixed(a, 32);
       if (lane == 0) red[60 + w] = a;
     }
     __syncthreads();

@@ -258,11 +258,9 @@ __global__ void __launch_bounds__(FICfg<N>::THREADS)
                                           [&](int q) { return u[q]; }, 0));
   }
   const auto finish = [&](double part) {
-    __syncthreads();
-    reduce_tail_grouped<C::THREADS, true>(
+    reduce_tail_grouped<C::THREADS>(
         fuse.part, fuse.max_blocks, fuse.cnt, RedCtx{nullptr, fuse.scal, fuse.flags},
-        fuse.rq ? part2 : part, fuse.rq ? part : 0.0, fuse.fin, -1, -1,
-        reinterpret_cast<double *>(smem_raw));
+        fuse.rq ? part2 : part, fuse.rq ? part : 0.0, fuse.fin);
   };
   if (__syncthreads_or(bad)) {
     const double part = fdm_cells_fp64<N>(Q64, L64, d, v, reinterpret_cast<double *>(S0), l, e,

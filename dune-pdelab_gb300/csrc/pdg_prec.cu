@@ -331,8 +331,7 @@ __global__ void __launch_bounds__(PCfg<D, N>::THREADS)
       s1 = (double)part;
     }
     reduce_tail_grouped<C::THREADS>(dot_part, dot_max_blocks, dot_cnt,
-                                    RedCtx{nullptr, dot_scal, dot_flags}, s0, s1, dot_fin, -1,
-                                    -1);
+                                    RedCtx{nullptr, dot_scal, dot_flags}, s0, s1, dot_fin);
   }
 }
 
@@ -774,7 +773,7 @@ __global__ void __launch_bounds__(FdmQ3Cfg::THREADS)
       s1 = (double)part;
     }
     reduce_tail_grouped<C::THREADS>(dot_part, dot_max_blocks, dot_cnt,
-                                    RedCtx{nullptr, dot_scal, dot_flags}, s0, s1, dot_fin, -1, -1);
+                                    RedCtx{nullptr, dot_scal, dot_flags}, s0, s1, dot_fin);
   }
 }
 
@@ -1003,7 +1002,7 @@ __global__ void __launch_bounds__(FdmQ3T::THREADS)
       s1 = (double)part;
     }
     reduce_tail_grouped<C::THREADS>(dot_part, dot_max_blocks, dot_cnt,
-                                    RedCtx{nullptr, dot_scal, dot_flags}, s0, s1, dot_fin, -1, -1);
+                                    RedCtx{nullptr, dot_scal, dot_flags}, s0, s1, dot_fin);
   }
 }
 

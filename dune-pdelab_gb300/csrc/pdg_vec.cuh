@@ -13,6 +13,7 @@
 // partials in block order and runs the "finisher" for the scalars.
 #pragma once
 
+#include "pdg_fixed.cuh"
 #include "pdg_internal.cuh"
 
 namespace pdg {
@@ -64,6 +65,24 @@ struct RedCtx {
   int *flags;         // [F_COUNT]
 };
 
+// FIN_CG_DEF_BETA in two independent parts.  CGSolver: the defect check after
+// b -= lambda q, then (when it goes on) rho = <M^{-1} b, b>, beta = rho / rholast
+__device__ __forceinline__ void finish_cg_def(const RedCtx &rc, double d0) {
+  const double def = sqrt(d0);
+  int state = 0;
+  if (!isfinite(def)) state = 2;
+  else if (def < rc.scal[S_DEF0] * rc.scal[S_RED] || def < 1e-30) state = 1;
+  rc.scal[S_DEF] = def;
+  if (state) {
+    rc.flags[F_STATE] = state;
+    rc.flags[F_XPEND] = 1;
+  }
+}
+__device__ __forceinline__ void finish_cg_beta(const RedCtx &rc, double d1) {
+  rc.scal[S_BETA] = d1 / rc.scal[S_RHO];
+  rc.scal[S_RHO] = d1;
+}
+
 // Finisher of a reduction: updates the Krylov scalars (dune-istl's
 // CGSolver / BiCGSTABSolver recurrences and breakdown tests) from the two
 // reduced sums d0, d1.
@@ -104,18 +123,6 @@ __device__ inline void run_finisher(const RedCtx &rc, int fin, int slot0, int sl
       s[S_BETA] = d0 / s[S_RHO];
       s[S_RHO] = d0;
       break;
-    case FIN_CG_DEF_BETA: {
-      // CGSolver: the defect check after b -= lambda q, then (when it goes
-      // on) rho = <M^{-1} b, b>, beta = rho / rholast
-      const double def = sqrt(d0);
-      s[S_DEF] = def;
-      if (!isfinite(def)) fl[F_STATE] = 2;
-      else if (def < s[S_DEF0] * s[S_RED] || def < 1e-30) fl[F_STATE] = 1;
-      if (fl[F_STATE]) fl[F_XPEND] = 1;
-      s[S_BETA] = d1 / s[S_RHO];
-      s[S_RHO] = d1;
-      break;
-    }
     // BiCGSTABSolver breakdown tests are absolute (rho, omega <= 1e-80,
     // |h| < 1e-80).  With S_GUARD > 0 (FP32 inner solves, whose dot products
     // carry ~1e-7 relative noise) a relative test is added:
@@ -155,119 +162,127 @@ __device__ inline void run_finisher(const RedCtx &rc, int fin, int slot0, int sl
 // its own output with the other operand per block.  Same determinism as the
 // dot kernels: block partials in a per-kernel array, the last block adds
 // them in block order and runs the finisher.  Blocks of any size <= MAXT.
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <int MAXT>
-__device__ __forceinline__ void block_sum2_with(double &a, double &b, double *sa, double *sb) {
-  __syncthreads();   // the arrays may still be read by a previous call
-  sa[threadIdx.x] = a;
-  sb[threadIdx.x] = b;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double x = 0.0, y = 0.0;
-    for (unsigned i = threadIdx.x; i < blockDim.x; i += 32) {
-      x += sa[i];
-      y += sb[i];
-    }
-    a = warp_sum_d(x);
-    b = warp_sum_d(y);
+// Sum over the first n lanes of a warp (all of which call it; the others do not
+// exist), in every one of them, in 57-bit fixed point: a tree of FP64 additions
+// takes five steps of about 105 cycles, this about 250 in all.  Values that are
+// not finite, or so small that the fixed point would lose them, are added in
+// FP64.  The result does not depend on the order of the lanes.
+__device__ __forceinline__ double warp_sum_fixed(double v, int n) {
+  const unsigned mask = n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+  const unsigned m = __reduce_max_sync(mask, (unsigned)__double2hiint(v) << 1);
+  const int b = (int)(m >> 21);
+  if (b == 0x7ff || (b < 128 && m != 0)) {
+    double s = 0.0;
+    for (int i = 0; i < n; i++) s += __shfl_sync(mask, v, i);
+    return s;
   }
+  const int eb = max(b, kFixMinBiased);
+  const long long x = fix_signed(v, eb);
+  const unsigned s0 = __reduce_add_sync(mask, (unsigned)x & 0x7ffffffu);
+  const unsigned s1 = __reduce_add_sync(mask, (unsigned)(x >> 27) & 0x7ffffffu);
+  const int s2 = __reduce_add_sync(mask, (int)(x >> 54));
+  const long long s = (long long)(((unsigned long long)(unsigned)s2 << 54) +
+                                  ((unsigned long long)s1 << 27) + s0);
+  return (double)s * __hiloint2double((eb - 56) << 20, 0);   // units of 2^(E - 57)
 }
 
-template <int MAXT>
-__device__ __forceinline__ void block_sum2_any(double &a, double &b) {
-  __shared__ double sa[MAXT], sb[MAXT];
-  block_sum2_with<MAXT>(a, b, sa, sb);
-}
-
-// block sums through a caller-provided scratch of 2 * MAXT doubles (the
-// kernel's dynamic shared memory) or static arrays
-template <int MAXT, bool kScratch>
-__device__ __forceinline__ void block_sum2_sel(double &a, double &b, double *scratch) {
-  if constexpr (kScratch) block_sum2_with<MAXT>(a, b, scratch, scratch + MAXT);
-  else block_sum2_any<MAXT>(a, b);
+// Block sums of two values (the second only if `two`): warp sums in sw (at
+// least 2 * number of warps), then threads 0 and 1 hold the sums in s0.
+__device__ __forceinline__ void block_sum2(double &s0, double s1, bool two, double *sw) {
+  const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  const int n = min(32, (int)blockDim.x - 32 * w);
+  s0 = warp_sum_fixed(s0, n);
+  if (two) s1 = warp_sum_fixed(s1, n);
+  if ((threadIdx.x & 31) == 0) {
+    sw[2 * w] = s0;
+    sw[2 * w + 1] = two ? s1 : 0.0;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    s0 = sw[threadIdx.x];
+    for (int i = 1; i < nw; i++) s0 += sw[2 * i + threadIdx.x];
+  }
 }
 
 // Two-level tail for grids of many blocks: the last block of each group of
 // kFuseGroup blocks adds the group's partials in block order into a group
 // partial; the last group to finish adds the group partials in group order
-// and runs the finisher.  The order of every sum is fixed, so the result does
-// not depend on which block finishes last.  Layout of `part`: 2 doubles per
-// block, then 2 per group from offset 2 * max_blocks; `cnt`: one int per
-// group, zero between launches (each group's last block resets its own).
+// and runs the finisher.  Up to kFuseOne blocks are one group.  The order of
+// every sum is fixed, so the result does not depend on which block finishes
+// last.  Layout of `part`: 2 doubles per block, then 2 per group from offset
+// 2 * max_blocks; `cnt`: one int per group, zero between launches (each
+// group's last block resets its own).
 constexpr int kFuseGroup = 256;
 constexpr unsigned kFuseOne = 1024;
 
-// (s0, s1): the block's sums, in thread 0
-template <int MAXT, bool kScratch = false>
-__device__ __forceinline__ void grouped_finish(double *part, long max_blocks, int *cnt,
-                                               const RedCtx &rc, double s0, double s1, int fin,
-                                               int slot0, int slot1, double *scratch = nullptr) {
+// publish (s0 of threads 0 and 1) and count; true in the last of `total`
+// publishers, which then sees what the others published
+__device__ __forceinline__ bool publish_last(double *slot, double s0, int *counter, int total) {
   __shared__ bool last;
-  // up to kFuseOne blocks: one group, one level
+  if (threadIdx.x < 32) {
+    const double c = __shfl_sync(0xffffffffu, s0, 1);
+    if (threadIdx.x == 0) {
+      *reinterpret_cast<double2 *>(slot) = make_double2(s0, c);
+      int n;
+      asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;"
+                   : "=r"(n)
+                   : "l"(counter)
+                   : "memory");
+      last = n == total - 1;
+    }
+  }
+  __syncthreads();
+  return last;
+}
+
+// the block's sums are in s0 of threads 0 and 1; blocks of at least 32 threads
+template <int MAXT>
+__device__ __forceinline__ void grouped_finish(double *part, long max_blocks, int *cnt,
+                                               const RedCtx &rc, double s0, int fin) {
+  __shared__ double sw[2 * ((MAXT + 31) / 32)];
+  const bool two = fin == FIN_CG_DEF_BETA;
   const int group = gridDim.x <= kFuseOne ? (int)gridDim.x : kFuseGroup;
   const int b = (int)blockIdx.x, g = b / group;
   const int ngroups = (int)((gridDim.x + group - 1) / group);
   const int gsize = min(group, (int)gridDim.x - g * group);
-  if (threadIdx.x == 0) {
-    part[2 * b] = s0;
-    part[2 * b + 1] = s1;
-    __threadfence();
-    last = atomicAdd(&cnt[g], 1) == gsize - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double a = 0.0, c = 0.0;
-  // (a warp-wide FP64 addition takes 64 cycles: the second sum only where used)
-  const bool two = fin == FIN_CG_DEF_BETA || slot1 >= 0;
-  for (int i = threadIdx.x; i < gsize; i += blockDim.x) {
-    a += __ldcg(part + 2 * (g * group + i));
-    if (two) c += __ldcg(part + 2 * (g * group + i) + 1);
-  }
-  block_sum2_sel<MAXT, kScratch>(a, c, scratch);
-  if (ngroups == 1) {
-    if (threadIdx.x == 0) {
-      cnt[0] = 0;
-      run_finisher(rc, fin, slot0, slot1, a, c);
+  if (!publish_last(part + 2 * (size_t)b, s0, &cnt[g], gsize)) return;
+  const double2 *p2 = reinterpret_cast<const double2 *>(part) + (size_t)g * group;
+  const auto sum = [&](const double2 *v, int n) {
+    double a = 0.0, c = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const double2 x = __ldcg(v + i);
+      a += x.x;
+      if (two) c += x.y;
     }
+    block_sum2(a, c, two, sw);
+    return a;
+  };
+  double a = sum(p2, gsize);
+  if (threadIdx.x == 0) cnt[g] = 0;
+  if (ngroups > 1) {
+    double *gpart = part + 2 * max_blocks;
+    if (!publish_last(gpart + 2 * g, a, &rc.flags[F_COUNTER], ngroups)) return;
+    a = sum(reinterpret_cast<const double2 *>(gpart), ngroups);
+    if (threadIdx.x == 0) rc.flags[F_COUNTER] = 0;
+  }
+  if (!two) {
+    if (threadIdx.x == 0) run_finisher(rc, fin, -1, -1, a, 0.0);
     return;
   }
-  double *gpart = part + 2 * max_blocks;
-  if (threadIdx.x == 0) {
-    gpart[2 * g] = a;
-    gpart[2 * g + 1] = c;
-    cnt[g] = 0;
-    __threadfence();
-    last = atomicAdd(&rc.flags[F_COUNTER], 1) == ngroups - 1;
-  }
+  // the square root and the quotient of FIN_CG_DEF_BETA by two warps
+  if (threadIdx.x < 2) sw[threadIdx.x] = a;
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  a = 0.0;
-  c = 0.0;
-  for (int i = threadIdx.x; i < ngroups; i += blockDim.x) {
-    a += __ldcg(gpart + 2 * i);
-    c += __ldcg(gpart + 2 * i + 1);
-  }
-  block_sum2_sel<MAXT, kScratch>(a, c, scratch);
-  if (threadIdx.x == 0) {
-    run_finisher(rc, fin, slot0, slot1, a, c);
-    rc.flags[F_COUNTER] = 0;
-  }
+  if (threadIdx.x == 0) finish_cg_def(rc, sw[0]);
+  if (threadIdx.x == (blockDim.x > 32 ? 32 : 0)) finish_cg_beta(rc, sw[1]);
 }
 
-template <int MAXT, bool kScratch = false>
+template <int MAXT>
 __device__ __forceinline__ void reduce_tail_grouped(double *part, long max_blocks, int *cnt,
                                                     const RedCtx &rc, double s0, double s1,
-                                                    int fin, int slot0, int slot1,
-                                                    double *scratch = nullptr) {
-  block_sum2_sel<MAXT, kScratch>(s0, s1, scratch);
-  grouped_finish<MAXT, kScratch>(part, max_blocks, cnt, rc, s0, s1, fin, slot0, slot1, scratch);
+                                                    int fin) {
+  __shared__ double sw[2 * ((MAXT + 31) / 32)];
+  block_sum2(s0, s1, fin == FIN_CG_DEF_BETA, sw);
+  grouped_finish<MAXT>(part, max_blocks, cnt, rc, s0, fin);
 }
 
 // A sum carried as an unevaluated pair of floats (48 bits): block sums of FP32
@@ -306,17 +321,15 @@ __device__ __forceinline__ void reduce_tail_two_float(double *part, long max_blo
     w1[threadIdx.x >> 5] = s1;
   }
   __syncthreads();
-  double a = 0.0, c = 0.0;
-  if (threadIdx.x == 0) {
+  // thread 0 adds the first values, thread 1 the second
+  double a = 0.0;
+  if (threadIdx.x < 2) {
+    TwoFloat v = threadIdx.x == 0 ? w0[0] : w1[0];
 #pragma unroll
-    for (int i = 1; i < T / 32; i++) {
-      s0 = two_add(s0, w0[i]);
-      s1 = two_add(s1, w1[i]);
-    }
-    a = (double)s0.h + (double)s0.l;
-    c = (double)s1.h + (double)s1.l;
+    for (int i = 1; i < T / 32; i++) v = two_add(v, threadIdx.x == 0 ? w0[i] : w1[i]);
+    a = (double)v.h + (double)v.l;
   }
-  grouped_finish<T>(part, max_blocks, cnt, rc, a, c, fin, -1, -1);
+  grouped_finish<T>(part, max_blocks, cnt, rc, a, fin);
 }
 
 int red_dot(pdg_context *ctx, const RedCtx &rc, long n, const double *a, const double *b,
