@@ -12,15 +12,15 @@
 // does all contractions of its cell without exchanging anything, so the only
 // shared-memory traffic is the staged input (read once) and the staged output.
 // 27 is odd, so the scalar reads of 32 consecutive cells fall on 32 banks.
-// The operator takes per cell 23 coefficients (K/h per direction, the reaction
+// The operator takes per cell 22 coefficients (K/h per direction, the reaction
 // term, and {kappa_e, kappa_o, penalty} of each face) instead of the assembled
 // 1D matrices A'_dir (57 at degree 2): with the shape matrices as constants
 // the self terms of a face share the jump and the normal derivatives with its
-// neighbour terms.  64^3 Q2 (7.1M DOF) takes 47 us for the operator and 38 us for
+// neighbour terms.  64^3 Q2 (7.1M DOF) takes 40 us for the operator and 33 us for
 // the block Jacobi with the residual update (plane-per-thread kernels with
 // exchanges: 81 and 68 us); the bytes need 12 and 22 us.  What is left is the
-// latency of load, compute and store within a block at 10 and 18 warps per SM.
-// 64 threads per block: 32 and 128 are slower on large or small grids (64^3
+// latency of load, compute and store within a block at 16 and 18 warps per SM.
+// Runs of 64 cells: 32 and 128 are slower on large or small grids (64^3
 // mixed CG 252, 252 and 281 ms, 32^3 gradient 69, 80 and 69 ms).
 //
 // Block sums of the fused dot products are formed in two-float arithmetic
@@ -38,12 +38,16 @@ namespace pdg {
 template <int N>
 struct C32Cfg {
   static constexpr int N2 = N * N, NB = N * N * N;
-  static constexpr int T = 64;                        // cells (threads) per block
-  static constexpr int REC = 23;                      // coefficients per cell (odd: no bank conflicts)
-  static constexpr int OWN = (T + 2) * NB, RUN = T * NB, RECS = T * REC;
+  static constexpr int T = 64;                        // cells of a run
+  static constexpr int REC = 22;                      // coefficients per cell
+  static constexpr int OWN = (T + 2) * NB, RUN = T * NB;
   // staged runs carry up to 3 floats of 16-byte phase of their source
-  static constexpr int OWNP = (OWN + 7) / 4 * 4, RUNP = (RUN + 7) / 4 * 4, RECP = (RECS + 7) / 4 * 4;
-  static constexpr int SMEM = OWNP + 4 * RUNP + RECP + NB;
+  static constexpr int OWNP = (OWN + 7) / 4 * 4, RUNP = (RUN + 7) / 4 * 4;
+  // the operator: two runs (their own cells, four y and two z neighbour runs;
+  // two more z neighbour runs unless the runs are each other's), one block of zeros
+  static constexpr int THREADS = 2 * T;
+  static constexpr int SMEM = (2 * OWNP + 6 * RUNP + NB + 3) / 4 * 4;
+  static constexpr int SMEM_SIDE = SMEM + 2 * RUNP;
   static constexpr int SMEM_FDM = 2 * RUNP + (T * 3 * N2 + 7) / 4 * 4 + (T * 3 * N + 7) / 4 * 4;
 };
 
@@ -54,7 +58,7 @@ struct C32Tab {
 };
 
 // {hp K_dir / h_dir (3), hp_x c h_x, per face {hp kappa_e / h, hp kappa_o / h,
-// hp penalty}}, formed in FP64 and rounded
+// hp penalty}}, formed in FP64 and rounded; [coefficient][cell]
 template <int N>
 __global__ void k_record_c32(const OpParams<double> p, float *__restrict__ rec) {
   const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -68,13 +72,13 @@ __global__ void k_record_c32(const OpParams<double> p, float *__restrict__ rec) 
     ix[2] = (int)q1;
   }
   const long stride[3] = {1, (long)p.nc[0], (long)p.nc[0] * p.nc[1]};
-  float *r = rec + e * C32Cfg<N>::REC;
+  const auto put = [&](int k, double v) { rec[k * p.ncell + e] = (float)v; };
   for (int dir = 0; dir < 3; dir++) {
     double hp = 1.0;
     for (int j = 0; j < 3; j++)
       if (j != dir) hp *= p.h[j];
-    r[dir] = (float)(hp * over_h(p, dir, kdir(p, e, dir)));
-    if (dir == 0) r[3] = (float)(p.c ? hp * p.c[e] * p.h[0] : 0.0);
+    put(dir, hp * over_h(p, dir, kdir(p, e, dir)));
+    if (dir == 0) put(3, p.c ? hp * p.c[e] * p.h[0] : 0.0);
     for (int hi = 0; hi < 2; hi++) {
       const int f = 2 * dir + hi;
       long nb;
@@ -82,10 +86,9 @@ __global__ void k_record_c32(const OpParams<double> p, float *__restrict__ rec) 
       else nb = ix[dir] > 0 ? e - stride[dir] : -1;
       double raw[3];
       face_coefficients(p, f, kdir(p, e, dir), nb, raw);
-      for (int j = 0; j < 3; j++) r[4 + 3 * f + j] = (float)(hp * raw[j]);
+      for (int j = 0; j < 3; j++) put(4 + 3 * f + j, hp * raw[j]);
     }
   }
-  r[22] = 0.f;
 }
 
 // Staging of a block's input runs.  A run of source elements [g0, g0 + count)
@@ -168,26 +171,32 @@ __device__ __forceinline__ void cell_line(const C32Tab<N> &tb, float k, const fl
   res[N - 1] += hi.pen * jh - hi.ke * duh - hi.ko * dh;
 }
 
-// write-back of a block's run staged in shared memory: element f(O[i], index)
-template <int N, class F>
-__device__ __forceinline__ void write_run(const float *O, float *y, long g0, long ndof, F f) {
-  using C = C32Cfg<N>;
-  const int count = (int)min((long)C::RUN, ndof - g0);
-  for (int i = threadIdx.x; i < count; i += C::T) y[g0 + i] = f(O[i], g0 + i);
+// write-back of a run staged in shared memory: element f(O[i], index), by the
+// threads i0, i0 + T, ..
+template <int T, class F>
+__device__ __forceinline__ void write_run(const float *O, float *y, long g0, int count, int i0,
+                                          F f) {
+  for (int i = i0; i < count; i += T) y[g0 + i] = f(O[i], g0 + i);
 }
-// the same unchanged, as one bulk store by thread 0 (full block, 16-byte
-// aligned y; g0 is a multiple of 64 N^3).  The caller has fenced the writes of
-// O for the async proxy before its barrier, and calls bulk_store_wait before
-// the block ends.
-template <int N>
-__device__ __forceinline__ bool bulk_store_ok(const float *y, long g0, long ndof) {
-  return (reinterpret_cast<uintptr_t>(y) & 15) == 0 && g0 + C32Cfg<N>::RUN <= ndof;
+// The same unchanged: O has the 16-byte phase of y + g0 (y aligned), whole
+// 16-byte chunks are one bulk store by thread i0 = 0, the ends go one by one.
+// The caller has fenced the writes of O for the async proxy before its barrier,
+// and calls bulk_store_wait in that thread before the block ends.
+template <int T>
+__device__ __forceinline__ void bulk_store_run(const float *O, float *y, long g0, int count,
+                                               int i0) {
+  const int head = min((int)((4 - (g0 & 3)) & 3), count), mid = (count - head) & ~3;
+  if (i0 == 0 && mid > 0) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(y + g0 + head),
+                 "r"(smem_u32(O + head)), "r"(4u * mid)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+  if (i0 < head) y[g0 + i0] = O[i0];
+  if (i0 < count - head - mid) y[g0 + head + mid + i0] = O[head + mid + i0];
 }
-__device__ __forceinline__ void bulk_store(float *y, const float *O, unsigned bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(y),
-               "r"(smem_u32(O)), "r"(bytes)
-               : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+__device__ __forceinline__ bool aligned16(const void *p) {
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0;
 }
 __device__ __forceinline__ void bulk_store_wait() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -196,37 +205,64 @@ __device__ __forceinline__ void fence_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-template <int N>
-__global__ void __launch_bounds__(C32Cfg<N>::T)
+// A block computes two runs of 64 cells.  kStack: the runs are one plane of the
+// slowest direction apart, each is the other's z neighbour; that stages 8.1
+// instead of 10.1 cells per computed pair and leaves room for 16 warps per SM
+// instead of 12.  Otherwise the runs lie side by side (planes that do not fill
+// runs of 64 cells, single planes).  64^3 Q2: one run per block with its
+// coefficients staged as well (10 warps per SM) 47 us, stacked runs with
+// coefficients read coalesced into registers 40 us.
+template <int N, bool kStack>
+__global__ void __launch_bounds__(C32Cfg<N>::THREADS)
     k_apply32_cell(const OpParams<float> p, const ApplyArgs<float> a,
                    const float *__restrict__ rec,
                    const __grid_constant__ C32Tab<N> tb, int *tma_err) {
   using C = C32Cfg<N>;
   constexpr int N2 = C::N2, NB = C::NB, T = C::T;
   extern __shared__ __align__(16) float sm[];
-  if (a.skip && *a.skip) return;
-  const long e0 = (long)blockIdx.x * T, ndof = p.ncell * NB;
-  const long sx = p.nc[0], sxy = (long)p.nc[0] * p.nc[1];
   __shared__ __align__(8) unsigned long long bar;
-  Stager<T> st(&bar);
-  float *Y0 = sm + C::OWNP;
-  float *R0 = Y0 + 4 * C::RUNP;
-  const float *RS = st.run(R0, rec, e0 * C::REC, p.ncell * C::REC, C::RECS);
-  const float *OWN = st.run(sm, a.x, (e0 - 1) * NB, ndof, C::OWN);
-  const float *YL = st.run(Y0, a.x, (e0 - sx) * NB, ndof, C::RUN);
-  const float *YH = st.run(Y0 + C::RUNP, a.x, (e0 + sx) * NB, ndof, C::RUN);
-  const float *ZL = st.run(Y0 + 2 * C::RUNP, a.x, (e0 - sxy) * NB, ndof, C::RUN);
-  const float *ZH = st.run(Y0 + 3 * C::RUNP, a.x, (e0 + sxy) * NB, ndof, C::RUN);
-  float *zero = R0 + C::RECP;   // stands in for an absent neighbour
-  if (threadIdx.x < NB) zero[threadIdx.x] = 0.f;
-  if (!st.wait()) {
-    if (threadIdx.x == 0) atomicExch(tma_err, 1);
-    return;
+  if (a.skip && *a.skip) return;
+  const long ndof = p.ncell * NB;
+  const long sx = p.nc[0], sxy = (long)p.nc[0] * p.nc[1];
+  // first cells of the two runs, and the cells of each
+  const int half = threadIdx.x / T, cs = threadIdx.x % T;
+  const long dz = kStack ? sxy : T;
+  long e0;
+  int count;
+  if constexpr (kStack) {
+    const unsigned chunks = (unsigned)((sxy + T - 1) / T), pair = blockIdx.x / chunks;
+    const long in = (long)(blockIdx.x - pair * chunks) * T;
+    e0 = (long)pair * 2 * sxy + in;
+    count = 2 * (int)pair + half < p.nc[2] ? (int)min((long)T, sxy - in) : 0;
+  } else {
+    e0 = (long)blockIdx.x * 2 * T;
+    count = (int)max(0l, min((long)T, p.ncell - e0 - half * T));
   }
+  const long er = e0 + half * dz;
+  const bool active = cs < count;
+  const long e = er + cs;
+  // coefficients first: coalesced, in flight beside the runs' copies
+  float R[C::REC];
+#pragma unroll
+  for (int k = 0; k < C::REC; k++) R[k] = rec[k * p.ncell + (active ? e : 0)];
 
-  const int cs = threadIdx.x;
-  const long e = e0 + cs;
-  const bool active = e < p.ncell;
+  Stager<C::THREADS> st(&bar);
+  float *Y0 = sm + 2 * C::OWNP;
+  const float *O0 = st.run(sm, a.x, (e0 - 1) * NB, ndof, C::OWN);
+  const float *O1 = st.run(sm + C::OWNP, a.x, (e0 + dz - 1) * NB, ndof, C::OWN);
+  const float *ZL = st.run(Y0 + 4 * C::RUNP, a.x, (e0 - sxy) * NB, ndof, C::RUN);
+  const float *ZH = st.run(Y0 + 5 * C::RUNP, a.x, (e0 + dz + sxy) * NB, ndof, C::RUN);
+  const float *ZL1 = O0 + NB, *ZH0 = O1 + NB;
+  if constexpr (!kStack) {
+    ZL1 = st.run(sm + C::SMEM, a.x, (e0 + dz - sxy) * NB, ndof, C::RUN);
+    ZH0 = st.run(sm + C::SMEM + C::RUNP, a.x, (e0 + sxy) * NB, ndof, C::RUN);
+  }
+  const float *YL0 = st.run(Y0, a.x, (e0 - sx) * NB, ndof, C::RUN);
+  const float *YH0 = st.run(Y0 + 2 * C::RUNP, a.x, (e0 + sx) * NB, ndof, C::RUN);
+  const float *YL1 = st.run(Y0 + C::RUNP, a.x, (e0 + dz - sx) * NB, ndof, C::RUN);
+  const float *YH1 = st.run(Y0 + 3 * C::RUNP, a.x, (e0 + dz + sx) * NB, ndof, C::RUN);
+  float *zero = Y0 + 6 * C::RUNP;   // stands in for an absent neighbour
+  if (threadIdx.x < NB) zero[threadIdx.x] = 0.f;
   int ix[3];
   {
     const unsigned ee = active ? (unsigned)e : 0u;
@@ -237,14 +273,17 @@ __global__ void __launch_bounds__(C32Cfg<N>::T)
     ix[2] = (int)q1;
   }
   const bool cp = !a.diag_only;
-  const float *U = OWN + (cs + 1) * NB;
+  const float *U = (half ? O1 : O0) + (cs + 1) * NB;
   const float *xl = cp && ix[0] > 0 ? U - NB : zero;
   const float *xh = cp && ix[0] + 1 < p.nc[0] ? U + NB : zero;
-  const float *yl = cp && ix[1] > 0 ? YL + cs * NB : zero;
-  const float *yh = cp && ix[1] + 1 < p.nc[1] ? YH + cs * NB : zero;
-  const float *zl = cp && ix[2] > 0 ? ZL + cs * NB : zero;
-  const float *zh = cp && ix[2] + 1 < p.nc[2] ? ZH + cs * NB : zero;
-  const float *R = RS + cs * C::REC;
+  const float *yl = cp && ix[1] > 0 ? (half ? YL1 : YL0) + cs * NB : zero;
+  const float *yh = cp && ix[1] + 1 < p.nc[1] ? (half ? YH1 : YH0) + cs * NB : zero;
+  const float *zl = cp && ix[2] > 0 ? (half ? ZL1 : ZL) + cs * NB : zero;
+  const float *zh = cp && ix[2] + 1 < p.nc[2] ? (half ? ZH : ZH0) + cs * NB : zero;
+  if (!st.wait()) {
+    if (threadIdx.x == 0) atomicExch(tma_err, 1);
+    return;
+  }
   const float a1 = a.transpose ? -p.theta : 1.f, a2 = a.transpose ? 1.f : -p.theta;
 
   float out[N][N][N];   // [z][y][x]
@@ -385,30 +424,30 @@ __global__ void __launch_bounds__(C32Cfg<N>::T)
       part = two_add(part, TwoFloat{s, 0.f});
     }
   }
-  __syncthreads();   // the YL run is free
+  __syncthreads();   // the y runs are free
+  float *O = Y0 + half * C::RUNP + ((er * NB) & 3);
 #pragma unroll
   for (int z = 0; z < N; z++)
 #pragma unroll
-    for (int i = 0; i < N2; i++) Y0[cs * NB + z * N2 + i] = out[z][i / N][i % N];
-  const bool plain = !a.accumulate && !a.add && a.alpha == 1.f &&
-                     bulk_store_ok<N>(a.y, e0 * NB, ndof);
+    for (int i = 0; i < N2; i++) O[cs * NB + z * N2 + i] = out[z][i / N][i % N];
+  const bool plain = !a.accumulate && !a.add && a.alpha == 1.f && aligned16(a.y);
   if (plain) fence_async();
   __syncthreads();
   if (plain) {
-    if (threadIdx.x == 0) bulk_store(a.y + e0 * NB, Y0, 4u * C::RUN);
+    bulk_store_run<T>(O, a.y, er * NB, count * NB, cs);
+    if (cs == 0) bulk_store_wait();
   } else {
-    write_run<N>(Y0, a.y, e0 * NB, ndof, [&](float v, long g) {
+    write_run<T>(O, a.y, er * NB, count * NB, cs, [&](float v, long g) {
       float r = a.alpha * v;
       if (a.accumulate) r += a.y[g];
       if (a.add) r += a.add[g];
       return r;
     });
   }
-  if (plain && threadIdx.x == 0) bulk_store_wait();
   if (a.dot_part)
-    reduce_tail_two_float<T>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
-                             RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, TwoFloat{0.f, 0.f},
-                             a.dot_fin);
+    reduce_tail_two_float<C::THREADS>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
+                                      RedCtx{nullptr, a.dot_scal, a.dot_flags}, part,
+                                      TwoFloat{0.f, 0.f}, a.dot_fin);
 }
 
 // v = scale (Qx (x) Qy (x) Qz) diag(1/(lx+ly+lz)) (Qx (x) Qy (x) Qz)^T d;
@@ -524,20 +563,19 @@ __global__ void __launch_bounds__(C32Cfg<N>::T, 9)
     s1 = two_add(s1, TwoFloat{s, 0.f});
   }
   if (!active) s0 = s1 = TwoFloat{0.f, 0.f};
-  const bool bulk = bulk_store_ok<N>(v, e0 * NB, ndof) && bulk_store_ok<N>(d, e0 * NB, ndof);
+  const bool bulk = aligned16(v) && aligned16(d);
   if (bulk) fence_async();
   __syncthreads();
+  const int count = (int)min((long)C::RUN, ndof - e0 * NB);
   if (bulk) {
-    if (threadIdx.x == 0) {
-      if (rq) bulk_store(d + e0 * NB, sm, 4u * C::RUN);
-      bulk_store(v + e0 * NB, sm + C::RUNP, 4u * C::RUN);
-    }
+    if (rq) bulk_store_run<T>(sm, d, e0 * NB, count, cs);
+    bulk_store_run<T>(sm + C::RUNP, v, e0 * NB, count, cs);
+    if (cs == 0) bulk_store_wait();
   } else {
     const auto same = [](float x, long) { return x; };
-    if (rq) write_run<N>(sm, d, e0 * NB, ndof, same);
-    write_run<N>(sm + C::RUNP, v, e0 * NB, ndof, same);
+    if (rq) write_run<T>(sm, d, e0 * NB, count, cs, same);
+    write_run<T>(sm + C::RUNP, v, e0 * NB, count, cs, same);
   }
-  if (bulk && threadIdx.x == 0) bulk_store_wait();
   if (dot_part)
     reduce_tail_two_float<T>(dot_part, dot_max_blocks, dot_cnt,
                              RedCtx{nullptr, dot_scal, dot_flags}, rq ? s0 : s1,
@@ -548,11 +586,14 @@ template <int N>
 static int launch_apply32_cell_n(pdg_context *ctx, const ApplyArgs<float> &a,
                                  const OpParams<float> &p) {
   using C = C32Cfg<N>;
-  const size_t smem = sizeof(float) * C::SMEM;
   static int attr_dev = -1;
   if (attr_dev != ctx->device) {
-    PDG_CUDA_TRY(cudaFuncSetAttribute(k_apply32_cell<N>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PDG_CUDA_TRY(cudaFuncSetAttribute(k_apply32_cell<N, true>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(float) * C::SMEM));
+    PDG_CUDA_TRY(cudaFuncSetAttribute(k_apply32_cell<N, false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(float) * C::SMEM_SIDE));
     attr_dev = ctx->device;
   }
   if (!ctx->rec32c_valid) {
@@ -571,9 +612,17 @@ static int launch_apply32_cell_n(pdg_context *ctx, const ApplyArgs<float> &a,
     tb.d0[i] = (float)ctx->tab_host[2 * C::N2 + i];
     tb.d1[i] = (float)ctx->tab_host[2 * C::N2 + N + i];
   }
-  const unsigned blocks = (unsigned)((ctx->ncell + C::T - 1) / C::T);
-  k_apply32_cell<N><<<blocks, C::T, smem, ctx->stream>>>(p, a, ctx->rec32c, tb,
-                                                          ctx->d_flag + F_TMA);
+  const long plane = ctx->ncell / p.nc[2];
+  const long stack = (plane + C::T - 1) / C::T * ((p.nc[2] + 1) / 2);
+  const long side = (ctx->ncell + 2 * C::T - 1) / (2 * C::T);
+  // stacked runs while they take at most a quarter more blocks
+  if (4 * stack <= 5 * side)
+    k_apply32_cell<N, true><<<(unsigned)stack, C::THREADS, sizeof(float) * C::SMEM, ctx->stream>>>(
+        p, a, ctx->rec32c, tb, ctx->d_flag + F_TMA);
+  else
+    k_apply32_cell<N, false>
+        <<<(unsigned)side, C::THREADS, sizeof(float) * C::SMEM_SIDE, ctx->stream>>>(
+            p, a, ctx->rec32c, tb, ctx->d_flag + F_TMA);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }

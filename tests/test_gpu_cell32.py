@@ -82,3 +82,13 @@ def test_fdm_and_mixed_solve(k, n):
         sol.append(u.cpu().numpy())
     assert rel(sol[1], sol[0]) <= 1e-8
     go.close()
+
+
+@pytest.mark.parametrize("k", [1, 2])
+@pytest.mark.parametrize("n", [(8, 8, 3), (16, 8, 5), (9, 14, 4), (64, 1, 2)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_stacked_runs(k, n, offset):
+    """Planes that (nearly) fill runs of 64 cells, odd and even numbers of them."""
+    test_apply(k, n, offset)
+    if offset == 0:
+        test_fdm_and_mixed_solve(k, n)
