@@ -21,7 +21,7 @@ SOURCES = ["pdg_abi.cu", "pdg_apply.cu", "pdg_prec.cu", "pdg_rhs.cu", "pdg_vec.c
            "pdg_noalloc.cu", "pdg_conv.cu", "pdg_assemble.cu",
            "pdg_blocksolve.cu", "pdg_apply32.cu",
            "pdg_nonlinear.cu", "pdg_basis.cu", "pdg_general.cu", "pdg_apply_fp.cu", "pdg_apply_m.cu",
-           "pdg_apply_i.cu", "pdg_tensor.cu", "pdg_fdm_i.cu",
+           "pdg_apply_i.cu", "pdg_apply_p.cu", "pdg_tensor.cu", "pdg_fdm_i.cu",
            "pdg_cell32.cu", "pdg_cg2d.cu", "pdg_conv_i.cu"]
 PROBE_SOURCES = ["probe_peak.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -1,4 +1,5 @@
-// pdg_apply_i.cu -- the coupled 3D FP64 cell operator in 64-bit fixed point.
+// pdg_apply_i.cu -- the coupled 3D FP64 cell operator in 64-bit fixed point
+// (degrees 1, 3 and 4; pdg_apply_p.cu has the kernel of degree 2).
 //
 // Same operator as k_apply<double, 3, N> (pdg_apply.cu; reference:
 // ConvectionDiffusionDG::jacobian_apply_volume / _skeleton / _boundary,
@@ -32,7 +33,7 @@ namespace pdg {
 template <int N>
 struct ICfg {
   static constexpr int N2 = N * N, NB = N * N * N, TPC = N * N, NF = 6;
-  static constexpr int CPB = (N == 4 ? 64 : 128) / TPC;   // 32, 14, 4, 5 cells
+  static constexpr int CPB = (N == 4 ? 64 : 128) / TPC;   // 32, 4, 5 cells (k = 1, 3, 4)
   static constexpr int THREADS = CPB * TPC;
   static constexpr int NW = NF * (N + 1);
   static constexpr int RECW = 3 * N2 + 2 * NW;       // the FP64 record (both forms)
@@ -43,35 +44,51 @@ struct ICfg {
   // counted on the CPU over paddings 0..15 (k = 4: 2352 per block instead of
   // 3128 without the right one)
   static constexpr int PER_CELL =
-      4 * NB + 12 * TPC + RECI + (N == 2 ? 6 : N == 3 ? 1 : N == 5 ? 10 : 0);
-  static constexpr int LN = N == 2 ? 1 : N == 5 ? 3 : 2;              // ceil log2 N
-  static constexpr int LD = N == 2 ? 0 : N == 3 ? 2 : N == 4 ? 5 : 6;  // ceil log2 max |d|
+      4 * NB + 12 * TPC + RECI + (N == 2 ? 6 : N == 5 ? 10 : 0);
+  static constexpr int LN = N == 2 ? 1 : N == 5 ? 3 : 2;   // ceil log2 N
+  static constexpr int LD = N == 2 ? 0 : N == 4 ? 5 : 6;   // ceil log2 max |d|
   // X, Y, Z are formed below 2^61 and shifted to 2^(61 - SHX) so that the
-  // masses (row sums 3, 20, 864, 2988) stay below 2^63: N <= 3 modulo 2^64,
+  // masses (row sums 3, 864, 2988) stay below 2^63: N = 2 modulo 2^64,
   // shifting by SHM after the first; N >= 4 with two sums, shifting by SHM
   // after each
-  static constexpr bool WIDE = N >= 3;
+  static constexpr bool WIDE = N > 2;
   static constexpr int SHX = N == 2 ? 2 : 0;
-  static constexpr int SHM = N == 2 ? 2 : N == 3 ? 5 : N == 4 ? 10 : 12;
+  static constexpr int SHM = N == 2 ? 2 : N == 4 ? 10 : 12;
   // exponent of one unit of the result over the cell's Etot
   static constexpr int OUTE = -61 + SHX + (WIDE ? 2 * SHM : SHM);
 };
 
+// place of entry i of cell e in the limb records of n entries per cell: cell by
+// cell, for the degree of k_apply_p entry by entry within a group of 32 cells
+template <int N>
+__device__ __forceinline__ size_t limb_at(long e, int n, int i) {
+  return N == 3 ? ((size_t)(e / kGroup) * n + i) * kGroup + e % kGroup : (size_t)e * n + i;
+}
+
 // Limb record of one form (operator, or its transpose): A'_dir / den^2, then
 // per face the line coefficients W[0..N-1] / den^2 and W[N] / (den^2 dden),
-// from the FP64 record.  The quotients are formed to more than FP64 (product
+// from the FP64 record (zero without a neighbour).  The quotients are formed to more than FP64 (product
 // with the reciprocal and its rest) before they are cut to 57 bits.
 // exps[e] = {EA, EW1[6], EW2[6], usable}: exponents of A' (all directions),
 // of the W[0..N-1] of each face and of each W[N].  One warp per cell.
 template <int N>
-__global__ void k_record_i(long ncell, const double *__restrict__ rec, int2 *__restrict__ out,
-                           int *__restrict__ exps, int transpose, double rd, double rd_lo,
-                           double rw, double rw_lo) {
+__global__ void k_record_i(const OpParams<double> p, const double *__restrict__ rec,
+                           int2 *__restrict__ out, int *__restrict__ exps, int transpose, double rd,
+                           double rd_lo, double rw, double rw_lo) {
   using C = ICfg<N>;
   constexpr int PER = (C::RECI + 31) / 32;
   const long e = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (e >= ncell) return;
+  if (e >= p.ncell) return;
+  unsigned has = 0;   // faces with a neighbour
+  {
+    const unsigned q0 = p.div0.div((unsigned)e), q1 = p.div1.div(q0);
+    const int ix[3] = {(int)((unsigned)e - q0 * (unsigned)p.nc[0]),
+                       (int)(q0 - q1 * (unsigned)p.nc[1]), (int)q1};
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      has |= (ix[d] > 0 ? 1u << 2 * d : 0u) | (ix[d] + 1 < p.nc[d] ? 2u << 2 * d : 0u);
+  }
   const double *r = rec + e * C::RECW;
   double q[PER], q2[PER];
   unsigned m[13];   // group maxima: A', W1 of 6 faces, W2 of 6 faces
@@ -93,7 +110,7 @@ __global__ void k_record_i(long ncell, const double *__restrict__ rec, int2 *__r
       const int w = i - 3 * C::N2, f = w / (N + 1);
       last = w % (N + 1) == N;
       g = last ? 7 + f : 1 + f;
-      v = r[3 * C::N2 + (transpose ? C::NW : 0) + w];
+      v = has >> f & 1 ? r[3 * C::N2 + (transpose ? C::NW : 0) + w] : 0.0;
     }
     const double ri = last ? rw : rd, rl = last ? rw_lo : rd_lo;
     q[s] = v * ri;
@@ -129,7 +146,7 @@ __global__ void k_record_i(long ncell, const double *__restrict__ rec, int2 *__r
       if (j == g) eb = E[j];
     int2 v = make_int2(0, 0);
     if (ok && eb > 0) v = limbs(fix_signed(q[s], eb) + fix_signed(q2[s], eb));
-    out[e * C::RECI + i] = v;
+    out[limb_at<N>(e, C::RECI, i)] = v;
   }
   if (lane < C::NEXP) {
     int v = 0;
@@ -137,7 +154,7 @@ __global__ void k_record_i(long ncell, const double *__restrict__ rec, int2 *__r
     for (int j = 0; j < 13; j++)
       if (j == lane) v = m[j] ? E[j] - 1022 : kFixZero;
     if (lane == 13) v = ok;
-    exps[e * C::NEXP + lane] = v;
+    exps[limb_at<N>(e, C::NEXP, lane)] = v;
   }
 }
 
@@ -224,10 +241,12 @@ __device__ __noinline__ double apply_cells_fp64(const OpParams<double> &p,
   return part;
 }
 
-// 24 or 20 warps per SM.  64^3 Q2: 197 us with 64 threads per block, 204 with
-// 128, 222 with 256; 128 is kept at k = 2 because the fused sums of a small CG
-// pay for every block (24^3 Q2 CG 28.2 against 29.3 ms).  33x29x37 Q4 183 ->
-// 167 us with five blocks instead of the four the register count alone gives.
+// 24 or 20 warps per SM.  33x29x37 Q4 183 -> 167 us with five blocks instead of
+// the four the register count alone gives, 156 with the results put together on
+// the integer pipe.  Degree 2 has its own kernel (k_apply_p); the exchanges
+// through shared memory, 12 loads and stores per value there, are what it avoids
+// (204 -> 145 us at 64^3 Q2).  At degrees 3 and 4 a plane per thread is 16 or
+// 25 values with 96-bit sums, which does not fit the registers.
 template <int N>
 __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6)
     k_apply_i(const __grid_constant__ OpParams<double> p,
@@ -353,9 +372,8 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
       mac2(hh, mid, u, w[q]);
       if (q == ((f & 1) ? 0 : N - 1)) mac2(h2, m2, u, w[N]);
     }
-    const bool on = nbr[f] >= 0;
-    const long long s1 = on ? mac2_value(hh, mid, Etot - eu - ex[1 + f] - 2) : 0;
-    const long long s2 = on ? mac2_value(h2, m2, Etot - eu - ex[7 + f] - 2) : 0;
+    const long long s1 = mac2_value(hh, mid, Etot - eu - ex[1 + f] - 2);
+    const long long s2 = mac2_value(h2, m2, Etot - eu - ex[7 + f] - 2);
     if (f < 4) {
       fa[(2 * f) * TPC + l] = split32(s1);
       fa[(2 * f + 1) * TPC + l] = split32(s2);
@@ -453,10 +471,6 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
   // ---- out = M_z W + M_y T1 ----
   double part = 0.0;
   if (active) {
-    // one unit of the integers below as an FP64 factor (0: all of the cell's
-    // data is zero)
-    const double unit =
-        Etot > kFixZero + 1000 ? __hiloint2double((Etot + C::OUTE + 1023) << 20, 0) : 0.0;
     double *ye = a.y + (size_t)e * NB;
     const double *ad = a.add ? a.add + (size_t)e * NB : nullptr;
     const bool scale = a.alpha != 1.0;
@@ -468,7 +482,7 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
         s.add(W[q], int_m<N>(z * N + q));
         s.add(ue[z * N2 + q * N + tx], My[q]);
       }
-      double r = (double)s.template shifted<C::WIDE ? C::SHM : 0>() * unit;
+      double r = fix_to_double(s.template shifted<C::WIDE ? C::SHM : 0>(), Etot + C::OUTE);
       if (scale) r *= a.alpha;
       const int idx = z * TPC + l;
       if (a.accumulate) r += ye[idx];
@@ -481,16 +495,17 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
 }
 
 template <int N>
-static int record_i_n(pdg_context *ctx, int transpose) {
+static int record_i_n(pdg_context *ctx, const OpParams<double> &p, int transpose) {
   using C = ICfg<N>;
   int2 *&out = transpose ? ctx->reciT : ctx->reci;
   int *&ex = transpose ? ctx->reciT_exp : ctx->reci_exp;
-  if (!out) PDG_CUDA_TRY(cudaMalloc(&out, sizeof(int2) * C::RECI * ctx->ncell));
-  if (!ex) PDG_CUDA_TRY(cudaMalloc(&ex, sizeof(int) * C::NEXP * ctx->ncell));
+  const long cells = N == 3 ? (ctx->ncell + kGroup - 1) / kGroup * kGroup : ctx->ncell;
+  if (!out) PDG_CUDA_TRY(cudaMalloc(&out, sizeof(int2) * C::RECI * cells));
+  if (!ex) PDG_CUDA_TRY(cudaMalloc(&ex, sizeof(int) * C::NEXP * cells));
   const double den = (double)IntTab<N>::den * IntTab<N>::den, denw = den * IntTab<N>::dden;
   const double rd = 1.0 / den, rw = 1.0 / denw;
   const unsigned blocks = (unsigned)((ctx->ncell + 3) / 4);
-  k_record_i<N><<<blocks, 128, 0, ctx->stream>>>(ctx->ncell, ctx->rec64, out, ex, transpose, rd,
+  k_record_i<N><<<blocks, 128, 0, ctx->stream>>>(p, ctx->rec64, out, ex, transpose, rd,
                                                  std::fma(-rd, den, 1.0) / den, rw,
                                                  std::fma(-rw, denw, 1.0) / denw);
   PDG_CUDA_TRY(cudaGetLastError());
@@ -503,12 +518,13 @@ int prepare_apply_i(pdg_context *ctx, int transpose) {
   int &valid = transpose ? ctx->reciT_valid : ctx->reci_valid;
   if (valid) return PDG_OK;
   if (!ctx->rec_valid) return set_error(PDG_EINVAL, "limb records need the FP64 records");
+  const OpParams<double> p = make_params<double>(ctx, ctx->K64, ctx->c64, ctx->tab64);
   int st;
   switch (ctx->N) {
-    case 2: st = record_i_n<2>(ctx, transpose); break;
-    case 3: st = record_i_n<3>(ctx, transpose); break;
-    case 4: st = record_i_n<4>(ctx, transpose); break;
-    case 5: st = record_i_n<5>(ctx, transpose); break;
+    case 2: st = record_i_n<2>(ctx, p, transpose); break;
+    case 3: st = record_i_n<3>(ctx, p, transpose); break;
+    case 4: st = record_i_n<4>(ctx, p, transpose); break;
+    case 5: st = record_i_n<5>(ctx, p, transpose); break;
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
   }
   if (st == PDG_OK) valid = 1;
@@ -520,6 +536,20 @@ int prepare_apply_i(pdg_context *ctx, int transpose) {
 // irrational and keep the FP64 kernel.
 bool apply_i_usable(const pdg_context *ctx) {
   return ctx->dim == 3 && (ctx->basis != PDG_BASIS_LOBATTO || ctx->k <= 2);
+}
+
+// the fused CG: <p, A p> -> lambda in the same launch
+static ApplyArgs<double> fused(const pdg_context *ctx, const ApplyArgs<double> &a) {
+  ApplyArgs<double> af = a;
+  if (ctx->fuse_fin && a.ncells == 0) {
+    af.dot_part = ctx->fuse_part;
+    af.dot_max_blocks = ctx->fuse_max_blocks;
+    af.dot_cnt = ctx->fuse_cnt;
+    af.dot_scal = ctx->red_out;
+    af.dot_flags = ctx->d_flag;
+    af.dot_fin = ctx->fuse_fin;
+  }
+  return af;
 }
 
 template <int N>
@@ -535,18 +565,8 @@ static int launch_i_n(pdg_context *ctx, const ApplyArgs<double> &a, const OpPara
   const long work = a.ncells > 0 ? a.ncells : ctx->ncell;
   if (work <= 0) return PDG_OK;
   const unsigned blocks = (unsigned)((work + C::CPB - 1) / C::CPB);
-  ApplyArgs<double> af = a;
-  if (ctx->fuse_fin && a.ncells == 0) {
-    // the fused CG: <p, A p> -> lambda in the same launch
-    af.dot_part = ctx->fuse_part;
-    af.dot_max_blocks = ctx->fuse_max_blocks;
-    af.dot_cnt = ctx->fuse_cnt;
-    af.dot_scal = ctx->red_out;
-    af.dot_flags = ctx->d_flag;
-    af.dot_fin = ctx->fuse_fin;
-  }
   k_apply_i<N><<<blocks, C::THREADS, smem, ctx->stream>>>(
-      p, af, a.transpose ? ctx->reciT : ctx->reci, a.transpose ? ctx->reciT_exp : ctx->reci_exp,
+      p, fused(ctx, a), a.transpose ? ctx->reciT : ctx->reci, a.transpose ? ctx->reciT_exp : ctx->reci_exp,
       ctx->rec64);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
@@ -556,7 +576,7 @@ int launch_apply_i(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<
   PDG_TRY(prepare_apply_i(ctx, a.transpose));
   switch (ctx->N) {
     case 2: return launch_i_n<2>(ctx, a, p);
-    case 3: return launch_i_n<3>(ctx, a, p);
+    case 3: return launch_apply_p(ctx, fused(ctx, a), p);
     case 4: return launch_i_n<4>(ctx, a, p);
     case 5: return launch_i_n<5>(ctx, a, p);
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");

@@ -1,0 +1,508 @@
+// pdg_apply_p.cu -- the coupled 3D FP64 cell operator of degree 2 in 64-bit
+// fixed point, one plane of a cell per thread.
+//
+// Same operator and the same fixed-point arithmetic as k_apply_i
+// (pdg_apply_i.cu; reference: ConvectionDiffusionDG::jacobian_apply_volume /
+// _skeleton / _boundary, localoperator/convectiondiffusiondg.hh:191-195,
+// 474-481, 892-899).  k_apply_i gives a thread one line of a cell and
+// exchanges every intermediate array through shared memory, which at 27 values
+// per cell is most of its work.  Here
+//
+// * a block has 32 consecutive cells, warp z holds plane z of all of them
+//   (lanes are cells: 27 is odd, so 8-byte accesses of consecutive cells are
+//   free of bank conflicts, and everything that depends on z is uniform in a
+//   warp); the x and y contractions and their masses stay in registers, only
+//   the z contraction and the z mass read other planes;
+// * the block's cells, one halo cell at each end and the four runs of y and z
+//   neighbours are staged by bulk copies.  x neighbours are read as the limbs
+//   their own cell converted: the lines of a face cover the neighbour cell, so
+//   the cell's sums are aligned to that cell's largest value in any case;
+// * the small integers of the mass and derivative tables are compile-time
+//   constants (shifts and adds), and the sums of the masses fit 64 bits (see
+//   PCfg), so that IMAD.WIDE is left to the limb products;
+// * loops over the lines of a plane are not unrolled (65 KB of straight code
+//   missed the instruction cache), their results wait in the thread's own part
+//   of a run that is used up;
+// * results are put together on the integer pipe, and nothing is left of the
+//   FP64 pipe (operations that are predicated off take it as well).
+//
+// 64^3 Q2 (7.1 M DOF): k_apply_i 204 us, this one 179 as first written, 153
+// with the record prefetched to the L2 cache, no FP64 and 96 registers, 145 with
+// the loops rolled (57 MB in, 57 MB out and 123 MB of records need 35 us).  What
+// is left is the integer work (4100 instructions per warp, issue slots 58 %,
+// ALU 55 %, IMAD 52 % busy) at 18 warps per SM; 15 warps without any spill take
+// 171 us.
+#include <cmath>
+
+#include "pdg_fixed.cuh"
+#include "pdg_ops.cuh"
+#include "pdg_stage.cuh"
+#include "pdg_vec.cuh"
+
+namespace pdg {
+
+struct PCfg {
+  static constexpr int N = 3, N2 = 9, NB = 27, NF = 6;
+  static constexpr int T = kGroup, THREADS = N * T;   // cells, threads of a block
+  static constexpr int NW = NF * (N + 1), RECW = 3 * N2 + 2 * NW, RECI = 3 * N2 + NW;
+  static constexpr int NEXP = 16;                     // see k_record_i
+  static constexpr int LN = 2, LD = 2;                // ceil log2 of N and of max |d|
+  // a staged run carries up to one double of 16-byte phase
+  static constexpr int OWNP = ((T + 2) * NB + 2) / 2 * 2, RUNP = (T * NB + 2) / 2 * 2;
+  static constexpr int SMEM = OWNP + 4 * RUNP;
+  // X, Y, Z come below 0.75 2^61 (three terms under 2^(Etot - 2) in units of
+  // 2^(Etot - 61)).  Shifted by 2 and with mass row sums of 20 a mass stays
+  // below 15 2^59 < 2^63; shifted by 6 again, M_y X + M_x Y is below 0.47 2^59
+  // and M_x Z below 0.24 2^59, so the last sum is below 14.1 2^59 < 2^63.
+  static constexpr int SHX = 2, SHM = 6;
+  static constexpr int OUTE = -61 + SHX + SHM;
+};
+
+// v * c for a small integer constant
+template <int c>
+__device__ __forceinline__ long long times(long long v) {
+  return v * c;
+}
+// a run-time one: two 32-bit products
+__device__ __forceinline__ long long times(long long v, int c) {
+  return (long long)((unsigned long long)v * (unsigned long long)(long long)c);
+}
+template <int S>
+__device__ __forceinline__ long long round_shift(long long v) {
+  return (v + (1ll << (S - 1))) >> S;
+}
+
+// The plane's values in plain FP64 (weak form, from the FP64 record): not a
+// fast path, it keeps what FP64 gives for infinities, NaN and values near the
+// ends of the range.
+__device__ __noinline__ void apply_plane_fp64(const OpParams<double> &p, const ApplyArgs<double> &a,
+                                              const double *__restrict__ rec, int z, long e,
+                                              unsigned has, double *out) {
+  using C = PCfg;
+  constexpr int N = C::N, N2 = C::N2, NB = C::NB;
+  const double *tM = p.tab, *td0 = p.tab + 2 * N2, *td1 = td0 + N;
+  const double *r = rec + (size_t)e * C::RECW;
+  const double *W = r + 3 * N2 + (a.transpose ? C::NW : 0);
+  const int sk = a.transpose ? 1 : N, sq = a.transpose ? N : 1;
+  const double *u = a.x + e * NB;
+  const long stride[3] = {1, (long)p.nc[0], (long)p.nc[0] * p.nc[1]};
+  for (int i = 0; i < N2; i++) out[i] = 0.0;
+  // line through point o in direction dir (value distance d), result at k
+  const auto line = [&](int dir, int k, int o, int d) {
+    double s = 0.0;
+    for (int q = 0; q < N; q++) s += r[dir * N2 + k * sk + q * sq] * u[o + q * d];
+    for (int hi = 0; hi < 2; hi++) {
+      const int f = 2 * dir + hi;
+      if (!(has >> f & 1)) continue;
+      const double *un = u + (hi ? 1 : -1) * stride[dir] * NB;
+      double s1 = 0.0;
+      for (int q = 0; q < N; q++) s1 += W[f * (N + 1) + q] * un[o + q * d];
+      if (k == (hi ? N - 1 : 0)) s += s1;
+      s += (hi ? td1 : td0)[k] * (W[f * (N + 1) + N] * un[o + (hi ? 0 : N - 1) * d]);
+    }
+    return s;
+  };
+  for (int zz = 0; zz < N; zz++)
+    for (int y = 0; y < N; y++)
+      for (int x = 0; x < N; x++) {
+        const double X = line(0, x, zz * N2 + y * N, 1), Y = line(1, y, zz * N2 + x, N);
+        for (int j = 0; j < N; j++) {
+          out[j * N + x] += tM[z * N + zz] * (tM[j * N + y] * X);
+          out[y * N + j] += tM[z * N + zz] * (tM[j * N + x] * Y);
+        }
+      }
+  for (int y = 0; y < N; y++)
+    for (int x = 0; x < N; x++) {
+      const double Z = line(2, z, y * N + x, N2);
+      for (int j = 0; j < N; j++)
+        for (int i = 0; i < N; i++) out[j * N + i] += tM[j * N + y] * (tM[i * N + x] * Z);
+    }
+}
+
+// sums of a neighbour line against its face coefficients w (W[0..N-1], W[N]),
+// aligned to the cell
+template <bool kHi>
+__device__ __forceinline__ void face_line(const int2 (&u)[PCfg::N], const int2 (&w)[PCfg::N + 1],
+                                          int sh1, int sh2, long long &s1, long long &s2) {
+  constexpr int N = PCfg::N;
+  long long hh = 0, mid = 0, h2 = 0, m2 = 0;
+#pragma unroll
+  for (int q = 0; q < N; q++) mac2(hh, mid, u[q], w[q]);
+  mac2(h2, m2, u[kHi ? 0 : N - 1], w[N]);
+  s1 = mac2_value(hh, mid, sh1);
+  s2 = mac2_value(h2, m2, sh2);
+}
+
+// a line with compile-time derivative tables: A' u plus the lifts of both faces
+__device__ __forceinline__ void line_sums(const int2 (&A)[PCfg::N2], const int2 (&u)[PCfg::N],
+                                          int shu, long long s1l, long long s2l, long long s1h,
+                                          long long s2h, long long (&X)[PCfg::N]) {
+  constexpr int N = PCfg::N;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    long long hh = 0, mid = 0;
+#pragma unroll
+    for (int q = 0; q < N; q++) mac2(hh, mid, A[i * N + q], u[q]);
+    X[i] = mac2_value(hh, mid, shu) + s2l * int_d0<N>(i) + s2h * int_d1<N>(i);
+  }
+  X[0] += s1l;
+  X[N - 1] += s1h;
+#pragma unroll
+  for (int i = 0; i < N; i++) X[i] = round_shift<PCfg::SHX>(X[i]);
+}
+
+__global__ void __launch_bounds__(PCfg::THREADS, 6)
+    k_apply_p(const __grid_constant__ OpParams<double> p,
+              const __grid_constant__ ApplyArgs<double> a, const int2 *__restrict__ rec,
+              const int *__restrict__ exps, const double *__restrict__ rec64, int *tma_err) {
+  using C = PCfg;
+  constexpr int N = C::N, N2 = C::N2, NB = C::NB, T = C::T, NF = C::NF;
+  extern __shared__ __align__(16) double smd[];
+  __shared__ __align__(8) unsigned long long bar;
+  __shared__ int eO[N][T + 2], eC[N][T];
+  if (a.skip && *a.skip) return;
+  const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
+  const long ncell = p.ncell, ndof = ncell * NB;
+  const long c0 = a.ncells > 0 ? a.cell0 : 0, c1 = a.ncells > 0 ? c0 + a.ncells : ncell;
+  const long group = blockIdx.x + c0 / T, e0 = group * T, e = e0 + lane;
+  const bool active = e >= c0 && e < c1;
+  const long sx = p.nc[0], sxy = (long)p.nc[0] * p.nc[1];
+
+  // the group's record to the L2 cache while the exponents are formed
+  if (threadIdx.x == 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rec +
+                                                                    (size_t)group * C::RECI * T),
+                 "r"((unsigned)(sizeof(int2) * C::RECI * T))
+                 : "memory");
+  Stager<C::THREADS, double> st(&bar);
+  double *OWN = st.run(smd, a.x, (e0 - 1) * NB, ndof, (T + 2) * NB);
+  double *YL = st.run(smd + C::OWNP, a.x, (e0 - sx) * NB, ndof, T * NB);
+  double *YH = st.run(smd + C::OWNP + C::RUNP, a.x, (e0 + sx) * NB, ndof, T * NB);
+  double *ZL = st.run(smd + C::OWNP + 2 * C::RUNP, a.x, (e0 - sxy) * NB, ndof, T * NB);
+  double *ZH = st.run(smd + C::OWNP + 3 * C::RUNP, a.x, (e0 + sxy) * NB, ndof, T * NB);
+
+  bool has[NF];
+  {
+    const unsigned ee = e < ncell ? (unsigned)e : 0u;
+    const unsigned q0 = p.div0.div(ee);
+    const unsigned q1 = p.div1.div(q0);
+    const int ix[3] = {(int)(ee - q0 * (unsigned)p.nc[0]), (int)(q0 - q1 * (unsigned)p.nc[1]),
+                       (int)q1};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      has[2 * d] = ix[d] > 0;
+      has[2 * d + 1] = ix[d] + 1 < p.nc[d];
+    }
+  }
+  const int2 *r = rec + (size_t)group * C::RECI * T + lane;   // [coefficient][cell of the group]
+  const int *ex = exps + (size_t)group * C::NEXP * T + lane;
+  // exponents of W[0..N-1] (low half) and W[N] of the faces
+  int EF[NF];
+#pragma unroll
+  for (int f = 0; f < NF; f++)
+    EF[f] = (ex[(1 + f) * T] & 0xffff) | (int)((unsigned)ex[(1 + NF + f) * T] << 16);
+  const auto ef1 = [&](int f) { return (int)(short)EF[f]; };
+  const auto ef2 = [&](int f) { return EF[f] >> 16; };
+  const int EA = ex[0];
+  bool bad = ex[13 * T] == 0;
+  if (!st.wait()) {
+    if (threadIdx.x == 0) atomicExch(tma_err, 1);
+    return;
+  }
+
+  // ---- exponents: own plane, the y neighbours' plane z, row z of all planes
+  // of the z neighbours ----
+  constexpr int kNotFinite = 5000;
+  const auto code = [](const BlockExp &b) { return b.finite() ? b.exponent() : kNotFinite; };
+  double *U = OWN + (lane + 1) * NB + z * N2, *YLp = YL + lane * NB + z * N2,
+         *YHp = YH + lane * NB + z * N2, *ZLp = ZL + lane * NB + z * N,
+         *ZHp = ZH + lane * NB + z * N;
+  double col[N2];
+  int eb[4];   // biased exponents of the y and z neighbours' data
+  {
+    BlockExp own;
+#pragma unroll
+    for (int i = 0; i < N2; i++) {
+      col[i] = U[i];
+      own.add(col[i]);
+    }
+    eO[z][lane + 1] = code(own);
+    int cand = 2 * kFixZero;
+#pragma unroll
+    for (int f = 2; f < NF; f++) {
+      const double *v = f == 2 ? YLp : f == 3 ? YHp : f == 4 ? ZLp : ZHp;
+      BlockExp b;
+#pragma unroll
+      for (int i = 0; i < N2; i++) b.add(v[f < 4 ? i : (i / N) * N2 + i % N]);
+      eb[f - 2] = b.biased();
+      if (has[f]) {
+        bad |= !b.finite();
+        // |e_i s1 + d_i s2| over the face's two terms
+        cand = max(cand, b.exponent() + max(ef1(f) + C::LN, ef2(f) + C::LD) + 1);
+      }
+    }
+    eC[z][lane] = cand;
+  }
+  // the halo cells' limbs: warp 0 the lower, warp 1 the upper one
+  if (z < 2) {
+    const int slot = z == 0 ? 0 : T + 1;
+    const long eh = e0 - 1 + slot;
+    int c = kFixZero;
+    if (eh >= 0 && eh < ncell) {
+      const double h = lane < NB ? OWN[slot * NB + lane] : 0.0;
+      BlockExp b;
+      b.add(h);
+      b.m = __reduce_max_sync(0xffffffffu, b.m);
+      b.any = __reduce_or_sync(0xffffffffu, b.any);
+      c = code(b);
+      if (lane < NB)
+        reinterpret_cast<int2 *>(OWN)[slot * NB + lane] = fix_limbs(h, b.biased());
+    }
+    if (lane < N) eO[lane][slot] = c;
+  }
+  __syncthreads();
+  int Exl = kFixZero, Ex = kFixZero, Exh = kFixZero, cand = 2 * kFixZero;
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    Exl = max(Exl, eO[q][lane]);
+    Ex = max(Ex, eO[q][lane + 1]);
+    Exh = max(Exh, eO[q][lane + 2]);
+    cand = max(cand, eC[q][lane]);
+  }
+  bad |= Ex == kNotFinite;
+  if (has[0]) {
+    bad |= Exl == kNotFinite;
+    cand = max(cand, Exl + max(ef1(0) + C::LN, ef2(0) + C::LD) + 1);
+  }
+  if (has[1]) {
+    bad |= Exh == kNotFinite;
+    cand = max(cand, Exh + max(ef1(1) + C::LN, ef2(1) + C::LD) + 1);
+  }
+  // three terms (volume, two faces) per direction
+  const int Etot = max(Ex + EA + C::LN, cand) + 2;
+  bad |= Etot > 900 || (Etot > kFixZero + 1000 && Etot < -780);
+  bad &= active;
+
+  // ---- own plane to limbs, in place ----
+  int2 *Up = reinterpret_cast<int2 *>(U);
+  {
+    const int ebx = max(Ex + 1022, kFixMinBiased);
+#pragma unroll
+    for (int i = 0; i < N2; i++) Up[i] = fix_limbs(col[i], ebx);
+  }
+  if (__syncthreads_or(bad)) {
+    unsigned mask = 0;
+#pragma unroll
+    for (int f = 0; f < NF; f++) mask |= (unsigned)has[f] << f;
+    if (active) apply_plane_fp64(p, a, rec64, z, e, mask, YHp);
+  } else {
+    const int shu = Etot - Ex - EA - 2;
+    // ---- y: M_x Y, over the YL plane (read by this thread only) ----
+    long long *W = reinterpret_cast<long long *>(YLp);
+    {
+      const int eul = eb[0] - 1022, euh = eb[1] - 1022;
+      const int sl1 = Etot - eul - ef1(2) - 2, sl2 = Etot - eul - ef2(2) - 2;
+      const int sh1 = Etot - euh - ef1(3) - 2, sh2 = Etot - euh - ef2(3) - 2;
+      int2 A[N2], wl[N + 1], wh[N + 1];
+#pragma unroll
+      for (int i = 0; i < N2; i++) A[i] = r[(N2 + i) * T];
+#pragma unroll
+      for (int i = 0; i <= N; i++) {
+        wl[i] = r[(3 * N2 + 2 * (N + 1) + i) * T];
+        wh[i] = r[(3 * N2 + 3 * (N + 1) + i) * T];
+      }
+#pragma unroll 1
+      for (int x = 0; x < N; x++) {
+        int2 u[N], l[N], h[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+          u[q] = Up[q * N + x];
+          l[q] = fix_limbs(YLp[q * N + x], eb[0]);
+          h[q] = fix_limbs(YHp[q * N + x], eb[1]);
+        }
+        long long s1l, s2l, s1h, s2h, Y[N];
+        face_line<false>(l, wl, sl1, sl2, s1l, s2l);
+        face_line<true>(h, wh, sh1, sh2, s1h, s2h);
+        line_sums(A, u, shu, s1l, s2l, s1h, s2h, Y);
+#pragma unroll
+        for (int y = 0; y < N; y++) W[y * N + x] = Y[y];
+      }
+#pragma unroll
+      for (int y = 0; y < N; y++) {
+        long long v[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) v[q] = W[y * N + q];
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+          long long s = 0;
+#pragma unroll
+          for (int q = 0; q < N; q++) s += v[q] * int_m<N>(j * N + q);
+          W[y * N + j] = round_shift<C::SHM>(s);
+        }
+      }
+    }
+    // ---- x: W = M_y X + M_x Y; scratch and the result over the YH plane ----
+    long long *S = reinterpret_cast<long long *>(YHp);
+    {
+      const int sl1 = Etot - Exl - ef1(0) - 2, sl2 = Etot - Exl - ef2(0) - 2;
+      const int sh1 = Etot - Exh - ef1(1) - 2, sh2 = Etot - Exh - ef2(1) - 2;
+      int2 A[N2], wl[N + 1], wh[N + 1];
+#pragma unroll
+      for (int i = 0; i < N2; i++) A[i] = r[i * T];
+#pragma unroll
+      for (int i = 0; i <= N; i++) {
+        wl[i] = r[(3 * N2 + i) * T];
+        wh[i] = r[(3 * N2 + (N + 1) + i) * T];
+      }
+#pragma unroll 1
+      for (int y = 0; y < N; y++) {
+        int2 u[N], l[N], h[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+          u[q] = Up[y * N + q];
+          l[q] = Up[y * N + q - NB];
+          h[q] = Up[y * N + q + NB];
+        }
+        long long s1l, s2l, s1h, s2h, X[N];
+        face_line<false>(l, wl, sl1, sl2, s1l, s2l);
+        face_line<true>(h, wh, sh1, sh2, s1h, s2h);
+        line_sums(A, u, shu, s1l, s2l, s1h, s2h, X);
+#pragma unroll
+        for (int x = 0; x < N; x++) S[y * N + x] = X[x];
+      }
+#pragma unroll
+      for (int x = 0; x < N; x++)
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+          long long s = 0;
+#pragma unroll
+          for (int q = 0; q < N; q++) s += S[q * N + x] * int_m<N>(j * N + q);
+          W[j * N + x] += round_shift<C::SHM>(s);
+        }
+    }
+    // ---- z faces of row z: over the values read (s1 in plane 0, s2 in plane 1) ----
+    {
+      const int eul = eb[2] - 1022, euh = eb[3] - 1022;
+      const int sl1 = Etot - eul - ef1(4) - 2, sl2 = Etot - eul - ef2(4) - 2;
+      const int sh1 = Etot - euh - ef1(5) - 2, sh2 = Etot - euh - ef2(5) - 2;
+      int2 wl[N + 1], wh[N + 1];
+#pragma unroll
+      for (int i = 0; i <= N; i++) {
+        wl[i] = r[(3 * N2 + 4 * (N + 1) + i) * T];
+        wh[i] = r[(3 * N2 + 5 * (N + 1) + i) * T];
+      }
+#pragma unroll 1
+      for (int x = 0; x < N; x++) {
+        int2 l[N], h[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+          l[q] = fix_limbs(ZLp[q * N2 + x], eb[2]);
+          h[q] = fix_limbs(ZHp[q * N2 + x], eb[3]);
+        }
+        long long s1l, s2l, s1h, s2h;
+        face_line<false>(l, wl, sl1, sl2, s1l, s2l);
+        face_line<true>(h, wh, sh1, sh2, s1h, s2h);
+        reinterpret_cast<long long *>(ZLp)[x] = s1l;
+        reinterpret_cast<long long *>(ZLp)[N2 + x] = s2l;
+        reinterpret_cast<long long *>(ZHp)[x] = s1h;
+        reinterpret_cast<long long *>(ZHp)[N2 + x] = s2h;
+      }
+    }
+    __syncthreads();
+    // ---- out = M_z W + M_y M_x Z ----
+    {
+      const int d0 = z == 0 ? int_d0<N>(0) : z == 1 ? int_d0<N>(1) : int_d0<N>(2);
+      const int d1 = z == 0 ? int_d1<N>(0) : z == 1 ? int_d1<N>(1) : int_d1<N>(2);
+      const int2 *Uc = reinterpret_cast<const int2 *>(OWN + (lane + 1) * NB);
+      int2 A[N];
+#pragma unroll
+      for (int q = 0; q < N; q++) A[q] = r[(2 * N2 + z * N + q) * T];
+      const long long *fl = reinterpret_cast<const long long *>(ZL + lane * NB),
+                      *fh = reinterpret_cast<const long long *>(ZH + lane * NB);
+#pragma unroll 1
+      for (int y = 0; y < N; y++) {
+        long long Z[N];
+#pragma unroll
+        for (int x = 0; x < N; x++) {
+          const int i = y * N + x;
+          long long hh = 0, mid = 0;
+#pragma unroll
+          for (int q = 0; q < N; q++) mac2(hh, mid, A[q], Uc[q * N2 + i]);
+          long long s = mac2_value(hh, mid, shu) + times(fl[N2 + i], d0) + times(fh[N2 + i], d1);
+          if (z == 0) s += fl[i];
+          if (z == N - 1) s += fh[i];
+          Z[x] = round_shift<C::SHX>(s);
+        }
+#pragma unroll
+        for (int x = 0; x < N; x++) {
+          long long t = 0;
+#pragma unroll
+          for (int q = 0; q < N; q++) t += Z[q] * int_m<N>(x * N + q);
+          S[y * N + x] = round_shift<C::SHM>(t);
+        }
+      }
+    }
+    const long long *Wc = reinterpret_cast<const long long *>(YL + lane * NB);
+    // row z of the mass matrix: 4 2 -1, 2 16 2, -1 2 4
+    const int m0 = z == 0 ? int_m<N>(0) : z == 1 ? int_m<N>(3) : int_m<N>(2),
+              m1 = z == 1 ? int_m<N>(4) : int_m<N>(1),
+              m2 = z == 0 ? int_m<N>(2) : z == 1 ? int_m<N>(3) : int_m<N>(0);
+#pragma unroll
+    for (int x = 0; x < N; x++) {
+      long long t[N];
+#pragma unroll
+      for (int q = 0; q < N; q++) t[q] = S[q * N + x];
+#pragma unroll
+      for (int j = 0; j < N; j++) {
+        const int i = j * N + x;
+        long long s = times(Wc[i], m0) + times(Wc[N2 + i], m1) + times(Wc[2 * N2 + i], m2);
+#pragma unroll
+        for (int q = 0; q < N; q++) s += t[q] * int_m<N>(j * N + q);
+        YHp[i] = fix_to_double(s, Etot + C::OUTE);
+      }
+    }
+  }
+  __syncthreads();
+  // ---- coalesced write-back; <x, y_out> of the fused CG ----
+  const long g0 = max(e0, c0) * NB, g1 = min(e0 + T, c1) * NB;
+  const double *Os = YH - e0 * NB;
+  double part = 0.0;
+  // (FP64 operations that are predicated off still take the pipe)
+  if (a.alpha == 1.0 && !a.accumulate && !a.add) {
+    for (long g = g0 + threadIdx.x; g < g1; g += C::THREADS) a.y[g] = Os[g];
+    if (a.dot_part)
+      for (long g = g0 + threadIdx.x; g < g1; g += C::THREADS) part += a.x[g] * Os[g];
+  } else {
+    for (long g = g0 + threadIdx.x; g < g1; g += C::THREADS) {
+      double v = a.alpha * Os[g];
+      if (a.accumulate) v += a.y[g];
+      if (a.add) v += a.add[g];
+      if (a.dot_part) part += a.x[g] * v;
+      a.y[g] = v;
+    }
+  }
+  if (a.dot_part)
+    reduce_tail_grouped<C::THREADS>(a.dot_part, a.dot_max_blocks, a.dot_cnt,
+                                    RedCtx{nullptr, a.dot_scal, a.dot_flags}, part, 0.0,
+                                    a.dot_fin);
+}
+
+int launch_apply_p(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<double> &p) {
+  using C = PCfg;
+  const size_t smem = sizeof(double) * C::SMEM;
+  static int attr_dev = -1;
+  if (attr_dev != ctx->device) {
+    PDG_CUDA_TRY(
+        cudaFuncSetAttribute(k_apply_p, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_dev = ctx->device;
+  }
+  const long c0 = a.ncells > 0 ? a.cell0 : 0, c1 = a.ncells > 0 ? c0 + a.ncells : ctx->ncell;
+  const unsigned blocks = (unsigned)((c1 - 1) / C::T - c0 / C::T + 1);
+  k_apply_p<<<blocks, C::THREADS, smem, ctx->stream>>>(
+      p, a, a.transpose ? ctx->reciT : ctx->reci, a.transpose ? ctx->reciT_exp : ctx->reci_exp,
+      ctx->rec64, ctx->d_flag + F_TMA);
+  PDG_CUDA_TRY(cudaGetLastError());
+  return PDG_OK;
+}
+
+}  // namespace pdg

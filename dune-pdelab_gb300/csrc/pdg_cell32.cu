@@ -30,7 +30,7 @@
 #include <cstdint>
 
 #include "pdg_ops.cuh"
-#include "pdg_tma.cuh"
+#include "pdg_stage.cuh"
 #include "pdg_vec.cuh"
 
 namespace pdg {
@@ -90,53 +90,6 @@ __global__ void k_record_c32(const OpParams<double> p, float *__restrict__ rec) 
     }
   }
 }
-
-// Staging of a block's input runs.  A run of source elements [g0, g0 + count)
-// lands at dst[ph + i], ph = g0 mod 4, so that source and destination share
-// their 16-byte phase.  Runs inside [0, lim) of an aligned source are one bulk
-// copy by thread 0, completing on `bar` (per-thread copies of all runs cost the
-// operator about 900 of its 3800 instructions per warp); runs that straddle an
-// end are copied element-wise with zeros outside, runs outside are left out
-// (an absent neighbour is read from a zero block).  All threads call it, then
-// wait().
-template <int T>
-struct Stager {
-  unsigned bar, bytes;
-  __device__ __forceinline__ explicit Stager(unsigned long long *b) : bar(smem_u32(b)), bytes(0) {
-    if (threadIdx.x == 0) mbar_init(bar, 1);
-    __syncthreads();
-  }
-  __device__ __forceinline__ float *run(float *dst, const float *src, long g0, long lim,
-                                        int count) {
-    const int ph = (int)(((g0 % 4) + 4) % 4);
-    const long ga = g0 - ph;
-    const int len = (ph + count + 3) & ~3;
-    if (ga + len <= 0 || ga >= lim) return dst + ph;
-    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && ga >= 0 && ga + len <= lim) {
-      if (threadIdx.x == 0) {
-        // every copy is announced before it is issued; the phase completes
-        // with the arrival in wait()
-        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar),
-                     "r"(4u * len)
-                     : "memory");
-        bulk_load(smem_u32(dst), src + ga, 4u * len, bar);
-      }
-    } else {
-      for (int c = threadIdx.x; c < len; c += T) {
-        const long g = ga + c;
-        dst[c] = (g >= 0 && g < lim) ? src[g] : 0.f;
-      }
-    }
-    return dst + ph;
-  }
-  // false: the copies did not arrive within the poll limit
-  __device__ __forceinline__ bool wait() {
-    if (threadIdx.x == 0)
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-    const bool ok = mbar_wait(bar, 0, kTmaPolls);
-    return __syncthreads_and(ok);
-  }
-};
 
 // coefficients of a face in the form of this launch: {a1 kappa_e, a1 kappa_o,
 // penalty, a2 kappa_e} with (a1, a2) = (1, -theta), transposed (-theta, 1)
@@ -246,7 +199,7 @@ __global__ void __launch_bounds__(C32Cfg<N>::THREADS)
 #pragma unroll
   for (int k = 0; k < C::REC; k++) R[k] = rec[k * p.ncell + (active ? e : 0)];
 
-  Stager<C::THREADS> st(&bar);
+  Stager<C::THREADS, float> st(&bar);
   float *Y0 = sm + 2 * C::OWNP;
   const float *O0 = st.run(sm, a.x, (e0 - 1) * NB, ndof, C::OWN);
   const float *O1 = st.run(sm + C::OWNP, a.x, (e0 + dz - 1) * NB, ndof, C::OWN);
@@ -466,7 +419,7 @@ __global__ void __launch_bounds__(C32Cfg<N>::T, 9)
   const long e0 = (long)blockIdx.x * T, ndof = ncell * NB;
   float *Q0 = sm + 2 * C::RUNP, *L0 = Q0 + (T * 3 * N2 + 7) / 4 * 4;
   __shared__ __align__(8) unsigned long long bar;
-  Stager<T> st(&bar);
+  Stager<T, float> st(&bar);
   // runs start at multiples of 64: no phase
   st.run(sm, d, e0 * NB, ndof, C::RUN);
   if (rq) st.run(sm + C::RUNP, rq, e0 * NB, ndof, C::RUN);

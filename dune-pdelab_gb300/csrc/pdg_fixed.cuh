@@ -20,6 +20,7 @@
 namespace pdg {
 
 constexpr int kFixBits = 57;        // |X| < 2^kFixBits
+constexpr int kGroup = 32;          // cells of a group of the degree-2 limb records
 constexpr int kFixZero = -5000;     // exponent of an all-zero block
 constexpr int kFixMinBiased = 64;   // smallest biased exponent a block is scaled to
 
@@ -154,5 +155,19 @@ template <> struct SmallSum<true> {
     return (long long)((unsigned long long)hi << (32 - S)) + (lo >> S);
   }
 };
+
+// v 2^E rounded to the nearest double (|v| < 2^63, the result in the normal
+// range or v = 0), put together on the integer pipe: the conversion of a 64-bit
+// integer is six FP64-pipe operations of 64 cycles per warp and sub-partition
+__device__ __forceinline__ double fix_to_double(long long v, int E) {
+  unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+  const int lz = __clzll((long long)m);
+  m <<= (lz & 63);
+  // 1.f 2^(63 - lz + E); the leading one of m >> 11 adds one to the exponent field
+  const unsigned long long bits =
+      ((unsigned long long)(unsigned)(63 - lz + E + 1022) << 52) + (m >> 11) + ((m >> 10) & 1);
+  const int hi = (int)(bits >> 32) | ((int)(v >> 32) & (int)0x80000000);
+  return v == 0 ? 0.0 : __hiloint2double(hi, (int)bits);
+}
 
 }  // namespace pdg

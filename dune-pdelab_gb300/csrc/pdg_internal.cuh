@@ -408,6 +408,8 @@ int prepare_apply_m(pdg_context *ctx, int transpose);
 bool apply_i_usable(const pdg_context *ctx);
 int launch_apply_i(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<double> &p);
 int prepare_apply_i(pdg_context *ctx, int transpose);
+// degree 2 of it, one plane of a cell per thread (pdg_apply_p.cu)
+int launch_apply_p(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<double> &p);
 
 // the iterations of a small 2D FP64 CG solve in one launch (pdg_cg2d.cu); *ran
 // false: the grid does not fit, nothing was launched

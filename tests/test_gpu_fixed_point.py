@@ -209,3 +209,37 @@ def test_convection_non_finite():
         else:
             assert np.max(np.abs(y[c] - ref[c])) <= 1e-12 * np.max(np.abs(ref))
     go.close()
+
+
+@pytest.mark.parametrize("n", [(32, 1, 1), (33, 1, 1), (11, 3, 2), (5, 8, 2), (9, 7, 5)])
+def test_degree2_groups(n):
+    """Degree 2 works on groups of 32 cells (pdg_apply_p.cu): one more than a
+    group, rows and planes that straddle groups, both forms."""
+    test_sizes(2, n)
+
+
+@pytest.mark.parametrize("e", [31, 32, 63])
+def test_degree2_non_finite_at_group_ends(e):
+    go, P, rng = problem(2, (70, 1, 1))
+    x = rng.uniform(-1, 1, (go.ncell, go.nbasis))
+    ref = P.jacobian_apply(x.ravel()).reshape(go.ncell, -1)
+    x[e] = np.nan
+    y = apply(go, x.ravel()).reshape(go.ncell, -1)
+    for c in range(go.ncell):
+        if abs(c - e) <= 1:
+            assert not np.isfinite(y[c]).any()
+        else:
+            assert np.max(np.abs(y[c] - ref[c])) <= 1e-12 * np.max(np.abs(ref))
+    go.close()
+
+
+def test_degree2_ranges():
+    """Host vectors run in slabs that start inside a group: the same bits as
+    one launch."""
+    import torch
+    go, P, rng = problem(2, (33, 31, 33))
+    x = rng.uniform(-1, 1, go.ndof)
+    xd, yd = torch.from_numpy(x).cuda(), torch.zeros(go.ndof, dtype=torch.float64, device="cuda")
+    pdg.OnTheFlyOperator(go).apply(xd, yd)
+    assert np.array_equal(apply(go, x), yd.cpu().numpy())
+    go.close()
