@@ -1630,13 +1630,19 @@ static int ensure_stage(pdg_context *ctx) {
 
 // ---- host-buffer applies pipelined over slabs of cells --------------------
 // Copying x in, applying and copying y out one after another costs the copies
-// on top of the kernel.  The grid is cut into slabs of whole planes of the
-// slowest direction (contiguous cell and DOF ranges); slab s is applied once
-// slabs s and s+1 are on the device (its faces read one neighbour plane) and
-// copied out while slab s+1 is applied, so the copies in, the kernels and the
-// copies out overlap, ordered by events.  Consecutive slabs are applied on
-// two alternating streams: they write disjoint ranges of y, and the last,
-// partly filled wave of one slab's grid overlaps the first of the next.
+// on top of the kernel.  x is copied in slabs of whole planes of the slowest
+// direction (contiguous DOF ranges); the cells one plane behind a copy (a cell
+// reads the next plane) are applied as soon as it has arrived, while the next
+// slab is copied.  A result in pinned memory is stored there by the kernel
+// itself (degree 2 in 3D): the stores take the link's other direction at the rate of a copy
+// (57 MB: 297 and 296 us) without one copy, one event and one wait per slab.
+// Otherwise each slab's result is copied out while the next is applied.
+// Consecutive slabs are applied on two alternating streams: they write disjoint
+// ranges of y, and the last, partly filled wave of one slab's grid overlaps the
+// first of the next.
+// 64^3 Q2, 57 MB each way: copies out and slabs two planes apart 540 us, stores
+// 491, and with the ranges above and 7 slabs instead of 16 475 (a copy in beside
+// the stores alone takes 390, a copy each way 341, in 16 parts 402).
 constexpr int kMaxSlabs = kPipeMaxSlabs;
 static_assert(sizeof(pdg_context::pipe_ev) / sizeof(cudaEvent_t) == 2 * kMaxSlabs + 3,
               "one event per slab each way, plus start, end and the second stream's");
@@ -1658,16 +1664,35 @@ static int pipe_ready(pdg_context *ctx) {
   return PDG_OK;
 }
 
-// number of slabs (1: no pipelining) and planes per slab
+// number of slabs (1: no pipelining) and planes per slab.  A slab costs about
+// 4 us, the first copy and the last kernel overlap nothing: with time T of the
+// whole copy 4 n + T / n is least at n = sqrt(T / 4 us), about one per MB
+// under the root (64^3 Q2, 57 MB: 4, 5, 6, 7, 8, 16 slabs take 484, 475, 476,
+// 474, 488, 493 us).
 static int pipe_slabs(const pdg_context *ctx, long *planes_per_slab) {
   const long planes = ctx->cfg.cells[ctx->dim - 1];
-  long s = ctx->ncell / kMinSlabCells;
+  long s = std::min(ctx->ncell / kMinSlabCells,
+                    (long)std::sqrt(sizeof(double) * (double)ctx->ndof / 1e6));
   if (s > kMaxSlabs) s = kMaxSlabs;
   if (s > planes) s = planes;
   if (s < 2) return 1;
   const long pps = (planes + s - 1) / s;
   *planes_per_slab = pps;
   return (int)((planes + pps - 1) / pps);
+}
+
+// the device's address of n doubles of pinned host memory, or null
+static double *mapped_host(const double *p, size_t n) {
+  cudaPointerAttributes a, b;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&b, p + (n - 1)) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
+      (double *)b.devicePointer != (double *)a.devicePointer + (n - 1))
+    return nullptr;
+  return (double *)a.devicePointer;
 }
 
 // y = (acc ? y : 0) + alpha J x + add with x and/or y in host memory;
@@ -1688,6 +1713,13 @@ static int apply_pipelined(pdg_context *ctx, const double *x, double *y, const d
   PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->pipe_d2h, ev_start, 0));
   PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->pipe_k2, ev_start, 0));
   cudaStream_t const ctx_stream = ctx->stream;
+  // k_apply_p stores runs of whole cells; the other kernels' stores of 32 to 200
+  // contiguous bytes are too short for the link (128^3 Q1 2045 against 985 us with
+  // copies, 32^3 Q4 398 against 347 us, 512^2 Q2 422 against 233 us)
+  const bool runs = ctx->N == 3 && apply_i_usable(ctx) && !ctx->f64_pair &&
+                    !general_coefficients(ctx) && !convection_on(ctx);
+  double *const ymap = hy && !acc && runs ? mapped_host(y, ctx->ndof) : nullptr;
+  if (ymap) ydev = ymap;
   auto range = [&](int s, long *c0, long *c1) {
     *c0 = s * pps * plane;
     *c1 = std::min(ctx->ncell, (s + 1) * pps * plane);
@@ -1706,17 +1738,19 @@ static int apply_pipelined(pdg_context *ctx, const double *x, double *y, const d
   }
   int st = PDG_OK;
   for (int s = 0; s < nslab && st == PDG_OK; s++) {
+    // one plane behind the copy: a cell reads the next plane
     long c0, c1;
     range(s, &c0, &c1);
+    if (s > 0) c0 -= plane;
+    if (s + 1 < nslab) c1 -= plane;
+    if (c1 == c0) continue;
     // the launchers enqueue on ctx->stream: point it at this slab's stream
     ctx->stream = (s & 1) ? ctx->pipe_k2 : ctx_stream;
-    if ((st = cuda_status(cudaStreamWaitEvent(ctx->stream, ev_in[std::min(s + 1, nslab - 1)],
-                                              0))))
-      break;
+    if ((st = cuda_status(cudaStreamWaitEvent(ctx->stream, ev_in[s], 0)))) break;
     ApplyArgs<double> a{xdev, ydev, add, alpha, acc, transpose, 0, nullptr, nullptr,
                         (int)(c1 - c0), (int)c0};
     if ((st = launch_apply<double>(ctx, a, ctx->K64, ctx->c64, ctx->tab64))) break;
-    if (hy) {
+    if (hy && !ymap) {
       const size_t off = (size_t)(c0 * nb), bytes = sizeof(double) * (size_t)((c1 - c0) * nb);
       if ((st = cuda_status(cudaEventRecord(ev_out[s], ctx->stream))) ||
           (st = cuda_status(cudaStreamWaitEvent(ctx->pipe_d2h, ev_out[s], 0))) ||
