@@ -938,6 +938,7 @@ static void invalidate(pdg_context *ctx, bool operator_changed) {
     ctx->rec64mT_valid = 0;
     ctx->reci_valid = 0;
     ctx->reciT_valid = 0;
+    ctx->rect_valid = 0;
     ctx->recfp_valid = 0;
     ctx->rec32_valid = 0;
     ctx->rec32q_valid = 0;
@@ -1253,7 +1254,8 @@ int pdg_destroy(pdg_context *c) {
                   c->fuse_part, c->fuse_cnt, c->Ac64, c->Aqv64, c->Aqf64, c->cq64, c->Ac32,
                   c->Aqv32, c->Aqf32, c->cq32, c->bqv64, c->bqf64, c->Kd64, c->Kd32,
                   c->recfp, c->tabfp, c->rec32q, c->rec32c, c->rec64m, c->rec64mT, c->tabm64,
-                  c->cg2_slots, c->convtabi, c->convexps, c->reci, c->reciT, c->reci_exp, c->reciT_exp};
+                  c->cg2_slots, c->convtabi, c->convexps, c->reci, c->reciT, c->reci_exp, c->reciT_exp, c->rect,
+                  c->rect_exp};
   for (void *b : bufs)
     if (b) cudaFree(b);
   for (int i = 0; i < 10; i++)

@@ -597,6 +597,7 @@ int prepare_apply64(pdg_context *ctx, int transpose) {
     if (apply_i_usable(ctx)) PDG_TRY(prepare_apply_i(ctx, transpose));
     else PDG_TRY(prepare_apply_m(ctx, transpose));
   }
+  if (tensor_i_usable(ctx) && !transpose) PDG_TRY(prepare_apply_tensor(ctx));
   if (ctx->f64_pair && ctx->dim == 3 && !general_coefficients(ctx))
     PDG_TRY(prepare_float_pair(ctx));
   return PDG_OK;

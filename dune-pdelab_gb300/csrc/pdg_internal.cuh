@@ -164,6 +164,9 @@ struct pdg_context {
   int2 *reci, *reciT;  // 3D: limb records of the operator / its transpose and the
   int *reci_exp, *reciT_exp;   // exponents of each cell's groups (k_apply_i)
   int reci_valid, reciT_valid;
+  int2 *rect;          // 3D: limb coefficients of the tensor operator and their exponents
+  int *rect_exp;       // (k_apply_tensor_i)
+  int rect_valid;
   double *tabm64;      // 3D: Mhat, Mhat^-1 e0, Mhat^-1 e_{N-1}, Mhat^-1 d0, Mhat^-1 d1, Mhat^-1
   double *tabt64;      // 3D: M, Dn, L = M^-1 Dn^T M, M^-1 e0, M^-1 e_{N-1}, d0, d1 of the
   float *tabt32;       // per-cell tensor operator (pdg_tensor.cu)
@@ -425,6 +428,8 @@ int launch_apply_general(pdg_context *ctx, const ApplyArgs<T> &a);
 // nodes (pdg_tensor.cu)
 template <typename T>
 int launch_apply_tensor(pdg_context *ctx, const ApplyArgs<T> &a, const OpParams<T> &p);
+bool tensor_i_usable(const pdg_context *ctx);
+int prepare_apply_tensor(pdg_context *ctx);
 // R(0)'s Dirichlet-data diffusion terms with the tensor (added to ctx->r0)
 int launch_rhs_general(pdg_context *ctx);
 // the face lattice (every face once: x-normal faces, then y, then z; planes

@@ -52,3 +52,77 @@ def test_sizes(k, n, symmetric):
         one[s] = v[s]
         assert rel(P.jacobian_apply(one)[s], x[s]) <= 1e-9
     go.close()
+
+
+def cells(k, n, seed, scale=1.0, sigma=0.0):
+    rng = np.random.default_rng(seed)
+    nc = int(np.prod(n))
+    G = rng.standard_normal((nc, 3, 3))
+    A = G @ G.transpose(0, 2, 1) + 0.2 * np.eye(3)
+    A *= scale * np.exp(sigma * rng.standard_normal((nc, 1, 1)))
+    go = pdg.GridOperator(3, k, n, alpha=3.0)
+    P = O.Problem(3, k, n, alpha=3.0)
+    go.set_permeability_tensor(A)
+    P.set(Acell=A)
+    return go, P, rng
+
+
+def apply(go, x):
+    y = np.zeros(go.ndof)
+    pdg.OnTheFlyOperator(go).apply(x, y)
+    return y
+
+
+@pytest.mark.parametrize("k", [1, 2, 3])
+def test_fixed_point_ranges(k):
+    """Degrees 1 to 3 run in 64-bit fixed point: values over 12 decades and
+    tensors over e^+-9 from cell to cell; 57-bit operands leave every cell 1e-12
+    of its own largest value."""
+    go, P, rng = cells(k, (5, 4, 3), 1, sigma=3.0)
+    x = rng.uniform(-1, 1, (go.ncell, go.nbasis)) * 10.0 ** rng.uniform(-6, 6, (go.ncell, 1))
+    y = apply(go, x.ravel()).reshape(go.ncell, -1)
+    ref = P.jacobian_apply(x.ravel()).reshape(go.ncell, -1)
+    for e in range(go.ncell):
+        assert np.max(np.abs(y[e] - ref[e])) <= 1e-12 * np.max(np.abs(ref[e])), e
+    assert not apply(go, np.zeros(go.ndof)).any()
+    go.close()
+
+
+@pytest.mark.parametrize("factor,scale", [(1e-290, 1.0), (1e200, 1.0), (1.0, 1e60)])
+def test_fixed_point_ends_of_the_range(factor, scale):
+    """Values and tensors beyond the exponents of the limbs: the FP64 form."""
+    go, P, rng = cells(2, (4, 3, 2), 2, scale=scale)
+    x = rng.uniform(-1, 1, go.ndof)
+    assert rel(apply(go, x * factor) / factor, P.jacobian_apply(x)) <= 1e-12
+    go.close()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_fixed_point_non_finite(value):
+    go, P, rng = cells(2, (7, 4, 3), 3)
+    x = rng.uniform(-1, 1, (go.ncell, go.nbasis))
+    ref = P.jacobian_apply(x.ravel()).reshape(go.ncell, -1)
+    e = 2 + 7 * (1 + 4 * 1)
+    x[e] = value
+    y = apply(go, x.ravel()).reshape(go.ncell, -1)
+    hit = {e, e - 1, e + 1, e - 7, e + 7, e - 28, e + 28}
+    for c in range(go.ncell):
+        if c in hit:
+            assert not np.isfinite(y[c]).all()
+        else:
+            assert np.max(np.abs(y[c] - ref[c])) <= 1e-12 * np.max(np.abs(ref))
+    go.close()
+
+
+def test_fixed_point_follows_the_coefficients():
+    """A changed tensor or reaction rebuilds the limb coefficients."""
+    go, P, rng = cells(2, (3, 3, 2), 4)
+    x = rng.uniform(-1, 1, go.ndof)
+    apply(go, x)
+    A = np.tile(np.array([[2.0, 0.3, 0.1], [0.3, 1.0, 0.2], [0.1, 0.2, 3.0]]), (go.ncell, 1, 1))
+    c = rng.uniform(0.5, 2.0, go.ncell)
+    go.set_permeability_tensor(A)
+    go.set_reaction(c)
+    P.set(Acell=A, c=c)
+    assert rel(apply(go, x), P.jacobian_apply(x)) <= 1e-13
+    go.close()
