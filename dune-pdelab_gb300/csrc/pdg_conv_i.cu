@@ -7,7 +7,7 @@
 // and the upwind fluxes at the face points; 11 N + 3 multiply-adds per DOF in
 // the volume and 36 on the faces.  In FP64 that is bound by the FP64 pipe (91 %
 // active); as limb contractions it takes three IMAD.WIDE each.  32^3 Q4 with
-// the diffusion operator: 410 us, with this part in FP64 993 us; the error
+// the diffusion operator: 386 us, with this part in FP64 993 us; the error
 // against 64 bits is the same (1.5e-14 against 1.4e-14).
 //
 // Scaling.  The cell's values, each neighbour's face layer, the cell's volume
@@ -83,8 +83,11 @@ __device__ __noinline__ void conv_block_fp64(const OpParams<double> &p, const Ap
   conv_block<double, N>(p, a, vrec, tabBD, smem_raw);
 }
 
+// Five blocks per SM at k = 4 (96 instead of 106 registers) and the records
+// prefetched: 32^3 Q4 with the diffusion operator 410 -> 396 -> 386 us (issue
+// slots were 40 % busy, a quarter of the stalls waited for the records).
 template <int N>
-__global__ void __launch_bounds__(CCfg<N>::THREADS)
+__global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N == 3 ? 7 : 9)
     k_conv_i(const __grid_constant__ OpParams<double> p,
              const __grid_constant__ ApplyArgs<double> a, const double *__restrict__ vrec,
              const double *__restrict__ tabBD, const int2 *__restrict__ tabi,
@@ -119,6 +122,18 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS)
   const double *rec = vrec + ee * (C::VREC + C::FREC);
   const int *ex = exps + ee * kConvNexp;
   const int tx = l % N, ty = l / N;   // also the face node / point (pa, pb)
+  // the cells' records to the L2 cache while the trial values are formed
+  {
+    const long r0 = ranged ? a.cell0 + (long)blockIdx.x * CPB : (long)blockIdx.x * CPB;
+    const long r1 = min(r0 + CPB, ranged ? (long)a.cell0 + a.ncells : p.ncell);
+    constexpr int RB = (int)sizeof(double) * (C::VREC + C::FREC);
+    const uintptr_t b0 = reinterpret_cast<uintptr_t>(vrec) + (uintptr_t)r0 * RB;
+    const uintptr_t b1 = (b0 + (uintptr_t)(r1 - r0) * RB) & ~(uintptr_t)15;
+    const uintptr_t b = (b0 + 15) & ~(uintptr_t)15;
+    if (t == 0 && b < b1)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((unsigned)(b1 - b))
+                   : "memory");
+  }
 
   // ---- own column, and this thread's node of each neighbour's face layer ----
   double col[N], nl[6];
