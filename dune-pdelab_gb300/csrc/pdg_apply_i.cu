@@ -53,6 +53,10 @@ struct ICfg {
   // after each
   static constexpr bool WIDE = N > 2;
   static constexpr int SHX = N == 2 ? 2 : 0;
+  // s2 carries FB more bits than s1: the derivative of the basis multiplies it,
+  // and its rounding, by up to 48 (with FB = 0 smooth data at 24^3 Q4 had 5 times
+  // the noise of FP64, with 3 less than that)
+  static constexpr int FB = N == 2 ? 0 : 3;
   static constexpr int SHM = N == 2 ? 2 : N == 4 ? 10 : 12;
   // exponent of one unit of the result over the cell's Etot
   static constexpr int OUTE = -61 + SHX + (WIDE ? 2 * SHM : SHM);
@@ -243,9 +247,9 @@ __device__ __noinline__ double apply_cells_fp64(const OpParams<double> &p,
 
 // 24 or 20 warps per SM.  33x29x37 Q4 183 -> 167 us with five blocks instead of
 // the four the register count alone gives, 156 with the results put together on
-// the integer pipe.  Degree 2 has its own kernel (k_apply_p); the exchanges
-// through shared memory, 12 loads and stores per value there, are what it avoids
-// (204 -> 145 us at 64^3 Q2).  At degrees 3 and 4 a plane per thread is 16 or
+// the integer pipe, 163 with s2 in finer units.  Degree 2 has its own kernel
+// (k_apply_p); the exchanges through shared memory, 12 loads and stores per value
+// there, are what it avoids (204 -> 161 us at 64^3 Q2).  At degrees 3 and 4 a plane per thread is 16 or
 // 25 values with 96-bit sums, which does not fit the registers.
 template <int N>
 __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6)
@@ -303,6 +307,7 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
   const double *xe = a.x + (size_t)ee * NB;
 #pragma unroll
   for (int z = 0; z < N; z++) col[z] = xe[z * TPC + l];
+  const int flip = sign_flip(xe[0]);
   double v[NF][N];
 #pragma unroll
   for (int f = 0; f < NF; f++) {
@@ -358,7 +363,7 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
   int2 uc[N], zf[4];   // own column; the z faces' data is read by this thread only
 #pragma unroll
   for (int z = 0; z < N; z++) {
-    uc[z] = fix_limbs(col[z], ebx);
+    uc[z] = fix_limbs(col[z], ebx, flip);
     ue[z * TPC + l] = uc[z];
   }
 #pragma unroll
@@ -368,12 +373,12 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
     long long hh = 0, mid = 0, h2 = 0, m2 = 0;
 #pragma unroll
     for (int q = 0; q < N; q++) {
-      const int2 u = fix_limbs(v[f][q], eb[f]);
+      const int2 u = fix_limbs(v[f][q], eb[f], flip);
       mac2(hh, mid, u, w[q]);
       if (q == ((f & 1) ? 0 : N - 1)) mac2(h2, m2, u, w[N]);
     }
     const long long s1 = mac2_value(hh, mid, Etot - eu - ex[1 + f] - 2);
-    const long long s2 = mac2_value(h2, m2, Etot - eu - ex[7 + f] - 2);
+    const long long s2 = mac2_value(h2, m2, Etot - eu - ex[7 + f] - 2 - C::FB);
     if (f < 4) {
       fa[(2 * f) * TPC + l] = split32(s1);
       fa[(2 * f + 1) * TPC + l] = split32(s2);
@@ -398,7 +403,14 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
   // ---- directional operators and face lifts ----
   const int tx = l % N, ty = l / N;
   const int shu = Etot - Ex - EA - 2;
-  constexpr long long kHalfX = C::SHX ? 1ll << (C::SHX > 0 ? C::SHX - 1 : 0) : 0;
+  // rounding constant of line entry i in units of s2: halves of the shifts below,
+  // and the half units that cutting took from the volume term, from s1 on the
+  // two ends and from the d_i s2 (d: sum of the entry's derivatives)
+  const auto cut = [](int i, int d) {
+    constexpr int kHalves =
+        (C::FB > 0 ? 1 << (C::FB - 1) : 0) + (C::SHX > 0 ? 1 << (C::SHX - 1 + C::FB) : 0);
+    return (long long)((((1 + (i == 0) + (i == N - 1)) << C::FB) + d) / 2 + kHalves);
+  };
   {
     int2 Ax[N], Ay[N];
 #pragma unroll
@@ -414,34 +426,37 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
         long long hh = 0, mid = 0;
 #pragma unroll
         for (int q = 0; q < N; q++) mac2(hh, mid, Ax[q], ue[z * N2 + ty * N + q]);
-        SmallSum<false> s(mac2_value(hh, mid, shu) + kHalfX);
+        SmallSum<false> s(mac2_value(hh, mid, shu));
         s.add(fa[0 * TPC + lx], tx == 0);
-        s.add(fa[1 * TPC + lx], d0x);
         s.add(fa[2 * TPC + lx], tx == N - 1);
-        s.add(fa[3 * TPC + lx], d1x);
-        Xs[z * N2 + l] = split32(s.template shifted<C::SHX>());
+        SmallSum<false> d(cut(tx, d0x + d1x));
+        d.add(fa[1 * TPC + lx], d0x);
+        d.add(fa[3 * TPC + lx], d1x);
+        Xs[z * N2 + l] = split32((s.total() + d.template shifted<C::FB>()) >> C::SHX);
       }
       {
         long long hh = 0, mid = 0;
 #pragma unroll
         for (int q = 0; q < N; q++) mac2(hh, mid, Ay[q], ue[z * N2 + q * N + tx]);
-        SmallSum<false> s(mac2_value(hh, mid, shu) + kHalfX);
+        SmallSum<false> s(mac2_value(hh, mid, shu));
         s.add(fa[4 * TPC + ly], ty == 0);
-        s.add(fa[5 * TPC + ly], d0y);
         s.add(fa[6 * TPC + ly], ty == N - 1);
-        s.add(fa[7 * TPC + ly], d1y);
-        Ys[z * N2 + l] = split32(s.template shifted<C::SHX>());
+        SmallSum<false> d(cut(ty, d0y + d1y));
+        d.add(fa[5 * TPC + ly], d0y);
+        d.add(fa[7 * TPC + ly], d1y);
+        Ys[z * N2 + l] = split32((s.total() + d.template shifted<C::FB>()) >> C::SHX);
       }
       {
         long long hh = 0, mid = 0;
 #pragma unroll
         for (int q = 0; q < N; q++) mac2(hh, mid, Am[2 * N2 + z * N + q], uc[q]);
-        SmallSum<false> s(mac2_value(hh, mid, shu) + kHalfX);
+        SmallSum<false> s(mac2_value(hh, mid, shu));
         if (z == 0) s.add(zf[0], 1);
-        s.add(zf[1], int_d0<N>(z));
         if (z == N - 1) s.add(zf[2], 1);
-        s.add(zf[3], int_d1<N>(z));
-        Zs[z * N2 + l] = split32(s.template shifted<C::SHX>());
+        SmallSum<false> d(cut(z, int_d0<N>(z) + int_d1<N>(z)));
+        d.add(zf[1], int_d0<N>(z));
+        d.add(zf[3], int_d1<N>(z));
+        Zs[z * N2 + l] = split32((s.total() + d.template shifted<C::FB>()) >> C::SHX);
       }
     }
   }
@@ -471,6 +486,7 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
   // ---- out = M_z W + M_y T1 ----
   double part = 0.0;
   if (active) {
+    const bool zero = Etot <= kFixZero + 1000;   // no data (but rounding constants)
     double *ye = a.y + (size_t)e * NB;
     const double *ad = a.add ? a.add + (size_t)e * NB : nullptr;
     const bool scale = a.alpha != 1.0;
@@ -482,7 +498,9 @@ __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6
         s.add(W[q], int_m<N>(z * N + q));
         s.add(ue[z * N2 + q * N + tx], My[q]);
       }
-      double r = fix_to_double(s.template shifted<C::WIDE ? C::SHM : 0>(), Etot + C::OUTE);
+      double r = zero ? 0.0
+                      : fix_to_double(s.template shifted<C::WIDE ? C::SHM : 0>(), Etot + C::OUTE,
+                                      flip);
       if (scale) r *= a.alpha;
       const int idx = z * TPC + l;
       if (a.accumulate) r += ye[idx];

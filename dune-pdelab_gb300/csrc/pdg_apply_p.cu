@@ -18,8 +18,8 @@
 //   their own cell converted: the lines of a face cover the neighbour cell, so
 //   the cell's sums are aligned to that cell's largest value in any case;
 // * the small integers of the mass and derivative tables are compile-time
-//   constants (shifts and adds), and the sums of the masses fit 64 bits (see
-//   PCfg), so that IMAD.WIDE is left to the limb products;
+//   constants (shifts and adds), and the sums of all but the last masses fit 64
+//   bits (see PCfg), so that IMAD.WIDE is left to the limb products and those;
 // * loops over the lines of a plane are not unrolled (65 KB of straight code
 //   missed the instruction cache), their results wait in the thread's own part
 //   of a run that is used up;
@@ -28,10 +28,10 @@
 //
 // 64^3 Q2 (7.1 M DOF): k_apply_i 204 us, this one 179 as first written, 153
 // with the record prefetched to the L2 cache, no FP64 and 96 registers, 145 with
-// the loops rolled (57 MB in, 57 MB out and 123 MB of records need 35 us).  What
-// is left is the integer work (4100 instructions per warp, issue slots 58 %,
-// ALU 55 %, IMAD 52 % busy) at 18 warps per SM; 15 warps without any spill take
-// 171 us.
+// the loops rolled, 161 with the last masses in two halves and the cells' signs
+// taken out (57 MB in, 57 MB out and 123 MB of records need 35 us).  What is
+// left is the integer work (issue slots 58 %, ALU 55 %, IMAD 52 % busy) at 18
+// warps per SM; 15 warps without any spill take 173 us.
 #include <cmath>
 
 #include "pdg_fixed.cuh"
@@ -52,10 +52,13 @@ struct PCfg {
   static constexpr int SMEM = OWNP + 4 * RUNP;
   // X, Y, Z come below 0.75 2^61 (three terms under 2^(Etot - 2) in units of
   // 2^(Etot - 61)).  Shifted by 2 and with mass row sums of 20 a mass stays
-  // below 15 2^59 < 2^63; shifted by 6 again, M_y X + M_x Y is below 0.47 2^59
-  // and M_x Z below 0.24 2^59, so the last sum is below 14.1 2^59 < 2^63.
-  static constexpr int SHX = 2, SHM = 6;
-  static constexpr int OUTE = -61 + SHX + SHM;
+  // below 15 2^59 < 2^63; shifted by 1 again, M_y X + M_x Y is below 15 2^59
+  // and M_x Z below 7.5 2^59.  The last masses are summed in two halves, below
+  // 450 2^59 < 2^68, and shifted by SHO.  (With 64-bit sums throughout, M_y X and
+  // M_x Z rounded to 2^(Etot - 53) instead, smooth data had twice the noise of
+  // FP64.)
+  static constexpr int SHX = 2, SHM = 1, SHO = 6;
+  static constexpr int OUTE = -61 + SHX + SHM + SHO;
 };
 
 // v * c for a small integer constant
@@ -66,6 +69,10 @@ __device__ __forceinline__ long long times(long long v) {
 // a run-time one: two 32-bit products
 __device__ __forceinline__ long long times(long long v, int c) {
   return (long long)((unsigned long long)v * (unsigned long long)(long long)c);
+}
+// limbs of -X for s = -1, of X for s = 0
+__device__ __forceinline__ int2 negate_if(int2 v, int s) {
+  return make_int2((v.x ^ s) - s, (v.y ^ s) - s);
 }
 template <int S>
 __device__ __forceinline__ long long round_shift(long long v) {
@@ -133,6 +140,13 @@ __device__ __forceinline__ void face_line(const int2 (&u)[PCfg::N], const int2 (
   s2 = mac2_value(h2, m2, sh2);
 }
 
+// rounding constant of line entry i: half of 2^SHX, and the half units that cutting
+// took from the volume term, from s1 on the two ends and from the d_i s2
+__host__ __device__ __forceinline__ constexpr int cut_bias(int i) {
+  constexpr int N = PCfg::N;
+  return (1 << (PCfg::SHX - 1)) +
+         (1 + (i == 0) + (i == N - 1) + int_d0<N>(i) + int_d1<N>(i) + 1) / 2;
+}
 // a line with compile-time derivative tables: A' u plus the lifts of both faces
 __device__ __forceinline__ void line_sums(const int2 (&A)[PCfg::N2], const int2 (&u)[PCfg::N],
                                           int shu, long long s1l, long long s2l, long long s1h,
@@ -143,12 +157,12 @@ __device__ __forceinline__ void line_sums(const int2 (&A)[PCfg::N2], const int2 
     long long hh = 0, mid = 0;
 #pragma unroll
     for (int q = 0; q < N; q++) mac2(hh, mid, A[i * N + q], u[q]);
-    X[i] = mac2_value(hh, mid, shu) + s2l * int_d0<N>(i) + s2h * int_d1<N>(i);
+    X[i] = mac2_value(hh, mid, shu) + s2l * int_d0<N>(i) + s2h * int_d1<N>(i) + cut_bias(i);
   }
   X[0] += s1l;
   X[N - 1] += s1h;
 #pragma unroll
-  for (int i = 0; i < N; i++) X[i] = round_shift<PCfg::SHX>(X[i]);
+  for (int i = 0; i < N; i++) X[i] >>= PCfg::SHX;
 }
 
 __global__ void __launch_bounds__(PCfg::THREADS, 6)
@@ -159,7 +173,7 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
   constexpr int N = C::N, N2 = C::N2, NB = C::NB, T = C::T, NF = C::NF;
   extern __shared__ __align__(16) double smd[];
   __shared__ __align__(8) unsigned long long bar;
-  __shared__ int eO[N][T + 2], eC[N][T];
+  __shared__ int eO[N][T + 2], eC[N][T], sF[T + 2];   // exponents; sign flips of the cells
   if (a.skip && *a.skip) return;
   const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
   const long ncell = p.ncell, ndof = ncell * NB;
@@ -227,6 +241,7 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
       own.add(col[i]);
     }
     eO[z][lane + 1] = code(own);
+    if (z == 0) sF[lane + 1] = sign_flip(col[0]);
     int cand = 2 * kFixZero;
 #pragma unroll
     for (int f = 2; f < NF; f++) {
@@ -255,8 +270,10 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
       b.m = __reduce_max_sync(0xffffffffu, b.m);
       b.any = __reduce_or_sync(0xffffffffu, b.any);
       c = code(b);
+      const int fh = __shfl_sync(0xffffffffu, sign_flip(h), 0);
+      if (lane == 0) sF[slot] = fh;
       if (lane < NB)
-        reinterpret_cast<int2 *>(OWN)[slot * NB + lane] = fix_limbs(h, b.biased());
+        reinterpret_cast<int2 *>(OWN)[slot * NB + lane] = fix_limbs(h, b.biased(), fh);
     }
     if (lane < N) eO[lane][slot] = c;
   }
@@ -282,13 +299,14 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
   const int Etot = max(Ex + EA + C::LN, cand) + 2;
   bad |= Etot > 900 || (Etot > kFixZero + 1000 && Etot < -780);
   bad &= active;
+  const int flip = sF[lane + 1];
 
   // ---- own plane to limbs, in place ----
   int2 *Up = reinterpret_cast<int2 *>(U);
   {
     const int ebx = max(Ex + 1022, kFixMinBiased);
 #pragma unroll
-    for (int i = 0; i < N2; i++) Up[i] = fix_limbs(col[i], ebx);
+    for (int i = 0; i < N2; i++) Up[i] = fix_limbs(col[i], ebx, flip);
   }
   if (__syncthreads_or(bad)) {
     unsigned mask = 0;
@@ -317,8 +335,8 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
 #pragma unroll
         for (int q = 0; q < N; q++) {
           u[q] = Up[q * N + x];
-          l[q] = fix_limbs(YLp[q * N + x], eb[0]);
-          h[q] = fix_limbs(YHp[q * N + x], eb[1]);
+          l[q] = fix_limbs(YLp[q * N + x], eb[0], flip);
+          h[q] = fix_limbs(YHp[q * N + x], eb[1], flip);
         }
         long long s1l, s2l, s1h, s2h, Y[N];
         face_line<false>(l, wl, sl1, sl2, s1l, s2l);
@@ -351,8 +369,9 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
       for (int i = 0; i < N2; i++) A[i] = r[i * T];
 #pragma unroll
       for (int i = 0; i <= N; i++) {
-        wl[i] = r[(3 * N2 + i) * T];
-        wh[i] = r[(3 * N2 + (N + 1) + i) * T];
+        // the neighbours' limbs carry their own cells' flips
+        wl[i] = negate_if(r[(3 * N2 + i) * T], flip ^ sF[lane]);
+        wh[i] = negate_if(r[(3 * N2 + (N + 1) + i) * T], flip ^ sF[lane + 2]);
       }
 #pragma unroll 1
       for (int y = 0; y < N; y++) {
@@ -377,7 +396,8 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
           long long s = 0;
 #pragma unroll
           for (int q = 0; q < N; q++) s += S[q * N + x] * int_m<N>(j * N + q);
-          W[j * N + x] += round_shift<C::SHM>(s);
+          reinterpret_cast<int2 *>(W)[j * N + x] =
+              split32(W[j * N + x] + round_shift<C::SHM>(s));
         }
     }
     // ---- z faces of row z: over the values read (s1 in plane 0, s2 in plane 1) ----
@@ -396,8 +416,8 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
         int2 l[N], h[N];
 #pragma unroll
         for (int q = 0; q < N; q++) {
-          l[q] = fix_limbs(ZLp[q * N2 + x], eb[2]);
-          h[q] = fix_limbs(ZHp[q * N2 + x], eb[3]);
+          l[q] = fix_limbs(ZLp[q * N2 + x], eb[2], flip);
+          h[q] = fix_limbs(ZHp[q * N2 + x], eb[3], flip);
         }
         long long s1l, s2l, s1h, s2h;
         face_line<false>(l, wl, sl1, sl2, s1l, s2l);
@@ -412,6 +432,7 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
     // ---- out = M_z W + M_y M_x Z ----
     {
       const int d0 = z == 0 ? int_d0<N>(0) : z == 1 ? int_d0<N>(1) : int_d0<N>(2);
+      const int cz = z == 0 ? cut_bias(0) : z == 1 ? cut_bias(1) : cut_bias(2);
       const int d1 = z == 0 ? int_d1<N>(0) : z == 1 ? int_d1<N>(1) : int_d1<N>(2);
       const int2 *Uc = reinterpret_cast<const int2 *>(OWN + (lane + 1) * NB);
       int2 A[N];
@@ -431,7 +452,7 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
           long long s = mac2_value(hh, mid, shu) + times(fl[N2 + i], d0) + times(fh[N2 + i], d1);
           if (z == 0) s += fl[i];
           if (z == N - 1) s += fh[i];
-          Z[x] = round_shift<C::SHX>(s);
+          Z[x] = (s + cz) >> C::SHX;
         }
 #pragma unroll
         for (int x = 0; x < N; x++) {
@@ -442,23 +463,28 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
         }
       }
     }
-    const long long *Wc = reinterpret_cast<const long long *>(YL + lane * NB);
+    const bool zero = Etot <= kFixZero + 1000;   // no data (but rounding constants)
+    const int2 *Wc = reinterpret_cast<const int2 *>(YL + lane * NB);
     // row z of the mass matrix: 4 2 -1, 2 16 2, -1 2 4
     const int m0 = z == 0 ? int_m<N>(0) : z == 1 ? int_m<N>(3) : int_m<N>(2),
               m1 = z == 1 ? int_m<N>(4) : int_m<N>(1),
               m2 = z == 0 ? int_m<N>(2) : z == 1 ? int_m<N>(3) : int_m<N>(0);
 #pragma unroll
     for (int x = 0; x < N; x++) {
-      long long t[N];
+      int2 t[N];
 #pragma unroll
-      for (int q = 0; q < N; q++) t[q] = S[q * N + x];
+      for (int q = 0; q < N; q++) t[q] = split32(S[q * N + x]);
 #pragma unroll
       for (int j = 0; j < N; j++) {
         const int i = j * N + x;
-        long long s = times(Wc[i], m0) + times(Wc[N2 + i], m1) + times(Wc[2 * N2 + i], m2);
+        SmallSum<true> s(1ll << (C::SHO - 1));
+        s.add(Wc[i], m0);
+        s.add(Wc[N2 + i], m1);
+        s.add(Wc[2 * N2 + i], m2);
 #pragma unroll
-        for (int q = 0; q < N; q++) s += t[q] * int_m<N>(j * N + q);
-        YHp[i] = fix_to_double(s, Etot + C::OUTE);
+        for (int q = 0; q < N; q++) s.add(t[q], int_m<N>(j * N + q));
+        YHp[i] = zero ? 0.0
+                      : fix_to_double(s.template shifted<C::SHO>(), Etot + C::OUTE, flip);
       }
     }
   }

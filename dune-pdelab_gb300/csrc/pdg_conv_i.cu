@@ -7,7 +7,7 @@
 // and the upwind fluxes at the face points; 11 N + 3 multiply-adds per DOF in
 // the volume and 36 on the faces.  In FP64 that is bound by the FP64 pipe (91 %
 // active); as limb contractions it takes three IMAD.WIDE each.  32^3 Q4 with
-// the diffusion operator: 386 us, with this part in FP64 993 us; the error
+// the diffusion operator: 393 us, with this part in FP64 993 us; the error
 // against 64 bits is the same (1.5e-14 against 1.4e-14).
 //
 // Scaling.  The cell's values, each neighbour's face layer, the cell's volume
@@ -84,7 +84,7 @@ __device__ __noinline__ void conv_block_fp64(const OpParams<double> &p, const Ap
 }
 
 // Five blocks per SM at k = 4 (96 instead of 106 registers) and the records
-// prefetched: 32^3 Q4 with the diffusion operator 410 -> 396 -> 386 us (issue
+// prefetched: 32^3 Q4 with the diffusion operator 410 -> 396 -> 389 us (issue
 // slots were 40 % busy, a quarter of the stalls waited for the records).
 template <int N>
 __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N == 3 ? 7 : 9)
@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   // ---- own column, and this thread's node of each neighbour's face layer ----
   double col[N], nl[6];
   const double *xe = a.x + ee * NB;
+  const int flip = sign_flip(xe[0]);
 #pragma unroll
   for (int z = 0; z < N; z++) col[z] = xe[z * N2 + l];
 #pragma unroll
@@ -188,13 +189,13 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   int2 uc[N];
 #pragma unroll
   for (int z = 0; z < N; z++) {
-    uc[z] = fix_limbs<kFixWide>(col[z], ebu);
+    uc[z] = fix_limbs<kFixWide>(col[z], ebu, flip);
     S3[z * N2 + l] = uc[z];
   }
 #pragma unroll
   for (int f = 0; f < 6; f++) {
     const int En = sE[7 * cs + 1 + f];
-    Un[f * N2 + l] = fix_limbs<kFixWide>(nl[f], En == kFixZero ? kFixMinBiased : En + 1022);
+    Un[f * N2 + l] = fix_limbs<kFixWide>(nl[f], En == kFixZero ? kFixMinBiased : En + 1022, flip);
   }
   const int sf = ce.lb - ce.eb, sb = ce.lbt - ce.eb;
   // forward z: S0 = B_z u
@@ -363,11 +364,13 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   }
   __syncthreads();
   if (!active) return;
-  const double uv = Evol > kNone
-                        ? __hiloint2double((Evol + ce.ldt + ce.lbt + 1 + ce.eb - kFixWide + 1023) << 20, 0)
-                        : 0.0;
+  const int sg = flip & (int)0x80000000;
+  const double uv =
+      Evol > kNone
+          ? __hiloint2double(sg | ((Evol + ce.ldt + ce.lbt + 1 + ce.eb - kFixWide + 1023) << 20), 0)
+          : 0.0;
   const double uf =
-      Efl > kNone ? __hiloint2double((Efl + ce.lbt + ce.eb - kFixWide + 1023) << 20, 0) : 0.0;
+      Efl > kNone ? __hiloint2double(sg | ((Efl + ce.lbt + ce.eb - kFixWide + 1023) << 20), 0) : 0.0;
   const long long *R = reinterpret_cast<const long long *>(fl);
   double *ye = a.y + e * NB;
 #pragma unroll

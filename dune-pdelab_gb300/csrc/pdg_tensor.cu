@@ -26,7 +26,7 @@
 // against 26 to 38 us.  The FP64 kernel is bound by its FP64 pipe, so its time
 // follows the count (41x37x39 Q2 380 us, at the Gauss points 1735 us); the
 // operator of degrees 1 to 3 runs in fixed point on the integer pipe instead
-// (k_apply_tensor_i below: 95 us).
+// (k_apply_tensor_i below: 100 us).
 //
 // Thread mapping: N*N threads per cell, thread (tx, ty) owns the z-column;
 // face steps: one face node per thread.
@@ -323,14 +323,14 @@ __global__ void __launch_bounds__(TCfg<N>::THREADS)
 // den, which are in the coefficients); products with the cell's coefficients
 // are limb products.  Exponents: own values Ex, values of each neighbour's
 // side Ef, gradients Ex + LD, the corrected gradient Eh, fluxes and face terms
-// Etot, each from bounds; F and t then have 60 bits.  The sum S = sum L F + m t
+// Etot, each from bounds; F and t then have 62 bits.  The sum S = sum L F + m t
 // is up to 150 (k = 2) times larger in the bound than what the masses leave of
 // it, so it is formed exactly (96 bits) and rounded to 61 bits of the cell's
 // actual largest value.
-// 41x37x39 Q2 375 -> 95 us, 30x31x32 Q3 101 us, 80^3 Q1 301 us (at the Gauss
-// points 1735, 1895, 5238 us); errors against 64 bits 2.7e-16 (2.6e-16).  With
-// 57 instead of 59 bits for the gradients and their corrected form, and a looser
-// bound of the latter, the error was 6.5e-16 at the same time.
+// 41x37x39 Q2 375 -> 100 us, 30x31x32 Q3 about 105 us, 80^3 Q1 about 310 us (at
+// the Gauss points 1735, 1895, 5238 us); errors against 64 bits 2.4e-16
+// (2.7e-16).  With 57 instead of 59 bits for the gradients and their corrected
+// form, and a looser bound of the latter, the error was 6.5e-16.
 // Degree 4 keeps the FP64 kernel (57-bit values times the derivative table's
 // row sum of 128 exceed 64 bits), as do the transpose, which needs twice the
 // products, single cells and cell lists.
@@ -532,6 +532,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
   const int tx = l % N, ty = l / N;
   double col[N], line[6][N];
   const double *xe = a.x + (size_t)ee * NB;
+  const int flip = sign_flip(xe[0]);
 #pragma unroll
   for (int z = 0; z < N; z++) col[z] = xe[z * TPC + l];
 #pragma unroll
@@ -579,7 +580,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
     Et = max(Et, max(max(xf[0] + Eg, xf[1] + Ef + B::LD) + 2, xf[2] + Ej) + 2);
   }
   Eh += 1;   // the gradient, the lifts of two faces
-  const int Etot = max(max(EA + Eh + 2, Et), ex[C::X_C] + Ex + 1);
+  const int Etot = max(max(EA + Eh + 2, Et), ex[C::X_C] + Ex + 4);
   bad |= Etot > 850 || (Etot > kFixZero + 1000 && Etot < -700);
   if (__syncthreads_or(bad && active)) {
     tensor_block_fp64<N>(p, a, Ac, tab, smem_raw);
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
   int2 gn[6];   // limbs of the neighbours' normal derivatives, at Ef + LD
 #pragma unroll
   for (int z = 0; z < N; z++) {
-    uc[z] = fix_signed(col[z], biased(Ex));
+    uc[z] = fix_signed(col[z], biased(Ex), flip);
     U[z * N2 + l] = split32(uc[z]);
   }
 #pragma unroll
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
     long long d = 0;
 #pragma unroll
     for (int q = 0; q < N; q++) {
-      const long long v = fix_signed(line[f][q], eb);
+      const long long v = fix_signed(line[f][q], eb, flip);
       d += v * int_dn<N>((f & 1) ? q : N2 - N + q);
       if (q == ((f & 1) ? 0 : N - 1)) Vn[f * N2 + l] = split32(v);
     }
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
   }
   __syncthreads();
 
-  // ---- face nodes: t (60 bits of Etot) and the lifted jump (units of 2^(Eh - 61)) ----
+  // ---- face nodes: t (62 bits of Etot) and the lifted jump (units of 2^(Eh - 61)) ----
 #pragma unroll
   for (int f = 0; f < 6; f++) {
     const int dir = f >> 1, hi = f & 1;
@@ -648,7 +649,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
     long long hh = 0, mid = 0;
 #pragma unroll
     for (int j = 0; j < 3; j++) mac2(hh, mid, cf[j], G[j * NB + nd]);
-    long long s = shr(mac2_value_wide(hh, mid), Etot - xf[0] - Eg + C::GB - 60);
+    long long s = mac2_round(hh, mid, Etot - xf[0] - Eg + C::GB - 60);
     SmallSum<false> d1(kHalfD), d2(kHalfD);
 #pragma unroll
     for (int q = 0; q < N; q++) {
@@ -659,16 +660,16 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
     mac2(hh, mid, cf[3 + dir], gn[f]);
     mac2(hh, mid, cf[3 + o1], limbs(d1.template shifted<C::GS>()));
     mac2(hh, mid, cf[3 + o2], limbs(d2.template shifted<C::GS>()));
-    s += shr(mac2_value_wide(hh, mid), Etot - xf[1] - Ef - B::LD + C::GB - 60);
+    s += mac2_round(hh, mid, Etot - xf[1] - Ef - B::LD + C::GB - 60);
     const int2 jump =
         limbs(shr(join32(U[nd]) * 4, Ej - Ex) - shr(join32(Vn[f * N2 + l]) * 4, Ej - Ef));   // 59 bits
     hh = mid = 0;
     mac2(hh, mid, cf[6], jump);
-    s += shr(mac2_value_wide(hh, mid), Etot - xf[2] - Ej - 1);
+    s += mac2_round(hh, mid, Etot - xf[2] - Ej - 1);
     Tf[f * N2 + l] = split32(s);
     hh = mid = 0;
     mac2(hh, mid, cf[7], jump);
-    Rf[f * N2 + l] = split32(shr(mac2_value_wide(hh, mid), Eh - xf[3] - Ej - 2));
+    Rf[f * N2 + l] = split32(mac2_round(hh, mid, Eh - xf[3] - Ej));
   }
   __syncthreads();
 
@@ -701,7 +702,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
       long long hh = 0, mid = 0;
 #pragma unroll
       for (int j = 0; j < 3; j++) mac2(hh, mid, Cf[k * 3 + j], h[j]);
-      G[k * NB + i] = split32(shr(mac2_value_wide(hh, mid), shf));
+      G[k * NB + i] = split32(mac2_round(hh, mid, shf));
     }
   }
   __syncthreads();
@@ -738,7 +739,7 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
       if (p.c) {
         long long hh = 0, mid = 0;
         mac2(hh, mid, cc, limbs(uc[z]));
-        s.lo += mac2_value(hh, mid, Etot - ex[C::X_C] - Ex - 1);
+        s.lo += mac2_round(hh, mid, Etot - ex[C::X_C] - Ex - 3);
       }
       sh[z] = s.hi + (s.lo >> 32);
       sl[z] = (long long)(unsigned)s.lo;
@@ -787,13 +788,13 @@ __global__ void __launch_bounds__(TICfg<N>::THREADS, N == 3 ? 6 : 5)
   if (!active) return;
   double *ye = a.y + (size_t)e * NB;
   const double *ad = a.add ? a.add + (size_t)e * NB : nullptr;
-  const int E = Etot - 60 + sn + 3 * C::SHM;
+  const int E = Etot - 62 + sn + 3 * C::SHM;
 #pragma unroll
   for (int z = 0; z < N; z++) {
     SmallSum<true> s(kHalfM);
 #pragma unroll
     for (int q = 0; q < N; q++) s.add(w[q], int_m<N>(z * N + q));
-    double r = fix_to_double(s.template shifted<C::SHM>(), E);
+    double r = fix_to_double(s.template shifted<C::SHM>(), E, flip);
     const int idx = z * TPC + l;
     if (a.alpha != 1.0) r *= a.alpha;
     if (a.accumulate) r += ye[idx];

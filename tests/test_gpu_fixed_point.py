@@ -243,3 +243,52 @@ def test_degree2_ranges():
     pdg.OnTheFlyOperator(go).apply(xd, yd)
     assert np.array_equal(apply(go, x), yd.cpu().numpy())
     go.close()
+
+
+@pytest.mark.parametrize("n", [(33, 1, 1), (11, 3, 2)])
+def test_degree2_unaligned_vectors(n):
+    """Vectors that start 8 bytes off a 16-byte boundary: the same bits."""
+    import torch
+    go, P, rng = problem(2, n)
+    x = torch.from_numpy(rng.uniform(-1, 1, go.ndof)).cuda()
+    y = torch.zeros_like(x)
+    pdg.OnTheFlyOperator(go).apply(x, y)
+    xo, yo = (torch.zeros(go.ndof + 1, dtype=torch.float64, device="cuda")[1:] for _ in range(2))
+    xo.copy_(x)
+    pdg.OnTheFlyOperator(go).apply(xo, yo)
+    assert torch.equal(y, yo) and rel(y.cpu().numpy(), P.jacobian_apply(x.cpu().numpy())) <= 1e-14
+    go.close()
+
+
+def smooth(k, n):
+    """sin sin sin at the nodes: J x is far below the terms it is the sum of."""
+    c = (np.arange(n)[:, None] + np.arange(k + 1)[None, :] / k) / n
+    f = np.sin(3.0 * c + 0.1)
+    u = (f[:, None, None, :, None, None] * f[None, :, None, None, :, None]
+         * f[None, None, :, None, None, :])
+    return u.reshape(-1).copy()
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+@pytest.mark.parametrize("kind", ["plain", "transpose", "tensor", "convection"])
+def test_odd_and_rounding_of_smooth_data(k, kind):
+    """J(-x) = -J(x) to the bit; and on smooth data, where the terms of J x cancel,
+    J(3x) - 3 J(x) is rounding of the size that FP64 leaves on those terms: with
+    random signs the same values do not cancel, |J(+-x)| is the size of the
+    terms, and two evaluations with a handful of roundings of 2^-53 each leave
+    no more than 3 * 8 * 2^-53 of it."""
+    n = (6, 6, 6)
+    go, P, rng = problem(k, n)
+    if kind == "tensor":
+        G = rng.standard_normal((216, 3, 3))
+        go.set_permeability_tensor(G @ G.transpose(0, 2, 1) + 0.2 * np.eye(3))
+    if kind == "convection":
+        go.set_velocity_modes(pdg.fourier_velocity_modes(1))
+    x = rng.uniform(-1, 1, go.ndof)
+    tr = kind == "transpose"
+    assert np.array_equal(apply(go, -x, tr), -apply(go, x, tr))
+    u = smooth(k, n[0])
+    terms = np.linalg.norm(apply(go, u * rng.choice([-1.0, 1.0], u.size), tr))
+    noise = np.linalg.norm(apply(go, 3 * u, tr) - 3 * apply(go, u, tr))
+    assert noise <= 3 * 8 * 2.0 ** -53 * terms
+    go.close()
