@@ -347,7 +347,10 @@ static bool cg_fusable(const pdg_context *ctx) {
 // is not what bounds these kernels: 2D grids (small, launch-bound) and the
 // fixed-point kernels in 3D (24^3 Q2: 57 -> 35 us per iteration).
 static bool cg_fusable64(const pdg_context *ctx, int transpose) {
-  const bool op = ctx->dim == 2 ? !transpose : apply_i_usable(ctx) && !ctx->f64_pair;
+  // in 3D where both kernels run in fixed point: fused sums and updates would add
+  // to the FP64 operations that bound the others
+  const bool op = ctx->dim == 2 ? !transpose
+                                : apply_i_usable(ctx) && fdm_i_usable(ctx) && !ctx->f64_pair;
   return op && !convection_on(ctx) && ctx->nl_deg == 0 &&
          !general_coefficients(ctx) && ctx->basis != PDG_BASIS_LEGENDRE && !ctx->use_matrix &&
          !ctx->ops32 && ctx->prec[PDG_F64].ready && ctx->prec[PDG_F64].kind == PDG_PREC_BJ_FDM;

@@ -21,6 +21,10 @@
 // 1/(lx+ly+lz) are normalised to the cell's largest before they are cut: the
 // spectrum of a block spans decades, and a static bound there cost 8 bits
 // (errors of 1e-13 at k = 4).
+// Degrees 1 to 3.  At degree 4 smooth data still had three times the rounding of
+// FP64 (M(3d) - 3 M(d) at 24^3 9.8e-16 of M d against 2.9e-16; degrees 1 to 3: 2.8e-16,
+// 1.4e-16, 1.9e-16 against 4.3e-16, 2.3e-16, 3.2e-16), so it keeps the FP64 kernel
+// (k_fdm_apply in pdg_prec.cu).
 // Cells with data that is not finite or far from the middle of the range send
 // their block to a plain FP64 evaluation.
 #include "pdg_fixed.cuh"
@@ -32,13 +36,13 @@ namespace pdg {
 template <int N>
 struct FICfg {
   static constexpr int N2 = N * N, NB = N * N * N, TPC = N * N;
-  static constexpr int CPB = (N == 4 ? 64 : 128) / TPC;   // 32, 14, 4, 5 cells
+  static constexpr int CPB = (N == 4 ? 64 : 128) / TPC;   // 32, 14, 4 cells
   static constexpr int THREADS = CPB * TPC;
   static constexpr int NEXP = 8;   // EB[3], EL, usable
   // two exchange arrays and the factors; padding with the fewest shared-memory
   // wavefronts, counted on the CPU over paddings 0..15
   static constexpr int PER_CELL =
-      2 * NB + 3 * N2 + (N == 3 ? 8 : N == 5 ? 4 : 0);
+      2 * NB + 3 * N2 + (N == 3 ? 8 : 0);
 };
 
 // exponent E with x < 2^E for a non-negative sum x rounded in FP64
@@ -367,7 +371,6 @@ int fdm_record_i(pdg_context *ctx) {
     case 2: return fdm_record_i_n<2>(ctx);
     case 3: return fdm_record_i_n<3>(ctx);
     case 4: return fdm_record_i_n<4>(ctx);
-    case 5: return fdm_record_i_n<5>(ctx);
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
   }
 }
@@ -401,7 +404,6 @@ int fdm_apply_i(pdg_context *ctx, const double *d, double *v, const int *skip, c
     case 2: return fdm_apply_i_n<2>(ctx, d, v, skip, cells, ncells, scale);
     case 3: return fdm_apply_i_n<3>(ctx, d, v, skip, cells, ncells, scale);
     case 4: return fdm_apply_i_n<4>(ctx, d, v, skip, cells, ncells, scale);
-    case 5: return fdm_apply_i_n<5>(ctx, d, v, skip, cells, ncells, scale);
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
   }
 }

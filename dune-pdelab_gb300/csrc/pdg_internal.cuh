@@ -335,6 +335,7 @@ int block_solve(pdg_context *ctx, const T *d, T *v, int transpose, const int *sk
 // FP64 FDM block Jacobi on 3D grids in 64-bit fixed point (pdg_fdm_i.cu): its
 // records from Q and Lsum_inv, and v = scale D^-1 d on a cell list (or all)
 int fdm_record_i(pdg_context *ctx);
+inline bool fdm_i_usable(const pdg_context *ctx) { return ctx->dim == 3 && ctx->N <= 4; }
 int fdm_apply_i(pdg_context *ctx, const double *d, double *v, const int *skip, const int *cells,
                 int ncells, double scale);
 int diag_blocks(pdg_context *ctx, double **D);   // row-major FP64 diagonal blocks

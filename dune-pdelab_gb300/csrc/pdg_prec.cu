@@ -157,9 +157,8 @@ struct PCfg {
 // counting the wavefronts of the kernel's shared accesses per padding).
 template <typename T, int D, int N>
 constexpr int fdm_pad() {
-  if (D != 3) return 0;
-  if (sizeof(T) == 4) return N == 2 ? 2 : N == 3 ? 15 : N == 4 ? 20 : N == 5 ? 5 : 0;
-  return N == 2 ? 2 : N == 3 ? 2 : N == 5 ? 5 : 0;
+  if (D != 3) return 0;   // (3D FP64 of degrees 1 to 3 is pdg_fdm_i.cu)
+  return N == 2 ? 2 : N == 3 ? 15 : N == 4 ? 20 : N == 5 ? 5 : 0;
 }
 
 // 1 / (Lx[x] + Ly[y] (+ Lz[z])) per DOF (local index x fastest), FP64
@@ -1065,7 +1064,7 @@ static int fdm_setup(pdg_context *ctx, int precision) {
     k_fdm_lsum_inv<<<b2, 256, 0, ctx->stream>>>(ctx->ndof, dim, N, (const double *)pd.L,
                                                    pd.Lsum_inv);
     PDG_CUDA_TRY(cudaGetLastError());
-    if (dim == 3) {
+    if (fdm_i_usable(ctx)) {
       const int st = fdm_record_i(ctx);
       if (st != PDG_OK) {
         cudaFree(dLi);
@@ -1298,7 +1297,9 @@ static int fdm_dispatch(pdg_context *ctx, const T *d, T *v, const int *skip, con
     default: break;
   }
   if constexpr (std::is_same<T, double>::value) {
-    if (ctx->dim == 3) return fdm_apply_i(ctx, d, v, skip, cells, ncells, scale);
+    if (ctx->dim == 3 && fdm_i_usable(ctx)) return fdm_apply_i(ctx, d, v, skip, cells, ncells, scale);
+    if (ctx->dim == 3 && ctx->k == 4)
+      return fdm_apply_dn<T, 3, 5>(ctx, d, v, skip, cells, ncells, scale);
   } else {
     switch (ctx->dim * 10 + ctx->k) {
       case 31: return fdm_apply_dn<T, 3, 2>(ctx, d, v, skip, cells, ncells, scale);
