@@ -7,15 +7,20 @@
 // and the upwind fluxes at the face points; 11 N + 3 multiply-adds per DOF in
 // the volume and 36 on the faces.  In FP64 that is bound by the FP64 pipe (91 %
 // active); as limb contractions it takes three IMAD.WIDE each.  32^3 Q4 with
-// the diffusion operator: 393 us, with this part in FP64 993 us; the error
-// against 64 bits is the same (1.5e-14 against 1.4e-14).
+// the diffusion operator: 421 us, with this part in FP64 993 us; the error
+// against 64 bits is the same (1.5e-14 against 1.4e-14), and on smooth data
+// J(3u) - 3 J(u) of the convection alone is 1.5e-15, 1.6e-15, 2.7e-15 and 3.8e-15 of
+// J u at 24^3, k = 1..4 (FP64: 3.2e-15, 3.6e-15, 8.8e-15, 1.2e-14).
 //
 // Scaling.  The cell's values, each neighbour's face layer, the cell's volume
 // weights and each face's outflow and inflow weights have an exponent each.
 // The 1D tables' row and column sums of magnitudes bound every contraction, so
 // the exponents of all stages follow from those; B and D (values and
 // derivatives at the Gauss points) are scaled so that the two products that
-// meet in one sum have the same unit (ConvExp).  The face fluxes share one
+// meet in one sum have the same unit (ConvExp).  The values at the points, after
+// the x test, before the z test and the fluxes are brought to 59 bits of their
+// largest: the bounds of all stages together cost 10 bits (13 times the rounding
+// of FP64 on smooth data at k = 4, at 393 us).  The face fluxes share one
 // exponent per cell, formed from what each face can let in or out, so a large
 // neighbour downstream costs nothing.  Blocks with data that is not finite or
 // far from the middle of the range are evaluated in FP64.
@@ -75,6 +80,16 @@ __device__ __forceinline__ long long conv_sum(FA fa, FB fb, int s) {
   return mac2_value_wide(hh, mid) >> s;
 }
 
+// significant bits of |v|, and v 2^-s, rounded for s > 0
+__device__ __forceinline__ int conv_bits(long long v) {
+  return v ? 64 - __clzll(v ^ (v >> 63)) : 0;
+}
+__device__ __forceinline__ long long conv_shift(long long v, int s) {
+  const int r = min(s, 62);
+  return s > 0 ? (v + ((1ll << r) >> 1)) >> r
+               : (long long)((unsigned long long)v << min(-s, 63));
+}
+
 template <int N>
 __device__ __noinline__ void conv_block_fp64(const OpParams<double> &p, const ApplyArgs<double> &a,
                                              const double *vrec, const double *tabBD,
@@ -84,7 +99,7 @@ __device__ __noinline__ void conv_block_fp64(const OpParams<double> &p, const Ap
 }
 
 // Five blocks per SM at k = 4 (96 instead of 106 registers) and the records
-// prefetched: 32^3 Q4 with the diffusion operator 410 -> 396 -> 389 us (issue
+// prefetched: 32^3 Q4 with the diffusion operator 410 -> 396 -> 389 us when measured (issue
 // slots were 40 % busy, a quarter of the stalls waited for the records).
 template <int N>
 __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N == 3 ? 7 : 9)
@@ -96,6 +111,8 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   constexpr int N2 = C::N2, NB = C::NB, TPC = C::TPC, CPB = C::CPB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int sE[7 * CPB];
+  // bits of the cell's largest value at the points, after the x test, of a flux
+  __shared__ int sB[3 * CPB];
   if (a.skip && *a.skip) return;
   int2 *tB = reinterpret_cast<int2 *>(smem_raw);   // B[q][a]
   int2 *tD = tB + N2;                              // D[q][a]
@@ -105,6 +122,7 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   int2 *fl = S3 + NB, *Ue = fl + 6 * N2, *Un = Ue + 6 * N2;
   for (int i = t; i < C::TAB; i += C::THREADS) tB[i] = tabi[i];
   for (int i = t; i < 7 * CPB; i += C::THREADS) sE[i] = kFixZero;
+  for (int i = t; i < 3 * CPB; i += C::THREADS) sB[i] = 0;
   const int li = blockIdx.x * CPB + cs;
   const bool ranged = a.ncells > 0;
   const bool active = ranged ? li < a.ncells : li < p.ncell;
@@ -209,6 +227,7 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   }
   // ---- volume ----
   long long r[N];
+  int up;   // exponent of the unit of r, less Evol
   {
     int2 B[N];
 #pragma unroll
@@ -221,13 +240,22 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   __syncthreads();
   {
     int2 B[N], uq[N];
+    long long w[N];
+    int bits = 0;
 #pragma unroll
     for (int k = 0; k < N; k++) B[k] = tB[tx * N + k];
 #pragma unroll
-    for (int z = 0; z < N; z++)
-      uq[z] = limbs(conv_sum<N>([&](int k) { return B[k]; },
-                                [&](int k) { return S1[z * N2 + ty * N + k]; }, sf));
+    for (int z = 0; z < N; z++) {
+      w[z] = conv_sum<N>([&](int k) { return B[k]; },
+                         [&](int k) { return S1[z * N2 + ty * N + k]; }, 0);
+      bits = max(bits, conv_bits(w[z]));
+    }
+    atomicMax(&sB[3 * cs], bits);
     __syncthreads();
+    const int sq = sB[3 * cs] - kFixWide;
+    up = sq - sf - kFixWide;
+#pragma unroll
+    for (int z = 0; z < N; z++) uq[z] = limbs(conv_shift(w[z], sq));
     // F_dir = G_dir u at the point (tx, ty, z)
     const int ebg = EG == kFixZero ? kFixMinBiased : EG + 1022;
 #pragma unroll
@@ -244,7 +272,9 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   __syncthreads();
   {
     // x: Tx = D^t F_x, Ty = B^t F_y, Tz = B^t F_z
-    int2 B[N], D[N], T[3][N];
+    int2 B[N], D[N];
+    long long T[3][N];
+    int bits = 0;
 #pragma unroll
     for (int k = 0; k < N; k++) {
       B[k] = tB[k * N + tx];
@@ -253,22 +283,29 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
 #pragma unroll
     for (int z = 0; z < N; z++) {
       const int i = z * N2 + ty * N;
-      T[0][z] = limbs(conv_sum<N>([&](int k) { return D[k]; }, [&](int k) { return S0[i + k]; }, sb));
-      T[1][z] = limbs(conv_sum<N>([&](int k) { return B[k]; }, [&](int k) { return S1[i + k]; }, sb));
-      T[2][z] = limbs(conv_sum<N>([&](int k) { return B[k]; }, [&](int k) { return S2[i + k]; }, sb));
+      T[0][z] = conv_sum<N>([&](int k) { return D[k]; }, [&](int k) { return S0[i + k]; }, 0);
+      T[1][z] = conv_sum<N>([&](int k) { return B[k]; }, [&](int k) { return S1[i + k]; }, 0);
+      T[2][z] = conv_sum<N>([&](int k) { return B[k]; }, [&](int k) { return S2[i + k]; }, 0);
+#pragma unroll
+      for (int d = 0; d < 3; d++) bits = max(bits, conv_bits(T[d][z]));
     }
+    atomicMax(&sB[3 * cs + 1], bits);
     __syncthreads();
+    const int st = sB[3 * cs + 1] - kFixWide;
+    up += st;
 #pragma unroll
     for (int z = 0; z < N; z++) {
-      S0[z * N2 + l] = T[0][z];
-      S1[z * N2 + l] = T[1][z];
-      S2[z * N2 + l] = T[2][z];
+      S0[z * N2 + l] = limbs(conv_shift(T[0][z], st));
+      S1[z * N2 + l] = limbs(conv_shift(T[1][z], st));
+      S2[z * N2 + l] = limbs(conv_shift(T[2][z], st));
     }
   }
   __syncthreads();
   {
     // y: Sxy = B^t Tx + D^t Ty, Sz = B^t Tz (same unit, one bit larger)
     int2 B[N], D[N], Sxy[N], Sz[N];
+    long long wxy[N], wz[N];
+    int bits = 0;
 #pragma unroll
     for (int k = 0; k < N; k++) {
       B[k] = tB[k * N + ty];
@@ -277,11 +314,18 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
 #pragma unroll
     for (int z = 0; z < N; z++) {
       const int i = z * N2 + tx;
-      Sxy[z] = limbs(conv_sum<2 * N>(
+      wxy[z] = conv_sum<2 * N>(
           [&](int k) { return k < N ? B[k < N ? k : 0] : D[k < N ? 0 : k - N]; },
-          [&](int k) { return k < N ? S0[i + k * N] : S1[i + (k - N) * N]; }, sb + 1));
-      Sz[z] = limbs(conv_sum<N>([&](int k) { return B[k]; },
-                                [&](int k) { return S2[i + k * N]; }, sb + 1));
+          [&](int k) { return k < N ? S0[i + k * N] : S1[i + (k - N) * N]; }, 0);
+      wz[z] = conv_sum<N>([&](int k) { return B[k]; }, [&](int k) { return S2[i + k * N]; }, 0);
+      bits = max(bits, max(conv_bits(wxy[z]), conv_bits(wz[z])));
+    }
+    const int sy = bits - kFixWide;   // of this thread's column
+    up += sy + ce.ed + 2 * ce.eb;
+#pragma unroll
+    for (int z = 0; z < N; z++) {
+      Sxy[z] = limbs(conv_shift(wxy[z], sy));
+      Sz[z] = limbs(conv_shift(wz[z], sy));
     }
     // z: r = B^t Sxy + D^t Sz
 #pragma unroll
@@ -309,9 +353,12 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
     }
   }
   __syncthreads();
-  // ---- upwind flux at the face points (into Un) ----
+  // ---- upwind flux at the face points (into Un), 59 bits of the largest ----
+  int sfl;
   {
     int2 B[N];
+    long long w6[6];
+    int s6[6], bits = -1000;
 #pragma unroll
     for (int k = 0; k < N; k++) B[k] = tB[ty * N + k];
 #pragma unroll
@@ -324,7 +371,8 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
       const bool own = out ? on || bc == PDG_BC_DIRICHLET || bc == PDG_BC_OUTFLOW
                            : !on && bc == PDG_BC_OUTFLOW;
       const bool inflow = !out && on && !a.diag_only;
-      int2 v = make_int2(0, 0);
+      w6[f] = 0;
+      s6[f] = 0;
       if (own || inflow) {
         const int2 *U = own ? Ue : fl;
         const int2 w = limbs(conv_sum<N>([&](int k) { return B[k]; },
@@ -333,11 +381,17 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
         const int Es = own ? Eu : sE[7 * cs + 1 + f];
         long long hh = 0, mid = 0;
         mac2(hh, mid, fix_limbs(bn, EF == kFixZero ? kFixMinBiased : EF + 1022), w);
-        const int s = min(Efl - (Es + 2 * ce.lb + EF), 62);
-        v = limbs((mac2_value_wide(hh, mid) + ((1ll << s) >> 1)) >> s);
+        w6[f] = mac2_value_wide(hh, mid);
+        s6[f] = Efl - (Es + 2 * ce.lb + EF);
+        if (w6[f]) bits = max(bits, conv_bits(w6[f]) - s6[f]);
       }
-      Un[f * N2 + l] = v;
     }
+    atomicMax(&sB[3 * cs + 2], bits + 1000);
+    __syncthreads();
+    const int top = sB[3 * cs + 2];
+    sfl = top ? top - 1000 - kFixWide : 0;   // (0: no flux)
+#pragma unroll
+    for (int f = 0; f < 6; f++) Un[f * N2 + l] = limbs(conv_shift(w6[f], s6[f] + sfl));
   }
   __syncthreads();
   // ---- test with the face basis: rows (into Ue), then columns (into fl) ----
@@ -367,10 +421,10 @@ __global__ void __launch_bounds__(CCfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 6 : N 
   const int sg = flip & (int)0x80000000;
   const double uv =
       Evol > kNone
-          ? __hiloint2double(sg | ((Evol + ce.ldt + ce.lbt + 1 + ce.eb - kFixWide + 1023) << 20), 0)
+          ? __hiloint2double(sg | ((Evol + up + 1023) << 20), 0)
           : 0.0;
   const double uf =
-      Efl > kNone ? __hiloint2double(sg | ((Efl + ce.lbt + ce.eb - kFixWide + 1023) << 20), 0) : 0.0;
+      Efl > kNone ? __hiloint2double(sg | ((Efl + ce.lbt + ce.eb + sfl - kFixWide + 1023) << 20), 0) : 0.0;
   const long long *R = reinterpret_cast<const long long *>(fl);
   double *ye = a.y + e * NB;
 #pragma unroll

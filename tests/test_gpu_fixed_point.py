@@ -292,3 +292,16 @@ def test_odd_and_rounding_of_smooth_data(k, kind):
     noise = np.linalg.norm(apply(go, 3 * u, tr) - 3 * apply(go, u, tr))
     assert noise <= 3 * 8 * 2.0 ** -53 * terms
     go.close()
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+def test_rounding_of_convection_alone(k):
+    """The bound of the test above where convection is all of J."""
+    go, P, rng = problem(k, (6, 6, 6), scale=1e-9)
+    go.set_velocity_modes(pdg.fourier_velocity_modes(1))
+    u = smooth(k, 6)
+    terms = np.linalg.norm(apply(go, u * rng.choice([-1.0, 1.0], u.size)))
+    noise = np.linalg.norm(apply(go, 3 * u) - 3 * apply(go, u))
+    assert noise <= 3 * 8 * 2.0 ** -53 * terms
+    assert not apply(go, np.zeros(go.ndof)).any()
+    go.close()
