@@ -30,6 +30,9 @@
 // record removes all divisions and matrix assembly from the apply, and in
 // 3D it carries per face the coefficients of the neighbour line (see
 // k_cell_record) so that each face point costs N + 1 FP64 operations.
+// In 3D this kernel runs cell lists, diagonal blocks and FP32 of degree 4;
+// whole grids run in fixed point (pdg_apply_p.cu, pdg_apply_i.cu), in
+// pdg_apply_m.cu, or in FP32 in pdg_cell32.cu and pdg_apply32.cu.
 //
 // Thread mapping (d = 3): N*N threads per cell, thread (tx,ty) holds the
 // z-column u[.,ty,tx] in registers; x/y contractions go through shared

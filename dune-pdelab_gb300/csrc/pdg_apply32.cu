@@ -1,19 +1,19 @@
-// pdg_apply32.cu -- the FP32 cell operator of the mixed-precision inner
-// solve (3D, degrees 1 to 3), laid out for shared-memory throughput.
+// pdg_apply32.cu -- the FP32 cell operator of degree 3 of the mixed-precision
+// inner solve (3D), laid out for shared-memory throughput.
 //
 // Same operator as k_apply (pdg_apply.cu; reference: ConvectionDiffusionDG::
 // jacobian_apply_volume / _skeleton / _boundary, localoperator/
 // convectiondiffusiondg.hh:191-195, 474-481, 892-899) in the Kronecker form
 //   y_e = sum_dir (A'_dir (x) Mhat (x) Mhat)_dir u_e + neighbour couplings,
 // with A'_dir and the face coefficients read from a per-cell FP32 record
-// (built from the FP64 arithmetic once per coefficient field).
+// (built from the FP64 arithmetic once per coefficient field).  Degrees 1 and 2
+// are pdg_cell32.cu.
 //
 // Layout.  A CTA owns CPB consecutive cells.  Its own cells (plus one halo
-// cell each side, the x-neighbours) and the four runs of y- and
-// z-neighbour cells (cells e -/+ nx and e -/+ nx*ny of a consecutive run
-// are consecutive runs as well) are copied into shared memory with
-// coalesced loads, so every cell value crosses the L1 once per CTA.  Each
-// thread then owns one z-plane of one cell (N threads per cell): the x and y
+// cell each side, the x-neighbours) and the runs of y-neighbour cells (cells
+// e -/+ nx of a consecutive run are consecutive runs as well) are staged in
+// shared memory, so every cell value crosses the L1 once per CTA.  Each thread
+// then owns one z-plane of one cell (4 threads per cell): the x and y
 // contractions of its plane run in registers, the z contractions read the
 // other planes from shared memory.
 //
@@ -23,8 +23,6 @@
 //   stage 2 (after P is shared):
 //     Z   = sum_z' A'_z[z][z'] u_z' + z-face terms
 //     out = (Mhat_y (x) Mhat_x) Z + sum_z' Mhat_z[z][z'] P_z'
-//
-// The output is staged in shared memory and written back coalesced.
 #include <cuda.h>
 
 #include <algorithm>

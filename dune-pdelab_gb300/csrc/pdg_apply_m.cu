@@ -1,5 +1,8 @@
 // pdg_apply_m.cu -- the 3D FP64 cell operator with the mass matrix factored
-// out (the form of the coupled applies, of the operator and of its transpose).
+// out: the coupled applies, of the operator and of its transpose, on the
+// Gauss-Lobatto nodes of degrees 3 and 4, whose mass matrices are not small
+// integers over a common denominator (on the others pdg_apply_i.cu and
+// pdg_apply_p.cu compute in fixed point).
 //
 // Same operator as k_apply<double, 3, N> (pdg_apply.cu; reference:
 // ConvectionDiffusionDG::jacobian_apply_volume / _skeleton / _boundary,
@@ -256,8 +259,6 @@ int prepare_apply_m(pdg_context *ctx, int transpose) {
     return set_error(PDG_EINVAL, "mass-factored records need the FP64 records and tables");
   int st;
   switch (ctx->N) {
-    case 2: st = record_m_n<2>(ctx, transpose); break;
-    case 3: st = record_m_n<3>(ctx, transpose); break;
     case 4: st = record_m_n<4>(ctx, transpose); break;
     case 5: st = record_m_n<5>(ctx, transpose); break;
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
@@ -288,8 +289,6 @@ static int launch_m_n(pdg_context *ctx, const ApplyArgs<double> &a, const OpPara
 int launch_apply_m(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<double> &p) {
   PDG_TRY(prepare_apply_m(ctx, a.transpose));
   switch (ctx->N) {
-    case 2: return launch_m_n<2>(ctx, a, p);
-    case 3: return launch_m_n<3>(ctx, a, p);
     case 4: return launch_m_n<4>(ctx, a, p);
     case 5: return launch_m_n<5>(ctx, a, p);
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");

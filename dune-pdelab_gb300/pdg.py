@@ -16,10 +16,11 @@ code keeps its shape:
 
 Vectors are numpy float64 arrays (host) or torch tensors on the GPU (device
 pointers are passed straight through).  Unless a stream is bound with
-``GridOperator.set_stream``, every call that can touch device buffers is
-ordered after the work already queued on torch's current stream, and torch's
-current stream waits for the call's work (events, no host synchronisation),
-so tensors made or read by torch around a call need no explicit
+``GridOperator.set_stream``, single operations on device vectors (applies,
+preconditioner applies) run on torch's current stream itself, and every other
+call that can touch device buffers is ordered after the work already queued
+there, with torch's current stream waiting for the call's work (events, no host
+synchronisation), so tensors made or read by torch around a call need no explicit
 ``torch.cuda.synchronize()``.  Every failure raises ``PDGError``
 with the library's message, as the reference raises Dune exceptions.
 There is no CPU fallback: without the CUDA library nothing here works.
