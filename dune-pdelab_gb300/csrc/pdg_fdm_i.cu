@@ -6,7 +6,7 @@
 // (backend/istl/matrixfree/assembledblockjacobipreconditioner.hh:162-233).
 // Six contractions with per-cell matrices, 6 N + 1 multiply-adds per DOF: in
 // FP64 bound by that pipe (1.8 lane operations per SM and cycle), here three
-// IMAD.WIDE each.  FP64 vectors in and out.  47x53x49 Q3: 136 us, in FP64
+// IMAD.WIDE each.  FP64 vectors in and out.  47x53x49 Q3: 127 us, in FP64
 // arithmetic 374 us; the error against 64 bits is the same (4.8e-15, that of
 // the factors).
 //
