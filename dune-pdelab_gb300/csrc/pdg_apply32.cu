@@ -1028,6 +1028,8 @@ __global__ void __launch_bounds__(Q3T::THREADS, 3)
     if (!mbar_wait(b ? bar1 : bar0, (unsigned)((it >> 1) & 1), kTmaPolls)) {
       if (threadIdx.x == 0) atomicExch(tma_err, 1);
       mbar_wait(b ? bar1 : bar0, (unsigned)((it >> 1) & 1), kTmaPolls);
+      if (r + G < nruns)   // the other region's copies are in flight as well
+        mbar_wait(b ? bar0 : bar1, (unsigned)(((it + 1) >> 1) & 1), kTmaPolls);
       return;
     }
     part += (double)q3_run<kTr>(p, a, tb, base + b * Q3P::STAGE, r * CPB, zl, zh);

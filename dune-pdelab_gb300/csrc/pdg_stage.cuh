@@ -32,9 +32,7 @@ struct Stager {
       if (threadIdx.x == 0) {
         // every copy is announced before it is issued; the phase completes
         // with the arrival in wait()
-        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar),
-                     "r"((unsigned)sizeof(V) * len)
-                     : "memory");
+        mbar_announce_tx(bar, (unsigned)sizeof(V) * len);
         bulk_load(smem_u32(dst), src + ga, (unsigned)sizeof(V) * len, bar);
       }
     } else {
@@ -45,11 +43,13 @@ struct Stager {
     }
     return dst + ph;
   }
-  // false: the copies did not arrive within the poll limit
+  // false: the copies did not arrive within the poll limit.  They may still be
+  // in flight then, and a block must not leave its shared memory to the next one
+  // while they are: a failed wait gives them the same time once more.
   __device__ __forceinline__ bool wait() {
-    if (threadIdx.x == 0)
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+    if (threadIdx.x == 0) mbar_arrive(bar);
     const bool ok = mbar_wait(bar, 0, kTmaPolls);
+    if (!ok) mbar_wait(bar, 0, kTmaPolls);
     return __syncthreads_and(ok);
   }
 };

@@ -21,6 +21,14 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+// more bytes of the current phase, without an arrival
+__device__ __forceinline__ void mbar_announce_tx(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 // true once phase `parity` of the barrier completed; at most `limit` polls
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int limit) {
   for (int it = 0; it < limit; it++) {
