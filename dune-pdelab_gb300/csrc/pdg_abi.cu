@@ -267,7 +267,22 @@ static RedCtx red_ctx(pdg_context *ctx) {
   return RedCtx{ctx->red_partials, ctx->red_out, ctx->d_flag};
 }
 
-// pinned host mirror: h_red[0..S_COUNT) scalars, then F_COUNT ints
+// A bounded device wait that ran out since the last report: the kernel left part of
+// its result unwritten.  Every call that has waited for the device looks; what an
+// asynchronous call left behind is reported by the next one that waits.
+static int report_waits(pdg_context *ctx) {
+  volatile int *flag = ctx->h_wait;
+  if (!*flag) return PDG_OK;
+  *flag = 0;
+  return set_error(PDG_ETIMEOUT, "a bounded device wait ran out");
+}
+// wait for the context's stream and report
+static int finish_call(pdg_context *ctx) {
+  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return report_waits(ctx);
+}
+
+// pinned host mirror: h_red[0..S_COUNT) scalars, then 3 F_COUNT ints, then h_wait
 static int fetch_state(pdg_context *ctx, double *scal, int *flags) {
   PDG_CUDA_TRY(cudaMemcpyAsync(ctx->h_red, ctx->red_out, sizeof(double) * S_COUNT,
                                cudaMemcpyDeviceToHost, ctx->stream));
@@ -277,8 +292,7 @@ static int fetch_state(pdg_context *ctx, double *scal, int *flags) {
   PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (scal) std::memcpy(scal, ctx->h_red, sizeof(double) * S_COUNT);
   if (flags) std::memcpy(flags, hf, sizeof(int) * F_COUNT);
-  if (hf[F_TMA]) return set_error(PDG_ETIMEOUT, "a bounded device wait ran out");
-  return PDG_OK;
+  return report_waits(ctx);
 }
 
 // after batch k of CG iterations: copy the flags behind it, and look at those
@@ -294,9 +308,8 @@ static int poll_batch(pdg_context *ctx, int k, bool *done) {
   if (k == 0) return PDG_OK;
   PDG_CUDA_TRY(cudaEventSynchronize(ctx->ev_poll[(k - 1) & 1]));
   const int *f = slots + F_COUNT * ((k - 1) & 1);
-  if (f[F_TMA]) return set_error(PDG_ETIMEOUT, "a bounded device wait ran out");
   if (f[F_STATE]) *done = true;
-  return PDG_OK;
+  return report_waits(ctx);
 }
 
 __global__ void k_set_scal(double *scal, int slot, double v) { scal[slot] = v; }
@@ -310,7 +323,6 @@ __global__ void k_init_solve(double *scal, int *flags, double red, double guard 
   flags[F_STATE] = 0;
   flags[F_COUNTER] = 0;
   flags[F_XPEND] = 0;
-  flags[F_TMA] = 0;   // a staging timeout is reported by the solve it happened in only
 }
 
 template <typename T>
@@ -836,8 +848,7 @@ template <typename T>
 static int stage_out(pdg_context *ctx, const Staged<T> &s) {
   if (!s.staged) return PDG_OK;
   PDG_CUDA_TRY(cudaMemcpyAsync(s.host, s.dev, s.n * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
-  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return PDG_OK;
+  return finish_call(ctx);
 }
 
 static int upload(pdg_context *ctx, double **dst, const double *src, size_t n) {
@@ -1133,7 +1144,7 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
       cudaMalloc(&c->red_partials, sizeof(double) * 2 * kRedBlocks) != cudaSuccess ||
       cudaMalloc(&c->red_out, sizeof(double) * S_COUNT) != cudaSuccess ||
       cudaMalloc(&c->d_flag, sizeof(int) * F_COUNT) != cudaSuccess ||
-      cudaMallocHost(&c->h_red, sizeof(double) * S_COUNT + sizeof(int) * 3 * F_COUNT) != cudaSuccess)
+      cudaMallocHost(&c->h_red, sizeof(double) * S_COUNT + sizeof(int) * (3 * F_COUNT + 1)) != cudaSuccess)
     return fail(set_error(PDG_ECUDA, "device allocation failed"));
   cudaMemcpy(c->tab64, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice);
   if (c->dim == 3) {
@@ -1211,6 +1222,8 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
   cudaMemcpy(c->K64, ones.data(), sizeof(double) * c->ncell, cudaMemcpyHostToDevice);
   cudaMemcpy(c->K32, ones32.data(), sizeof(float) * c->ncell, cudaMemcpyHostToDevice);
   cudaMemset(c->d_flag, 0, sizeof(int) * F_COUNT);
+  c->h_wait = reinterpret_cast<int *>(c->h_red + S_COUNT) + 3 * F_COUNT;
+  *c->h_wait = 0;
   cudaMemset(c->red_out, 0, sizeof(double) * S_COUNT);
   if (c->basis == PDG_BASIS_LEGENDRE) {
     double lt[2 * kMaxN1 * kMaxN1];
@@ -1770,8 +1783,7 @@ static int apply_pipelined(pdg_context *ctx, const double *x, double *y, const d
   PDG_CUDA_TRY(cudaEventRecord(ev_end, ctx->pipe_d2h));
   PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ev_k2, 0));
   PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ev_end, 0));
-  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return PDG_OK;
+  return finish_call(ctx);
 }
 
 // y = (acc ? y : 0) + alpha J x + (with_r0 ? R(0) : 0), host or device vectors
@@ -2110,8 +2122,8 @@ int pdg_newton_solve(pdg_context *ctx, const pdg_newton_options *opt,
   res->elapsed = ms * 1e-3;
   res->status = st;
   for (auto &b : buf) cudaFree(b);
-  const int so = stage_out<double>(ctx, su);
-  return st != PDG_OK ? st : so;
+  const int so = stage_out<double>(ctx, su), sw = so == PDG_OK ? report_waits(ctx) : so;
+  return st != PDG_OK ? st : sw;
 }
 
 int pdg_mass_apply(pdg_context *ctx, const double *x, double *y) {
@@ -2123,8 +2135,7 @@ int pdg_mass_apply(pdg_context *ctx, const double *x, double *y) {
   PDG_TRY(stage_in<double>(ctx, y, ctx->ndof, ctx->stage_b, false, &sy));
   PDG_TRY(mass_apply(ctx, sx.dev, sy.dev, 1.0, 0, 0));
   PDG_TRY(stage_out<double>(ctx, sy));
-  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return PDG_OK;
+  return finish_call(ctx);
 }
 
 // Tables of instationary/onestepparameter.hh (the published schemes:
@@ -2357,6 +2368,7 @@ int pdg_onestep_apply(pdg_context *ctx, int stages, const double *A, const doubl
   if (ctx->mass_shift_on) set_mass_shift(ctx, 0.0, true, ctx->c_orig64, ctx->c_orig32);
   ctx->mass_shift_on = 0;
   for (auto &p : buf) cudaFree(p);
+  if (st == PDG_OK) st = report_waits(ctx);
   res->status = st;
   if (st != PDG_OK) return st;
   PDG_TRY(stage_out<double>(ctx, sn));
@@ -2466,7 +2478,7 @@ int pdg_solve_linear_problem(pdg_context *ctx, const pdg_solver_options *opt, do
   // x -= z   (:294)
   if (st == PDG_OK || st == PDG_ENOTCONVERGED) PDG_TRY(vec_axpy(ctx, n, -1.0, z, sx.dev));
   PDG_TRY(stage_out<double>(ctx, sx));
-  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  PDG_TRY(finish_call(ctx));
   return st;
 }
 
@@ -2496,7 +2508,7 @@ int pdg_adjoint_solve(pdg_context *ctx, const pdg_solver_options *opt, const dou
     o.preconditioner = (o.preconditioner & ~PDG_PREC_BLOCK_MASK) | PDG_PREC_BJ_DENSE;
   const int st = solve_correction(ctx, &o, sl.dev, r, transpose, res);
   PDG_TRY(stage_out<double>(ctx, sl));
-  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  PDG_TRY(finish_call(ctx));
   return st;
 }
 
@@ -2524,8 +2536,7 @@ int pdg_grad_logK(pdg_context *ctx, const double *u, const double *lambda, doubl
   if (hg)
     PDG_CUDA_TRY(cudaMemcpyAsync(g, gd, sizeof(double) * ctx->ncell, cudaMemcpyDeviceToHost,
                                  ctx->stream));
-  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return PDG_OK;
+  return finish_call(ctx);
 }
 
 int pdg_grad_source(pdg_context *ctx, const double *lambda, double *g) {
@@ -2546,8 +2557,7 @@ int pdg_grad_source(pdg_context *ctx, const double *lambda, double *g) {
   if (hg)
     PDG_CUDA_TRY(cudaMemcpyAsync(g, gd, sizeof(double) * ctx->ncell, cudaMemcpyDeviceToHost,
                                  ctx->stream));
-  PDG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return PDG_OK;
+  return finish_call(ctx);
 }
 
 }  // extern "C"

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(Q3Cfg::THREADS, 5)
     }
     if (!mbar_wait(bar, 0, kTmaPolls)) {
       // record the failure, give the copies a last chance to land, leave
-      if (threadIdx.x == 0) atomicExch(tma_err, 1);
+      if (threadIdx.x == 0) raise_timeout(tma_err);
       mbar_wait(bar, 0, kTmaPolls);
       return;
     }
@@ -935,7 +935,7 @@ __global__ void __launch_bounds__(Q3T::THREADS, 5)
       bulk_load(smem_u32(base + C::REC_B), rec + e0 * REC, rbytes, bar);
     }
     if (!mbar_wait(bar, 0, kTmaPolls)) {
-      if (threadIdx.x == 0) atomicExch(tma_err, 1);
+      if (threadIdx.x == 0) raise_timeout(tma_err);
       mbar_wait(bar, 0, kTmaPolls);
       return;
     }
@@ -1026,7 +1026,7 @@ __global__ void __launch_bounds__(Q3T::THREADS, 3)
     float4 nzl[N], nzh[N];
     if (r + G < nruns) q3_zrows(p, a.x, r + G, nzl, nzh);
     if (!mbar_wait(b ? bar1 : bar0, (unsigned)((it >> 1) & 1), kTmaPolls)) {
-      if (threadIdx.x == 0) atomicExch(tma_err, 1);
+      if (threadIdx.x == 0) raise_timeout(tma_err);
       mbar_wait(b ? bar1 : bar0, (unsigned)((it >> 1) & 1), kTmaPolls);
       if (r + G < nruns)   // the other region's copies are in flight as well
         mbar_wait(b ? bar0 : bar1, (unsigned)(((it + 1) >> 1) & 1), kTmaPolls);
@@ -1159,7 +1159,7 @@ static int launch32_q3(pdg_context *ctx, const ApplyArgs<float> &a, const OpPara
   }
   const EdgeTab &tb = edge_tab(ctx);
   const unsigned blocks = (unsigned)((ctx->ncell + Q3Cfg::CPB - 1) / Q3Cfg::CPB);
-  int *err = ctx->d_flag + F_TMA;
+  int *err = ctx->h_wait;
   const CUtensorMap *own = nullptr, *run = nullptr;
   // TMA needs a 16-byte aligned vector (and records, from cudaMalloc)
   if ((reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(rec) & 15) == 0 &&

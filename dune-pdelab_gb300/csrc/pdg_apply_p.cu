@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
   const int EA = ex[0];
   bool bad = ex[13 * T] == 0;
   if (!st.wait()) {
-    if (threadIdx.x == 0) atomicExch(tma_err, 1);
+    if (threadIdx.x == 0) raise_timeout(tma_err);
     return;
   }
 
@@ -526,7 +526,7 @@ int launch_apply_p(pdg_context *ctx, const ApplyArgs<double> &a, const OpParams<
   const unsigned blocks = (unsigned)((c1 - 1) / C::T - c0 / C::T + 1);
   k_apply_p<<<blocks, C::THREADS, smem, ctx->stream>>>(
       p, a, a.transpose ? ctx->reciT : ctx->reci, a.transpose ? ctx->reciT_exp : ctx->reci_exp,
-      ctx->rec64, ctx->d_flag + F_TMA);
+      ctx->rec64, ctx->h_wait);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }

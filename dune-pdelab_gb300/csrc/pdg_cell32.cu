@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(C32Cfg<N>::THREADS)
   const float *zl = cp && ix[2] > 0 ? (half ? ZL1 : ZL) + cs * NB : zero;
   const float *zh = cp && ix[2] + 1 < p.nc[2] ? (half ? ZH : ZH0) + cs * NB : zero;
   if (!st.wait()) {
-    if (threadIdx.x == 0) atomicExch(tma_err, 1);
+    if (threadIdx.x == 0) raise_timeout(tma_err);
     return;
   }
   const float a1 = a.transpose ? -p.theta : 1.f, a2 = a.transpose ? 1.f : -p.theta;
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(C32Cfg<N>::T, 9)
   st.run(Q0, Q, e0 * 3 * N2, ncell * 3 * N2, T * 3 * N2);
   st.run(L0, L, e0 * 3 * N, ncell * 3 * N, T * 3 * N);
   if (!st.wait()) {
-    if (threadIdx.x == 0) atomicExch(tma_err, 1);
+    if (threadIdx.x == 0) raise_timeout(tma_err);
     return;
   }
   const int cs = threadIdx.x;
@@ -571,11 +571,11 @@ static int launch_apply32_cell_n(pdg_context *ctx, const ApplyArgs<float> &a,
   // stacked runs while they take at most a quarter more blocks
   if (4 * stack <= 5 * side)
     k_apply32_cell<N, true><<<(unsigned)stack, C::THREADS, sizeof(float) * C::SMEM, ctx->stream>>>(
-        p, a, ctx->rec32c, tb, ctx->d_flag + F_TMA);
+        p, a, ctx->rec32c, tb, ctx->h_wait);
   else
     k_apply32_cell<N, false>
         <<<(unsigned)side, C::THREADS, sizeof(float) * C::SMEM_SIDE, ctx->stream>>>(
-            p, a, ctx->rec32c, tb, ctx->d_flag + F_TMA);
+            p, a, ctx->rec32c, tb, ctx->h_wait);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }
@@ -599,7 +599,7 @@ static int fdm32_cell_n(pdg_context *ctx, const float *d, float *v, const int *s
       const_cast<float *>(d), v, skip, scale, fuse ? ctx->fuse_part : nullptr,
       ctx->fuse_max_blocks, ctx->fuse_cnt, ctx->red_out, ctx->d_flag, ctx->fuse_fin,
       (fuse && ctx->fuse_fin == FIN_CG_DEF_BETA) ? (const float *)ctx->fuse_q : nullptr,
-      ctx->d_flag + F_TMA);
+      ctx->h_wait);
   PDG_CUDA_TRY(cudaGetLastError());
   return PDG_OK;
 }

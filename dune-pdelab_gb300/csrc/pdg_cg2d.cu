@@ -34,6 +34,7 @@
 #include <algorithm>
 
 #include "pdg_ops.cuh"
+#include "pdg_tma.cuh"
 #include "pdg_vec.cuh"
 
 namespace pdg {
@@ -64,7 +65,7 @@ struct Cg2Args {
   unsigned long long *slots;   // [kCg2Sets][2][grid] partial sums, all empty,
   unsigned long long *result;  // [kCg2Sets][kCg2Copies][16] scalars, all empty
   double *scal;
-  int *flags;
+  int *flags, *timeout;
   int maxit, cells_per_block;
 };
 
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(kCg2Threads)
     g.scal[S_ITER] = it;
     if (state > 0) g.flags[F_STATE] = state;
   }
-  if (state < 0 && t == 0) atomicExch(&g.flags[F_TMA], 1);
+  if (state < 0 && t == 0) raise_timeout(g.timeout);
 }
 
 __global__ void k_cg2d_slots(unsigned long long *s, int n) {
@@ -398,7 +399,7 @@ static int cg2d_n(pdg_context *ctx, double *x, double *b, double *p, double *p2,
   OpParams<double> pr = make_params<double>(ctx, ctx->K64, ctx->c64, ctx->tab64);
   const PrecData &pd = ctx->prec[PDG_F64];
   Cg2Args g{ctx->rec64, (const double *)pd.Q, pd.Lsum_inv, x, b, {p, p2}, z, ctx->cg2_slots,
-            ctx->cg2_slots + npart, ctx->red_out, ctx->d_flag, maxit, cap};
+            ctx->cg2_slots + npart, ctx->red_out, ctx->d_flag, ctx->h_wait, maxit, cap};
   void *args[] = {&pr, &g};
   PDG_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_cg2d<N>, dim3(grid), dim3(kCg2Threads), args, smem,
                                            ctx->stream));

@@ -253,6 +253,8 @@ struct pdg_context {
   double *red_partials;    // [kRedBlocks * 4]
   double *red_out;         // [16] device results
   double *h_red;           // pinned host mirror [16]
+  int *h_wait;             // pinned: set by a kernel whose bounded wait ran out, cleared by
+                           // the call that reports it
 
   // local basis (PDG_BASIS_*).  Nodal bases: the k+1 nodes on [0,1].  The
   // modal (Legendre) basis runs the nodal kernels between changes of basis:

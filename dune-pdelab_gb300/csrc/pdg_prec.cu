@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(FdmQ3T::THREADS)
       bulk_load(smem_u32(base + C::LS_B), L + e0 * 12, (unsigned)(cmax * 48), bar);
     }
     if (!mbar_wait(bar, 0, kTmaPolls)) {
-      if (threadIdx.x == 0) atomicExch(tma_err, 1);
+      if (threadIdx.x == 0) raise_timeout(tma_err);
       mbar_wait(bar, 0, kTmaPolls);
       return;
     }
@@ -1237,7 +1237,7 @@ static int fdm_apply_dn(pdg_context *ctx, const T *d, T *v, const int *skip, con
             ctx->ncell, (const float *)ctx->prec[PDG_F32].Q, (const float *)ctx->prec[PDG_F32].L,
             const_cast<float *>(d), v, skip, scale, fuse ? ctx->fuse_part : nullptr,
             ctx->fuse_max_blocks, ctx->fuse_cnt, ctx->red_out, ctx->d_flag, ctx->fuse_fin, rq,
-            *md, rq ? *mq : *md, ctx->d_flag + F_TMA);
+            *md, rq ? *mq : *md, ctx->h_wait);
         PDG_CUDA_TRY(cudaGetLastError());
         return PDG_OK;
       }

@@ -58,6 +58,12 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigne
           "r"(dst), "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
+// a bounded wait ran out: the flag (pdg_context::h_wait) is in host memory, so the
+// host sees it without a copy once the kernel has ended
+__device__ __forceinline__ void raise_timeout(int *flag) {
+  *reinterpret_cast<volatile int *>(flag) = 1;
+}
+
 // polls of the staging barrier before a launch gives up (far above any
 // real copy time); the kernel then records the failure and returns
 constexpr int kTmaPolls = 1 << 22;

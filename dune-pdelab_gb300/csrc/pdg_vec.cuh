@@ -41,9 +41,8 @@ enum Slot {
 
 // flag words (int): [0] state (0 running, 1 converged, 2 non-finite,
 // 3 breakdown), [1] reduction counter (last-block detection), [2] the CG
-// x update of the stopping iteration is still to be applied, [3] a kernel's
-// TMA staging did not complete within its poll limit (sticky)
-enum { F_STATE = 0, F_COUNTER = 1, F_XPEND = 2, F_TMA = 3, F_COUNT = 4 };
+// x update of the stopping iteration is still to be applied
+enum { F_STATE = 0, F_COUNTER = 1, F_XPEND = 2, F_COUNT = 3 };
 
 enum Finisher {
   FIN_STORE = 0,        // scal[slot0] = d0 ; scal[slot1] = d1
