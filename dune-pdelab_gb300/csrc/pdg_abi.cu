@@ -369,12 +369,13 @@ static bool cg_fusable64(const pdg_context *ctx, int transpose) {
 }
 
 static int ensure_fuse(pdg_context *ctx) {
-  if (ctx->fuse_part) return PDG_OK;
   // the fused kernels run at least 4 cells per block
   const long maxb = ctx->ncell / 4 + 2;
   const long ngroups = (maxb + kFuseGroup - 1) / kFuseGroup;
-  PDG_CUDA_TRY(cudaMalloc(&ctx->fuse_part, sizeof(double) * 2 * (maxb + ngroups)));
-  PDG_CUDA_TRY(cudaMalloc(&ctx->fuse_cnt, sizeof(int) * ngroups));
+  if (!ctx->fuse_part)
+    PDG_CUDA_TRY(cudaMalloc(&ctx->fuse_part, sizeof(double) * 2 * (maxb + ngroups)));
+  if (!ctx->fuse_cnt) PDG_CUDA_TRY(cudaMalloc(&ctx->fuse_cnt, sizeof(int) * ngroups));
+  // for every solve: a launch with a block that gave up leaves its counts behind
   PDG_CUDA_TRY(cudaMemsetAsync(ctx->fuse_cnt, 0, sizeof(int) * ngroups, ctx->stream));
   ctx->fuse_max_blocks = maxb;
   return PDG_OK;

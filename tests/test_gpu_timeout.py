@@ -16,8 +16,16 @@ import pdg  # noqa: E402
 CSRC = os.path.join(os.path.dirname(os.path.abspath(pdg.__file__)), "csrc")
 
 POKE = r"""
+#include <vector>
 #include "pdg_vec.cuh"
 extern "C" void timeout_set(pdg_context *ctx) { *ctx->h_wait = 1; }
+// the counts that a launch with a block that gave up leaves behind: one each
+extern "C" int counts_set(pdg_context *ctx) {
+  const int n = (int)((ctx->ncell / 4 + 2 + pdg::kFuseGroup - 1) / pdg::kFuseGroup);
+  const std::vector<int> one(n, 1);
+  return ctx->fuse_cnt ? (int)cudaMemcpy(ctx->fuse_cnt, one.data(), sizeof(int) * n,
+                                         cudaMemcpyHostToDevice) : -1;
+}
 """
 
 
@@ -31,7 +39,7 @@ def poke(tmp_path_factory):
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     lib = ctypes.CDLL(str(d / "poke.so"))
-    lib.timeout_set.argtypes = [ctypes.c_void_p]
+    lib.timeout_set.argtypes = lib.counts_set.argtypes = [ctypes.c_void_p]
     return lib
 
 
@@ -76,4 +84,20 @@ def test_kept_for_the_next_call_that_waits(poke):
     u.zero_()
     slp.apply()
     assert slp.result().converged
+    go.close()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_solve_after_a_launch_that_gave_up(poke, mixed):
+    """The block counts of the fused sums start from zero in every solve."""
+    torch, go, x = operator((12, 11, 10))
+    u = torch.zeros(go.ndof, dtype=torch.float64, device="cuda")
+    ls = pdg.ISTLBackend_SEQ_MatrixFree_Base(go, mixed=mixed)
+    slp = pdg.StationaryLinearProblemSolver(go, ls, u, 1e-8)
+    slp.apply()
+    first, its = u.clone(), slp.result().iterations
+    assert poke.counts_set(go.handle) == 0
+    u.zero_()
+    slp.apply()
+    assert torch.equal(u, first) and slp.result().iterations == its
     go.close()
