@@ -968,22 +968,52 @@ static void invalidate(pdg_context *ctx, bool operator_changed) {
 
 using namespace pdg;
 
-#define PDG_CHECK_CTX(ctx)                                                     \
-  do {                                                                         \
-    if (!(ctx)) return set_error(PDG_EINVAL, "null context");                 \
-    PDG_CUDA_TRY(cudaSetDevice((ctx)->device));                                \
-    if (!(ctx)->run_active) PDG_TRY(own_stream_entry(ctx));                    \
-  } while (0)
-
-// a call on the context's own (or bound) stream follows the calls that ran on
-// callers' streams
-static int own_stream_entry(pdg_context *ctx) {
-  ctx->own_dirty = 1;
-  if (!ctx->own_must_wait) return PDG_OK;
-  ctx->own_must_wait = 0;
-  PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->ev_run, 0));
+// in capture: events recorded outside cannot be waited for, nor the other way round
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    cudaGetLastError();   // the legacy stream beside a capture elsewhere
+    return true;
+  }
+  return cs != cudaStreamCaptureStatusNone;
+}
+static int mark(cudaEvent_t *ev, cudaStream_t s) {
+  if (!*ev) PDG_CUDA_TRY(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+  PDG_CUDA_TRY(cudaEventRecord(*ev, s));
   return PDG_OK;
 }
+
+// One call on a context.  Work of the context may have run on three kinds of
+// streams: its own, one bound by pdg_set_stream, callers' (pdg_run_on).  A call on
+// the own stream follows the last pdg_run_on; the end of a call on a bound stream
+// is marked, since that stream may be gone when the context leaves it.
+struct CtxCall {
+  pdg_context *const ctx;
+  int status;
+  explicit CtxCall(pdg_context *c) : ctx(c), status(enter()) {}
+  CtxCall(const CtxCall &) = delete;
+  ~CtxCall() {
+    if (status == PDG_OK && !ctx->run_active && ctx->stream != ctx->own_stream &&
+        !capturing(ctx->stream))
+      mark(&ctx->ev_bound, ctx->stream);
+  }
+
+ private:
+  int enter() const {
+    PDG_CUDA_TRY(cudaSetDevice(ctx->device));
+    if (ctx->run_active || ctx->stream != ctx->own_stream) return PDG_OK;
+    ctx->own_dirty = 1;
+    if (!ctx->own_must_wait || capturing(ctx->stream)) return PDG_OK;
+    ctx->own_must_wait = 0;
+    PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->ev_run, 0));
+    return PDG_OK;
+  }
+};
+
+#define PDG_CHECK_CTX(ctx)                                \
+  if (!(ctx)) return set_error(PDG_EINVAL, "null context"); \
+  const CtxCall ctx_call(ctx);                            \
+  if (ctx_call.status != PDG_OK) return ctx_call.status
 
 extern "C" {
 
@@ -1253,6 +1283,7 @@ int pdg_destroy(pdg_context *c) {
   if (c->run_pending) cudaEventSynchronize(c->ev_run);
   if (c->ev_run) cudaEventDestroy(c->ev_run);
   if (c->ev_own) cudaEventDestroy(c->ev_own);
+  if (c->ev_bound) cudaEventDestroy(c->ev_bound);
   if (c->pipe_h2d) {
     cudaStreamSynchronize(c->pipe_h2d);
     cudaStreamSynchronize(c->pipe_d2h);
@@ -1297,9 +1328,25 @@ int pdg_destroy(pdg_context *c) {
 }
 
 int pdg_set_stream(pdg_context *ctx, void *stream) {
-  PDG_CHECK_CTX(ctx);
+  if (!ctx) return set_error(PDG_EINVAL, "null context");
   if (ctx->run_active) return set_error(PDG_ESTATE, "pdg_set_stream inside pdg_run_on");
-  ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;
+  PDG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const cudaStream_t s = stream ? (cudaStream_t)stream : ctx->own_stream, old = ctx->stream;
+  if (s == old) return PDG_OK;
+  // the new stream follows what ran on the others
+  if (!capturing(s)) {
+    if (ctx->run_pending) PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_run, 0));
+    if (ctx->ev_bound) PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_bound, 0));
+    if (old == ctx->own_stream && ctx->own_dirty && !capturing(old)) {
+      PDG_TRY(mark(&ctx->ev_own, old));
+      PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_own, 0));
+    }
+    if (s == ctx->own_stream) {
+      ctx->own_must_wait = 0;
+      ctx->own_dirty = 1;   // for the next pdg_run_on
+    }
+  }
+  ctx->stream = s;
   return PDG_OK;
 }
 
@@ -1318,12 +1365,8 @@ int pdg_run_on(pdg_context *ctx, void *stream) {
   // graph's launches are ordered by the caller
   ctx->run_capturing = cs != cudaStreamCaptureStatusNone;
   if (!ctx->run_capturing) {
-    if (!ctx->ev_run) {
-      PDG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ev_run, cudaEventDisableTiming));
-      PDG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ev_own, cudaEventDisableTiming));
-    }
     if (ctx->own_dirty) {
-      PDG_CUDA_TRY(cudaEventRecord(ctx->ev_own, ctx->own_stream));
+      PDG_TRY(mark(&ctx->ev_own, ctx->own_stream));
       PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_own, 0));
       ctx->own_dirty = 0;
     }
@@ -1340,7 +1383,7 @@ int pdg_run_done(pdg_context *ctx) {
   ctx->stream = ctx->own_stream;
   ctx->run_active = 0;
   if (ctx->run_capturing) return PDG_OK;
-  PDG_CUDA_TRY(cudaEventRecord(ctx->ev_run, s));
+  PDG_TRY(mark(&ctx->ev_run, s));
   ctx->run_pending = ctx->own_must_wait = 1;
   return PDG_OK;
 }

@@ -136,8 +136,9 @@ struct pdg_context {
   cudaStream_t stream;
   cudaStream_t own_stream;
   // calls run on a caller's stream (pdg_run_on): ev_run marks the end of the
-  // last such call, ev_own the own stream's work before it
-  cudaEvent_t ev_run, ev_own;
+  // last such call, ev_own the own stream's work before it, ev_bound the last call
+  // on a stream bound by pdg_set_stream
+  cudaEvent_t ev_run, ev_own, ev_bound;
   int run_active, run_capturing, run_pending, own_must_wait, own_dirty;
   int device;
 

@@ -201,7 +201,9 @@ const char *pdg_last_error(void);
 void pdg_default_solver_options(pdg_solver_options *opt);
 
 /* Stream for all subsequent work (cudaStream_t passed as void*; NULL =
-   the context's own non-blocking stream).  No reference counterpart (the
+   the context's own non-blocking stream).  Unless that stream is in capture,
+   its work follows what the context did on other streams before.  PDG_ESTATE
+   between pdg_run_on and pdg_run_done.  No reference counterpart (the
    reference runs on the host). */
 int pdg_set_stream(pdg_context *ctx, void *stream);
 
