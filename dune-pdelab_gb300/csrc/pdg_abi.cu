@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -987,10 +988,14 @@ static int mark(cudaEvent_t *ev, cudaStream_t s) {
 // streams: its own, one bound by pdg_set_stream, callers' (pdg_run_on).  A call on
 // the own stream follows the last pdg_run_on; the end of a call on a bound stream
 // is marked, since that stream may be gone when the context leaves it.
+//
+// The stream and much else that a call sets for its launches stands in the context,
+// so calls of several host threads go one after another.
 struct CtxCall {
   pdg_context *const ctx;
+  const std::lock_guard<std::recursive_mutex> lock;
   int status;
-  explicit CtxCall(pdg_context *c) : ctx(c), status(enter()) {}
+  explicit CtxCall(pdg_context *c) : ctx(c), lock(c->mutex), status(enter()) {}
   CtxCall(const CtxCall &) = delete;
   ~CtxCall() {
     if (status == PDG_OK && !ctx->run_active && ctx->stream != ctx->own_stream &&
@@ -1102,8 +1107,7 @@ int pdg_create(const pdg_config *cfg, pdg_context **out) {
   if (cfg->basis < PDG_BASIS_LAGRANGE || cfg->basis > PDG_BASIS_LOBATTO)
     return set_error(PDG_EINVAL, "bad basis");
   PDG_CUDA_TRY(cudaSetDevice(cfg->device));
-  pdg_context *c = new pdg_context;
-  std::memset(c, 0, sizeof(*c));
+  pdg_context *c = new pdg_context();   // all zero
   c->cfg = *cfg;
   pdg_default_prec_options(&c->popt);
   c->device = cfg->device;
@@ -1329,6 +1333,7 @@ int pdg_destroy(pdg_context *c) {
 
 int pdg_set_stream(pdg_context *ctx, void *stream) {
   if (!ctx) return set_error(PDG_EINVAL, "null context");
+  const std::lock_guard<std::recursive_mutex> lock(ctx->mutex);
   if (ctx->run_active) return set_error(PDG_ESTATE, "pdg_set_stream inside pdg_run_on");
   PDG_CUDA_TRY(cudaSetDevice(ctx->device));
   const cudaStream_t s = stream ? (cudaStream_t)stream : ctx->own_stream, old = ctx->stream;
@@ -1352,6 +1357,7 @@ int pdg_set_stream(pdg_context *ctx, void *stream) {
 
 int pdg_run_on(pdg_context *ctx, void *stream) {
   if (!ctx) return set_error(PDG_EINVAL, "null context");
+  std::unique_lock<std::recursive_mutex> lock(ctx->mutex);
   if (ctx->run_active || ctx->stream != ctx->own_stream)
     return set_error(PDG_ESTATE, "pdg_run_on needs the context on its own stream");
   PDG_CUDA_TRY(cudaSetDevice(ctx->device));
@@ -1374,11 +1380,15 @@ int pdg_run_on(pdg_context *ctx, void *stream) {
   }
   ctx->stream = s;
   ctx->run_active = 1;
+  lock.release();   // until pdg_run_done
   return PDG_OK;
 }
 int pdg_run_done(pdg_context *ctx) {
   if (!ctx) return set_error(PDG_EINVAL, "null context");
-  if (!ctx->run_active) return set_error(PDG_ESTATE, "pdg_run_done without pdg_run_on");
+  std::unique_lock<std::recursive_mutex> lock(ctx->mutex, std::try_to_lock);
+  if (!lock || !ctx->run_active)
+    return set_error(PDG_ESTATE, "pdg_run_done without pdg_run_on on this thread");
+  ctx->mutex.unlock();   // pdg_run_on's; this call still has its own
   const cudaStream_t s = ctx->stream;
   ctx->stream = ctx->own_stream;
   ctx->run_active = 0;
@@ -1389,6 +1399,7 @@ int pdg_run_done(pdg_context *ctx) {
 }
 int pdg_get_stream(const pdg_context *ctx, void **stream) {
   if (!ctx || !stream) return set_error(PDG_EINVAL, "null argument");
+  const std::lock_guard<std::recursive_mutex> lock(ctx->mutex);
   *stream = (void *)ctx->stream;
   return PDG_OK;
 }

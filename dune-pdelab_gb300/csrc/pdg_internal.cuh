@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <type_traits>
 
@@ -140,6 +141,8 @@ struct pdg_context {
   // on a stream bound by pdg_set_stream
   cudaEvent_t ev_run, ev_own, ev_bound;
   int run_active, run_capturing, run_pending, own_must_wait, own_dirty;
+  // one host thread at a time: held during a call, and from pdg_run_on to pdg_run_done
+  mutable std::recursive_mutex mutex;
   int device;
 
   // coefficients on the device

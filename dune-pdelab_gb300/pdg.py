@@ -31,6 +31,7 @@ import ctypes as C
 import functools
 import os
 import sys
+import threading
 
 import numpy as np
 
@@ -257,18 +258,20 @@ def _on_current_stream(method):
     def wrapper(self, *args, **kw):
         go = getattr(self, "go", self)
         torch = sys.modules.get("torch")
-        if (torch is None or go._explicit_stream or not go._h or go._running
+        if (torch is None or go._explicit_stream or not go._h
+                or go._running == threading.get_ident()
                 or not torch.cuda.is_initialized()):
             return method(self, *args, **kw)
         if kw or any(isinstance(a, np.ndarray) for a in args):
             return ordered(self, *args, **kw)
         lib = load()
         _check(lib.pdg_run_on(go._h, torch.cuda.current_stream(go.cfg.device).cuda_stream))
-        go._running = True
+        # other threads wait in pdg_run_on until pdg_run_done
+        go._running = threading.get_ident()
         try:
             return method(self, *args)
         finally:
-            go._running = False
+            go._running = None
             _check(lib.pdg_run_done(go._h))
     return wrapper
 
@@ -356,7 +359,7 @@ class GridOperator:
         self.cfg = cfg
         self.dim, self.degree, self.basis = dim, degree, basis
         self._explicit_stream = False
-        self._running = False        # inside a call on torch's current stream
+        self._running = None         # the thread inside a call on torch's current stream
         self._lib_stream = None
         self._h = _vp()
         _check(load().pdg_create(C.byref(cfg), C.byref(self._h)))

@@ -18,6 +18,10 @@
  *
  * Streams: every call is ordered on the context's stream (pdg_set_stream);
  * calls that return host values (solves, norms, dots) synchronise it.
+ *
+ * Threads: calls of several host threads on one context go one after another
+ * (a call waits until another thread's has returned, and until its
+ * pdg_run_done).  Contexts are independent of each other.
  */
 #ifndef PDG_H
 #define PDG_H
@@ -213,7 +217,8 @@ int pdg_set_stream(pdg_context *ctx, void *stream);
    whatever stream that runs.  For single operations between a caller's own
    work on that stream; a solve replays CUDA graphs on the context's stream and
    should run there.  PDG_ESTATE while a stream is bound by pdg_set_stream, or
-   nested.  A stream in capture is not ordered against work outside the
+   nested.  Other threads' calls on the context wait from pdg_run_on to
+   pdg_run_done, which the same thread makes.  A stream in capture is not ordered against work outside the
    capture.  No reference counterpart. */
 int pdg_run_on(pdg_context *ctx, void *stream);
 int pdg_run_done(pdg_context *ctx);

@@ -1,0 +1,145 @@
+"""Two host threads on one operator.  Each one's single operations run on its own
+current stream of torch; the library lets one thread in at a time from
+pdg_run_on to pdg_run_done.  On CPU with a fake library that has that rule, and
+on the GPU with results."""
+import ctypes
+import sys
+import threading
+import types
+
+import numpy as np
+import pytest
+
+WAIT = 10.0        # seconds after which a hand-over between the threads has failed
+
+
+class _FakeLib:
+    """pdg_run_on .. pdg_run_done as in pdg.h; what ran, on which stream."""
+
+    def __init__(self):
+        self.mutex, self.stream, self.ran = threading.Lock(), "own", []
+        self.waiting = {}              # thread -> it has called pdg_run_on
+
+    def pdg_run_on(self, h, stream):
+        self.waiting.setdefault(threading.get_ident(), threading.Event()).set()
+        if not self.mutex.acquire(timeout=WAIT):
+            return 5
+        self.stream = stream
+        return 0
+
+    def pdg_run_done(self, h):
+        self.stream = "own"
+        self.mutex.release()
+        return 0
+
+
+def test_each_thread_runs_on_its_own_stream(monkeypatch):
+    import pdg
+    lib, local = _FakeLib(), threading.local()
+    monkeypatch.setattr(pdg, "load", lambda *a: lib)
+    cuda = types.SimpleNamespace(
+        is_initialized=lambda: True,
+        current_stream=lambda device=None: types.SimpleNamespace(cuda_stream=local.stream))
+    monkeypatch.setitem(sys.modules, "torch", types.SimpleNamespace(cuda=cuda))
+    go = types.SimpleNamespace(_h=ctypes.c_void_p(1), _explicit_stream=False, _lib_stream=None,
+                               _running=None, cfg=types.SimpleNamespace(device=0))
+    inside, b_seen, errors = threading.Event(), threading.Event(), []
+
+    class Op:
+        def __init__(self):
+            self.go = go
+
+        @pdg._on_current_stream
+        def apply(self, name):
+            lib.ran.append((name, lib.stream))
+            if name == "A":
+                inside.set()
+                b_seen.wait(WAIT)      # until B has tried to come in
+            return self.nested(name)
+
+        @pdg._on_current_stream
+        def nested(self, name):        # within the same thread: no second pdg_run_on
+            lib.ran.append((name, lib.stream))
+            return name
+
+    def thread(name, stream):
+        try:
+            local.stream = stream
+            if name == "B":
+                inside.wait(WAIT)
+                lib.waiting[threading.get_ident()] = b_seen
+            assert Op().apply(name) == name
+        except Exception as e:
+            errors.append(e)
+        finally:
+            if name == "B":
+                b_seen.set()
+
+    ts = [threading.Thread(target=thread, args=a) for a in (("A", 1), ("B", 2))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors
+    assert lib.ran == [("A", 1), ("A", 1), ("B", 2), ("B", 2)]
+    assert go._running is None
+
+
+@pytest.mark.gpu
+def test_threads_on_one_operator():
+    """Applies of two threads behind writes on their own streams, beside a third
+    one's solves: the results are those of one thread."""
+    import pdg
+    import torch
+    rng = np.random.default_rng(1)
+    go = pdg.GridOperator(3, 2, (12, 11, 10), alpha=3.0)
+    go.set_permeability(np.exp(rng.standard_normal(go.ncell)))
+    go.set_source(fc=np.ones(go.ncell))
+    op = pdg.OnTheFlyOperator(go)
+    xs = [torch.tensor(rng.uniform(-1, 1, go.ndof), device="cuda") for _ in range(2)]
+    refs = [torch.zeros_like(x) for x in xs]
+    for x, r in zip(xs, refs):
+        op.apply(x, r)
+    u = torch.zeros_like(xs[0])
+    ls = pdg.ISTLBackend_SEQ_MatrixFree_Base(go)
+    slp = pdg.StationaryLinearProblemSolver(go, ls, u, 1e-8)
+    slp.apply()
+    uref = u.clone()
+    torch.cuda.synchronize()
+    errors = []
+
+    def applies(i):
+        try:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                for n in range(100):
+                    if n % 20 == 0:
+                        torch.cuda._sleep(2_000_000)
+                    x = xs[i] * 1.0
+                    y = torch.zeros_like(x)
+                    op.apply(x, y)
+                    d = (y - refs[i]).abs().max()
+                    if float(d) != 0.0:
+                        raise AssertionError(f"thread {i}, apply {n}: {float(d)}")
+        except BaseException as e:
+            errors.append(e)
+
+    def solves():
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for n in range(10):
+                    u.zero_()
+                    slp.apply()
+                    if not torch.equal(u, uref):
+                        raise AssertionError(f"solve {n}")
+        except BaseException as e:
+            errors.append(e)
+
+    ts = [threading.Thread(target=applies, args=(i,)) for i in range(2)]
+    ts.append(threading.Thread(target=solves))
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    go.close()
