@@ -265,7 +265,11 @@ def _on_current_stream(method):
         if kw or any(isinstance(a, np.ndarray) for a in args):
             return ordered(self, *args, **kw)
         lib = load()
-        _check(lib.pdg_run_on(go._h, torch.cuda.current_stream(go.cfg.device).cuda_stream))
+        st = lib.pdg_run_on(go._h, torch.cuda.current_stream(go.cfg.device).cuda_stream)
+        if st == PDG_ESTATE:
+            # a stream was bound by a C call: ordered against it with events
+            return ordered(self, *args)
+        _check(st)
         # other threads wait in pdg_run_on until pdg_run_done
         go._running = threading.get_ident()
         try:

@@ -85,6 +85,46 @@ def test_each_thread_runs_on_its_own_stream(monkeypatch):
     assert go._running is None
 
 
+def test_stream_bound_by_a_c_call(monkeypatch):
+    """pdg_run_on refuses while a stream is bound; a binding that did not bind it
+    itself orders against that stream with events, as every other call does."""
+    import pdg
+    log = []
+
+    class Stream:
+        def __init__(self, name):
+            self.name, self.cuda_stream = name, 7
+
+        def wait_stream(self, other):
+            log.append(f"{self.name} waits {other.name}")
+
+    def get_stream(h, out):
+        out._obj.value = 0x1000
+        return pdg.PDG_OK
+
+    lib = types.SimpleNamespace(pdg_run_on=lambda h, s: pdg.PDG_ESTATE, pdg_get_stream=get_stream)
+    monkeypatch.setattr(pdg, "load", lambda *a: lib)
+    cuda = types.SimpleNamespace(is_initialized=lambda: True,
+                                 ExternalStream=lambda ptr, device=None: Stream("bound"),
+                                 current_stream=lambda device=None: Stream("torch"))
+    monkeypatch.setitem(sys.modules, "torch",
+                        types.SimpleNamespace(cuda=cuda, device=lambda *a: a))
+    go = types.SimpleNamespace(_h=ctypes.c_void_p(1), _explicit_stream=False, _lib_stream=None,
+                               _running=None, cfg=types.SimpleNamespace(device=0))
+
+    class Op:
+        def __init__(self):
+            self.go = go
+
+        @pdg._on_current_stream
+        def apply(self):
+            log.append("call")
+            return 7
+
+    assert Op().apply() == 7
+    assert log == ["bound waits torch", "call", "torch waits bound"]
+
+
 @pytest.mark.gpu
 def test_threads_on_one_operator():
     """Applies of two threads behind writes on their own streams, beside a third
