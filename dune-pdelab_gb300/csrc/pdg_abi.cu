@@ -250,7 +250,7 @@ static int ensure_r0(pdg_context *ctx) {
       PDG_CUDA_TRY(cudaMemcpyAsync(ctx->r0, ctx->legw64[0], sizeof(double) * ctx->ndof,
                                    cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    ctx->r0_valid = 1;
+    mark_built(ctx, &ctx->r0_valid);
   }
   return PDG_OK;
 }
@@ -965,12 +965,9 @@ static void invalidate(pdg_context *ctx, bool operator_changed) {
   }
 }
 
-}  // namespace pdg
-
-using namespace pdg;
-
-// in capture: events recorded outside cannot be waited for, nor the other way round
-static bool capturing(cudaStream_t s) {
+// (events recorded outside a capture cannot be waited for inside, nor the other
+// way round)
+bool in_capture(cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
     cudaGetLastError();   // the legacy stream beside a capture elsewhere
@@ -978,6 +975,11 @@ static bool capturing(cudaStream_t s) {
   }
   return cs != cudaStreamCaptureStatusNone;
 }
+
+}  // namespace pdg
+
+using namespace pdg;
+
 static int mark(cudaEvent_t *ev, cudaStream_t s) {
   if (!*ev) PDG_CUDA_TRY(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
   PDG_CUDA_TRY(cudaEventRecord(*ev, s));
@@ -999,7 +1001,7 @@ struct CtxCall {
   CtxCall(const CtxCall &) = delete;
   ~CtxCall() {
     if (status == PDG_OK && !ctx->run_active && ctx->stream != ctx->own_stream &&
-        !capturing(ctx->stream))
+        !in_capture(ctx->stream))
       mark(&ctx->ev_bound, ctx->stream);
   }
 
@@ -1008,7 +1010,7 @@ struct CtxCall {
     PDG_CUDA_TRY(cudaSetDevice(ctx->device));
     if (ctx->run_active || ctx->stream != ctx->own_stream) return PDG_OK;
     ctx->own_dirty = 1;
-    if (!ctx->own_must_wait || capturing(ctx->stream)) return PDG_OK;
+    if (!ctx->own_must_wait || in_capture(ctx->stream)) return PDG_OK;
     ctx->own_must_wait = 0;
     PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->ev_run, 0));
     return PDG_OK;
@@ -1339,10 +1341,10 @@ int pdg_set_stream(pdg_context *ctx, void *stream) {
   const cudaStream_t s = stream ? (cudaStream_t)stream : ctx->own_stream, old = ctx->stream;
   if (s == old) return PDG_OK;
   // the new stream follows what ran on the others
-  if (!capturing(s)) {
+  if (!in_capture(s)) {
     if (ctx->run_pending) PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_run, 0));
     if (ctx->ev_bound) PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_bound, 0));
-    if (old == ctx->own_stream && ctx->own_dirty && !capturing(old)) {
+    if (old == ctx->own_stream && ctx->own_dirty && !in_capture(old)) {
       PDG_TRY(mark(&ctx->ev_own, old));
       PDG_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_own, 0));
     }

@@ -569,7 +569,7 @@ static int ensure_record32(pdg_context *ctx) {
     case 5: st = record32_n<5>(ctx); break;
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
   }
-  if (st == PDG_OK) ctx->rec32_valid = 1;
+  if (st == PDG_OK) mark_built(ctx, &ctx->rec32_valid);
   return st;
 }
 
@@ -588,7 +588,7 @@ static int ensure_record(pdg_context *ctx) {
     case 34: st = record_dn<3, 5>(ctx); break;
     default: return set_error(PDG_EUNSUPPORTED, "dim/degree not compiled in");
   }
-  if (st == PDG_OK) ctx->rec_valid = 1;
+  if (st == PDG_OK) mark_built(ctx, &ctx->rec_valid);
   return st;
 }
 

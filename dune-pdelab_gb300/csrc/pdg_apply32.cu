@@ -1172,7 +1172,7 @@ static int launch32_q3(pdg_context *ctx, const ApplyArgs<float> &a, const OpPara
         k_record_q3t<<<(unsigned)((ctx->ncell + 127) / 128), 128, 0, ctx->stream>>>(p, rec,
                                                                                    ctx->rec32q);
         PDG_CUDA_TRY(cudaGetLastError());
-        ctx->rec32q_valid = 1;
+        mark_built(ctx, &ctx->rec32q_valid);
       }
       static int attr_t = -1, sms = 0;
       if (attr_t != ctx->device) {

@@ -416,7 +416,7 @@ static int ensure_pairs(pdg_context *ctx, long rec_doubles) {
   k_to_pairs<<<(unsigned)((rec_doubles + 255) / 256), 256, 0, ctx->stream>>>(
       rec_doubles, ctx->rec64, (fpair *)ctx->recfp);
   PDG_CUDA_TRY(cudaGetLastError());
-  ctx->recfp_valid = 1;
+  mark_built(ctx, &ctx->recfp_valid);
   return PDG_OK;
 }
 

@@ -535,7 +535,7 @@ static int record_i_n(pdg_context *ctx, const OpParams<double> &p, int transpose
 int prepare_apply_i(pdg_context *ctx, int transpose) {
   int &valid = transpose ? ctx->reciT_valid : ctx->reci_valid;
   if (valid) return PDG_OK;
-  if (!ctx->rec_valid) return set_error(PDG_EINVAL, "limb records need the FP64 records");
+  if (!ctx->rec64) return set_error(PDG_EINVAL, "limb records need the FP64 records");
   const OpParams<double> p = make_params<double>(ctx, ctx->K64, ctx->c64, ctx->tab64);
   int st;
   switch (ctx->N) {
@@ -545,7 +545,7 @@ int prepare_apply_i(pdg_context *ctx, int transpose) {
     case 5: st = record_i_n<5>(ctx, p, transpose); break;
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
   }
-  if (st == PDG_OK) valid = 1;
+  if (st == PDG_OK) mark_built(ctx, &valid);
   return st;
 }
 

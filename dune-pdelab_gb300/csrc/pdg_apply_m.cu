@@ -255,7 +255,7 @@ static int record_m_n(pdg_context *ctx, int transpose) {
 int prepare_apply_m(pdg_context *ctx, int transpose) {
   int &valid = transpose ? ctx->rec64mT_valid : ctx->rec64m_valid;
   if (valid) return PDG_OK;
-  if (!ctx->rec_valid || !ctx->tabm64)
+  if (!ctx->rec64 || !ctx->tabm64)
     return set_error(PDG_EINVAL, "mass-factored records need the FP64 records and tables");
   int st;
   switch (ctx->N) {
@@ -263,7 +263,7 @@ int prepare_apply_m(pdg_context *ctx, int transpose) {
     case 5: st = record_m_n<5>(ctx, transpose); break;
     default: return set_error(PDG_EUNSUPPORTED, "degree not compiled in");
   }
-  if (st == PDG_OK) valid = 1;
+  if (st == PDG_OK) mark_built(ctx, &valid);
   return st;
 }
 

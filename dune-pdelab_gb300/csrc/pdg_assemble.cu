@@ -231,7 +231,7 @@ int assemble_jacobian(pdg_context *ctx) {
     }
   ctx->use_matrix = use;
   PDG_CUDA_TRY(cudaGetLastError());
-  ctx->A_valid = 1;
+  mark_built(ctx, &ctx->A_valid);
   return PDG_OK;
 }
 

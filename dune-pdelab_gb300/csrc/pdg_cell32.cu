@@ -554,7 +554,7 @@ static int launch_apply32_cell_n(pdg_context *ctx, const ApplyArgs<float> &a,
     const OpParams<double> pd = make_params<double>(ctx, ctx->K64, ctx->c64, ctx->tab64);
     k_record_c32<N><<<(unsigned)((ctx->ncell + 127) / 128), 128, 0, ctx->stream>>>(pd, ctx->rec32c);
     PDG_CUDA_TRY(cudaGetLastError());
-    ctx->rec32c_valid = 1;
+    mark_built(ctx, &ctx->rec32c_valid);
   }
   C32Tab<N> tb;
   for (int i = 0; i < C::N2; i++) {

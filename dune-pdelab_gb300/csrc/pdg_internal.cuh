@@ -301,6 +301,13 @@ struct pdg_context {
 
 namespace pdg {
 
+// whether work on the stream goes into a graph instead of running
+bool in_capture(cudaStream_t s);
+// Data that launches on the context's stream build on first use is there for later
+// calls once they have been queued; under capture they run with each replay only,
+// and calls outside the graph build the data themselves.
+inline void mark_built(const pdg_context *ctx, int *valid) { *valid = !in_capture(ctx->stream); }
+
 constexpr int kRedBlocks = 1024;   // partials per reduction (grid size cap)
 
 // kernels / launchers implemented in the .cu files

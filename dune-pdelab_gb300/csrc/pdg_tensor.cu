@@ -824,7 +824,7 @@ int prepare_apply_tensor(pdg_context *ctx) {
   if (ctx->rect_valid) return PDG_OK;
   PDG_TRY(ctx->N == 2 ? record_tensor_n<2>(ctx)
                       : ctx->N == 3 ? record_tensor_n<3>(ctx) : record_tensor_n<4>(ctx));
-  ctx->rect_valid = 1;
+  mark_built(ctx, &ctx->rect_valid);
   return PDG_OK;
 }
 
