@@ -84,6 +84,18 @@ __device__ __forceinline__ unsigned long long fix_mag(double x, int eb) {
       ((unsigned long long)__funnelshift_l(lo, mh, F - 53) << 32) | (unsigned)(lo << (F - 53));
   return t >> sh;
 }
+// x rounded to units of 2^(E - 57), E = eb - 1022 (x finite, biased exponent at
+// most eb, eb >= 64; halves away from zero, zeros and subnormals give 0)
+__device__ __forceinline__ long long fix_round(double x, int eb) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int sh = min(eb - (int)((hi >> 20) & 0x7ffu), 63);
+  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+  const unsigned long long t =
+      ((unsigned long long)__funnelshift_l(lo, mh, kFixBits - 53) << 32) |
+      (unsigned)(lo << (kFixBits - 53));
+  const long long r = (long long)((t + ((1ull << sh) >> 1)) >> sh);
+  return (int)hi < 0 ? -r : r;
+}
 // The operators compute a cell with the sign of its first value taken out of all
 // its data (flip: 0 or -1, sign_flip of that value): rounding then sees the same
 // integers for x and -x, so J(-x) = -J(x) to the bit, as in FP64.

@@ -161,28 +161,48 @@ __device__ inline void run_finisher(const RedCtx &rc, int fin, int slot0, int sl
 // its own output with the other operand per block.  Same determinism as the
 // dot kernels: block partials in a per-kernel array, the last block adds
 // them in block order and runs the finisher.  Blocks of any size <= MAXT.
+
+// sum over the lanes of the mask of integers below 2^58
+__device__ __forceinline__ long long warp_sum_i64(unsigned mask, long long x) {
+  const unsigned s0 = __reduce_add_sync(mask, (unsigned)x & 0x7ffffffu);
+  const unsigned s1 = __reduce_add_sync(mask, (unsigned)(x >> 27) & 0x7ffffffu);
+  const int s2 = __reduce_add_sync(mask, (int)(x >> 54));
+  return (long long)(((unsigned long long)(unsigned)s2 << 54) + ((unsigned long long)s1 << 27) +
+                     s0);
+}
+
+// sum of the lanes' values rounded to 57 bits under the power of two above the
+// largest (biased exponent b; 128 or more, or all zero), put together on the integer
+// pipe (the conversion of a 64-bit integer takes the FP64 pipe 400 cycles)
+__device__ __forceinline__ double warp_sum_scaled(unsigned mask, double v, int b) {
+  const int eb = max(b, kFixMinBiased);
+  return fix_to_double(warp_sum_i64(mask, fix_round(v, eb)), eb - 1022 - kFixBits);
+}
+// (a call: unrolled in line it costs the kernels' instruction cache)
+static __device__ __noinline__ double warp_sum_rare(unsigned mask, double v, int n, int b) {
+  if (b != 0x7ff) {   // so small that the unit would be subnormal
+    v *= 0x1p512;
+    b = (int)(__reduce_max_sync(mask, (unsigned)__double2hiint(v) << 1) >> 21);
+    return warp_sum_scaled(mask, v, b) * 0x1p-512;
+  }
+  double s = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < n; i++) s += __shfl_sync(mask, v, i);
+  return s;
+}
 // Sum over the first n lanes of a warp (all of which call it; the others do not
 // exist), in every one of them, in 57-bit fixed point: a tree of FP64 additions
-// takes five steps of about 105 cycles, this about 250 in all.  Values that are
-// not finite, or so small that the fixed point would lose them, are added in
-// FP64.  The result does not depend on the order of the lanes.
+// takes five steps of about 105 cycles, this about 250 in all.  Every lane is
+// rounded to 2^-57 of the power of two above the largest, so a warp is off by at
+// most 2^-53 of that, and not to one side (lanes cut toward zero made sums of one
+// sign too small).  Values that are not finite are added in FP64.  The result does
+// not depend on the order of the lanes.
 __device__ __forceinline__ double warp_sum_fixed(double v, int n) {
   const unsigned mask = n >= 32 ? 0xffffffffu : (1u << n) - 1u;
   const unsigned m = __reduce_max_sync(mask, (unsigned)__double2hiint(v) << 1);
   const int b = (int)(m >> 21);
-  if (b == 0x7ff || (b < 128 && m != 0)) {
-    double s = 0.0;
-    for (int i = 0; i < n; i++) s += __shfl_sync(mask, v, i);
-    return s;
-  }
-  const int eb = max(b, kFixMinBiased);
-  const long long x = fix_signed(v, eb);
-  const unsigned s0 = __reduce_add_sync(mask, (unsigned)x & 0x7ffffffu);
-  const unsigned s1 = __reduce_add_sync(mask, (unsigned)(x >> 27) & 0x7ffffffu);
-  const int s2 = __reduce_add_sync(mask, (int)(x >> 54));
-  const long long s = (long long)(((unsigned long long)(unsigned)s2 << 54) +
-                                  ((unsigned long long)s1 << 27) + s0);
-  return (double)s * __hiloint2double((eb - 56) << 20, 0);   // units of 2^(E - 57)
+  if (b == 0x7ff || (b < 128 && m != 0)) return warp_sum_rare(mask, v, n, b);
+  return warp_sum_scaled(mask, v, b);
 }
 
 // Block sums of two values (the second only if `two`): warp sums in sw (at
