@@ -23,9 +23,8 @@
 // Runs of 64 cells: 32 and 128 are slower on large or small grids (64^3
 // mixed CG 252, 252 and 281 ms, 32^3 gradient 69, 80 and 69 ms).
 //
-// Block sums of the fused dot products are formed in two-float arithmetic
-// (the FP64 pipe takes 17 cycles for one warp-wide addition, and a block sum
-// in FP64 needs about 18 of them).
+// A thread adds its part of the fused dot products in two-float arithmetic; the
+// sums over threads are in 57-bit fixed point and FP64 (reduce_tail_two_float).
 #include <algorithm>
 #include <cstdint>
 

@@ -304,9 +304,10 @@ __device__ __forceinline__ void reduce_tail_grouped(double *part, long max_block
   grouped_finish<MAXT>(part, max_blocks, cnt, rc, s0, fin);
 }
 
-// A sum carried as an unevaluated pair of floats (48 bits): block sums of FP32
-// kernels on the FP32 pipe.  GB300's FP64 pipe takes 17 cycles for one
-// warp-wide addition, a block sum in FP64 about 18 of them.
+// A thread's sum of FP32 values carried as an unevaluated pair of floats: a few
+// additions per thread on the FP32 pipe instead of the FP64 pipe's 17 cycles for each
+// warp-wide one.  (48 bits: enough for a handful of terms with 24, not for the sums
+// over threads, which warp_sum_two and FP64 do.)
 struct TwoFloat {
   float h, l;
 };
@@ -318,13 +319,50 @@ __device__ __forceinline__ TwoFloat two_add(TwoFloat a, TwoFloat b) {
   // a sum that is not finite stays what it is
   return TwoFloat{h, isfinite(h) ? __fsub_rn(e, __fsub_rn(h, s)) : 0.f};
 }
-__device__ __forceinline__ TwoFloat warp_sum_two(TwoFloat v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const TwoFloat w{__shfl_down_sync(0xffffffffu, v.h, o), __shfl_down_sync(0xffffffffu, v.l, o)};
-    v = two_add(v, w);
-  }
-  return v;
+// A float x below 2^(E + 1) as a multiple of 2^(E - 21): adding s = 1.5 2^(E + 2), whose
+// last place that is, rounds it there, and the sum's bits count it.  x becomes the
+// rest, exactly.
+__device__ __forceinline__ int take_chunk(float &x, float s) {
+  const float t = __fadd_rn(x, s);
+  x = __fsub_rn(x, __fsub_rn(t, s));
+  return __float_as_int(t) - __float_as_int(s);
+}
+// sum of the pairs of a whole warp, biased exponent eb of the largest high part in
+// 42..251: every pair as three integers of 22 bits, down to 2^-65 of the power of two
+// above the largest, summed without rounding; the result has 57 bits before its
+// own rounding
+__device__ __forceinline__ double warp_sum_chunks(TwoFloat v, int eb) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const auto magic = [&](int d) { return __int_as_float(((eb + 3 - d) << 23) | 0x400000); };
+  const int c1 = take_chunk(v.h, magic(0));
+  const float s2 = magic(22);
+  const int c2 = take_chunk(v.h, s2) + take_chunk(v.l, s2);
+  float rest = __fadd_rn(v.h, v.l);
+  const int c3 = take_chunk(rest, magic(44));
+  const long long n1 = __reduce_add_sync(kAll, c1), n2 = __reduce_add_sync(kAll, c2);
+  const int n3 = __reduce_add_sync(kAll, c3);
+  // units of 2^(E - 21), 2^(E - 43) and 2^(E - 65), E = eb - 126
+  return fix_to_double(n1 * (1ll << 36) + n2 * (1ll << 14) + ((n3 + 128) >> 8),
+                       eb - 126 - kFixBits);
+}
+// (a call: in line it costs the kernels' instruction cache)
+static __device__ __noinline__ double warp_sum_two_rare(TwoFloat v, int eb) {
+  constexpr unsigned kAll = 0xffffffffu;
+  if (eb == 0xff) return warp_sum_rare(kAll, (double)v.h + (double)v.l, 32, 0x7ff);
+  // to the middle of the range and back
+  const float up = eb < 42 ? 0x1p100f : 0x1p-8f;
+  const TwoFloat w{__fmul_rn(v.h, up), __fmul_rn(v.l, up)};
+  const int e = (int)(__reduce_max_sync(kAll, __float_as_uint(w.h) << 1) >> 24);
+  if (e == 0) return 0.0;
+  return warp_sum_chunks(w, e) * (eb < 42 ? 0x1p-100 : 0x1p8);
+}
+// Sum of the pairs of a whole warp, in every lane, as exact as warp_sum_fixed, and
+// with fewer instructions than a tree of additions of pairs.  Infinities and NaN are
+// added in FP64.
+__device__ __forceinline__ double warp_sum_two(TwoFloat v) {
+  const int eb = (int)(__reduce_max_sync(0xffffffffu, __float_as_uint(v.h) << 1) >> 24);
+  if (eb < 42 || eb > 251) return warp_sum_two_rare(v, eb);
+  return warp_sum_chunks(v, eb);
 }
 // reduce_tail_grouped with two-float sums of each thread (blocks of T threads,
 // T a multiple of 32)
@@ -332,21 +370,20 @@ template <int T>
 __device__ __forceinline__ void reduce_tail_two_float(double *part, long max_blocks, int *cnt,
                                                       const RedCtx &rc, TwoFloat s0, TwoFloat s1,
                                                       int fin) {
-  __shared__ TwoFloat w0[T / 32], w1[T / 32];
-  s0 = warp_sum_two(s0);
-  s1 = warp_sum_two(s1);
+  __shared__ double sw[2][T / 32];
+  const bool two = fin == FIN_CG_DEF_BETA;
+  const double a0 = warp_sum_two(s0), a1 = two ? warp_sum_two(s1) : 0.0;
   if ((threadIdx.x & 31) == 0) {
-    w0[threadIdx.x >> 5] = s0;
-    w1[threadIdx.x >> 5] = s1;
+    sw[0][threadIdx.x >> 5] = a0;
+    sw[1][threadIdx.x >> 5] = a1;
   }
   __syncthreads();
   // thread 0 adds the first values, thread 1 the second
   double a = 0.0;
   if (threadIdx.x < 2) {
-    TwoFloat v = threadIdx.x == 0 ? w0[0] : w1[0];
+    a = sw[threadIdx.x][0];
 #pragma unroll
-    for (int i = 1; i < T / 32; i++) v = two_add(v, threadIdx.x == 0 ? w0[i] : w1[i]);
-    a = (double)v.h + (double)v.l;
+    for (int i = 1; i < T / 32; i++) a += sw[threadIdx.x][i];
   }
   grouped_finish<T>(part, max_blocks, cnt, rc, a, fin);
 }

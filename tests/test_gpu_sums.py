@@ -23,6 +23,14 @@ __global__ void k_fixed(const double *v, int n, double *out) {
     out[blockIdx.x * n + threadIdx.x] = s;
   }
 }
+__global__ void k_two(const float *v, double *out) {
+  const int i = 32 * blockIdx.x + threadIdx.x;
+  out[i] = warp_sum_two(TwoFloat{v[2 * i], v[2 * i + 1]});
+}
+extern "C" int sum_two(const float *v, int rows, double *out) {
+  k_two<<<rows, 32>>>(v, out);
+  return (int)cudaDeviceSynchronize();
+}
 extern "C" int sum_fixed(const double *v, int rows, int n, double *out) {
   k_fixed<<<rows, n>>>(v, n, out);
   return (int)cudaDeviceSynchronize();
@@ -71,3 +79,34 @@ def test_warp_sum_fixed(lib, n):
         s, tol = bound(row) if row.any() else (0.0, 0.0)
         assert (o == o[0]).all()
         assert abs(o[0] - s) <= tol
+
+
+def test_warp_sum_two(lib):
+    """Pairs of floats: the sums over a warp keep what FP64 keeps of them."""
+    import torch
+    rng = np.random.default_rng(5)
+    rows = [rng.uniform(-1, 1, 32), rng.uniform(0, 1, 32), rng.uniform(0, 1, 32) ** 8,
+            rng.uniform(0, 1, 32) * 1e-30, np.zeros(32), np.ones(32),
+            rng.uniform(-1, 1, 32) * 10.0 ** rng.uniform(-8, 8, 32)]
+    h = np.array(rows).astype(np.float32)
+    low = (np.array(rows) - h.astype(np.float64)).astype(np.float32)
+    v = torch.tensor(np.stack([h, low], axis=2), device="cuda")
+    out = torch.zeros((len(rows), 32), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.sum_two(ctypes.c_void_p(v.data_ptr()), len(rows),
+                       ctypes.c_void_p(out.data_ptr())) == 0
+    for hr, lr, o in zip(h, low, out.cpu().numpy()):
+        both = [float(x) for x in hr] + [float(x) for x in lr]
+        s, tol = bound(both) if hr.any() else (0.0, 0.0)
+        assert (o == o[0]).all()
+        assert abs(o[0] - s) <= tol
+    special = np.zeros((3, 32, 2), np.float32)
+    special[0, 3, 0] = np.inf
+    special[1, 4, 0] = np.nan
+    special[2, :, 0] = 1e-44                     # subnormal in FP32
+    v = torch.tensor(special, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.sum_two(ctypes.c_void_p(v.data_ptr()), 3, ctypes.c_void_p(out.data_ptr())) == 0
+    o = out.cpu().numpy()
+    assert np.isposinf(o[0]).all() and np.isnan(o[1]).all()
+    assert (o[2] == float(np.float32(1e-44)) * 32).all()
