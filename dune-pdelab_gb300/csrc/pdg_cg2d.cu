@@ -32,6 +32,7 @@
 // threads of a block must cover all four quarters.  With one cell per thread
 // the 2D Q1 64^2 iteration took 19.5 us.
 #include <algorithm>
+#include <mutex>
 
 #include "pdg_ops.cuh"
 #include "pdg_tma.cuh"
@@ -371,25 +372,41 @@ static int cg2d_n(pdg_context *ctx, double *x, double *b, double *p, double *p2,
                   int maxit, bool *ran) {
   using C = CG2Cfg<N>;
   *ran = false;
-  static int dev = -1, sms = 0, coop = 0, smem_max = 0;
-  if (dev != ctx->device) {
-    PDG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    PDG_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-    PDG_CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin,
-                                        ctx->device));
-    cudaFuncAttributes fa;
-    PDG_CUDA_TRY(cudaFuncGetAttributes(&fa, k_cg2d<N>));
-    smem_max -= (int)fa.sharedSizeBytes;
-    PDG_CUDA_TRY(cudaFuncSetAttribute(k_cg2d<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem_max));
-    dev = ctx->device;
+  // the device's limits, shared by the contexts of all host threads
+  struct Limits {
+    int dev, sms, coop, smem;
+  };
+  static std::mutex mutex;
+  static Limits known{-1, 0, 0, 0};
+  Limits lim;
+  {
+    const std::lock_guard<std::mutex> lock(mutex);
+    if (known.dev != ctx->device) {
+      lim.dev = ctx->device;
+      PDG_CUDA_TRY(cudaDeviceGetAttribute(&lim.sms, cudaDevAttrMultiProcessorCount, lim.dev));
+      PDG_CUDA_TRY(cudaDeviceGetAttribute(&lim.coop, cudaDevAttrCooperativeLaunch, lim.dev));
+      PDG_CUDA_TRY(
+          cudaDeviceGetAttribute(&lim.smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, lim.dev));
+      cudaFuncAttributes fa;
+      PDG_CUDA_TRY(cudaFuncGetAttributes(&fa, k_cg2d<N>));
+      lim.smem -= (int)fa.sharedSizeBytes;
+      PDG_CUDA_TRY(cudaFuncSetAttribute(k_cg2d<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        lim.smem));
+      known = lim;
+    }
+    lim = known;
   }
-  if (!coop || sms < 1) return PDG_OK;
+  const int sms = lim.sms;
+  if (!lim.coop || sms < 1) return PDG_OK;
   const int grid = (int)std::min<long>(sms, ctx->ncell);
   const int cap = (int)((ctx->ncell + grid - 1) / grid);
   const size_t smem =
       sizeof(double) * ((size_t)C::PER_CELL * cap + C::TAB + 64 + 2 * (size_t)grid);
-  if (smem > (size_t)smem_max) return PDG_OK;   // the cells do not fit on the SMs
+  // A grid whose cells do not fit on the SMs keeps the launches.  One that fits is
+  // faster here at every size: us per iteration with three launches and in one, Q1
+  // 64^2 31 and 11, 128^2 36 and 17, 228^2 53 and 44; Q2 48^2 34 and 12, 166^2 59 and
+  // 44; Q3 110^2 53 and 32; Q4 90^2 64 and 40 (log-normal K).
+  if (smem > (size_t)lim.smem) return PDG_OK;
   const int npart = kCg2Sets * grid * 2, nslots = npart + kCg2Sets * kCg2Copies * 16;
   if (!ctx->cg2_slots)
     PDG_CUDA_TRY(cudaMalloc(&ctx->cg2_slots,

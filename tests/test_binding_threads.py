@@ -183,3 +183,40 @@ def test_threads_on_one_operator():
         t.join()
     assert not errors, errors
     go.close()
+
+
+@pytest.mark.gpu
+def test_threads_on_their_own_operators():
+    """Contexts are independent: 2D solves (one cooperative launch each) of two
+    threads, the first of their kind in both."""
+    import pdg
+    import torch
+    out, errors = [[], []], []
+    start = threading.Barrier(2)
+
+    def solves(i):
+        try:
+            go = pdg.GridOperator(2, 2, (24, 20 + i), alpha=3.0)
+            rng = np.random.default_rng(i)
+            go.set_permeability(np.exp(rng.standard_normal(go.ncell)))
+            go.set_source(fc=np.ones(go.ncell))
+            u = torch.zeros(go.ndof, dtype=torch.float64, device="cuda")
+            ls = pdg.ISTLBackend_SEQ_MatrixFree_Base(go)
+            slp = pdg.StationaryLinearProblemSolver(go, ls, u, 1e-8)
+            start.wait()
+            for _ in range(5):
+                u.zero_()
+                slp.apply()
+                out[i].append(u.cpu().numpy())
+            go.close()
+        except BaseException as e:
+            errors.append(e)
+
+    ts = [threading.Thread(target=solves, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    for o in out:
+        assert all(np.array_equal(v, o[0]) for v in o) and np.abs(o[0]).max() > 0
