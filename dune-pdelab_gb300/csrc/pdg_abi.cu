@@ -8,6 +8,8 @@
 //     matrixfree/gridoperatorpreconditioner.hh:45-84)
 // with dune-istl's CGSolver / BiCGSTABSolver recurrences (external to the
 // reference; restated from the published algorithms).
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -16,6 +18,7 @@
 #include <vector>
 
 #include "pdg_gmres.cuh"
+#include "pdg_hostmap.h"
 #include "pdg_internal.cuh"
 #include "pdg_vec.cuh"
 
@@ -1756,18 +1759,46 @@ static int pipe_slabs(const pdg_context *ctx, long *planes_per_slab) {
   return (int)((planes + pps - 1) / pps);
 }
 
-// the device's address of n doubles of pinned host memory, or null
+typedef CUresult (*PointerAttributesFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+static PointerAttributesFn pointer_attributes() {
+  static PointerAttributesFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault,
+                                         &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PointerAttributesFn>(f);
+    cudaGetLastError();
+  });
+  return fn;
+}
+
+// the device's address of n doubles of pinned host memory in one registered range
+// that it may write, or null
 static double *mapped_host(const double *p, size_t n) {
-  cudaPointerAttributes a, b;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-      cudaPointerGetAttributes(&b, p + (n - 1)) != cudaSuccess) {
+  cudaPointerAttributes a;
+  unsigned flags = 0;
+  const PointerAttributesFn fn = pointer_attributes();
+  if (!fn || cudaPointerGetAttributes(&a, p) != cudaSuccess || a.type != cudaMemoryTypeHost ||
+      !a.devicePointer || cudaHostGetFlags(&flags, const_cast<double *>(p)) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
-      (double *)b.devicePointer != (double *)a.devicePointer + (n - 1))
-    return nullptr;
-  return (double *)a.devicePointer;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  unsigned access = 0;
+  CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                 CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                 CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+  void *data[] = {&start, &size, &access};
+  if (fn(3, which, data, (CUdeviceptr)a.devicePointer) != CUDA_SUCCESS) return nullptr;
+  const HostMapping m{true,
+                      access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE &&
+                          !(flags & cudaHostRegisterReadOnly),
+                      (uintptr_t)a.devicePointer, (uintptr_t)start, size};
+  return (double *)mapped_range(m, n * sizeof(double));
 }
 
 // y = (acc ? y : 0) + alpha J x + add with x and/or y in host memory;
