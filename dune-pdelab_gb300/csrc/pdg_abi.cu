@@ -825,6 +825,15 @@ static bool is_device_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+static bool is_pinned(const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
 template <typename T>
 struct Staged {
   T *dev;
@@ -1742,15 +1751,21 @@ static int pipe_ready(pdg_context *ctx) {
   return PDG_OK;
 }
 
-// number of slabs (1: no pipelining) and planes per slab.  A slab costs about
-// 4 us, the first copy and the last kernel overlap nothing: with time T of the
-// whole copy 4 n + T / n is least at n = sqrt(T / 4 us), about one per MB
-// under the root (64^3 Q2, 57 MB: 4, 5, 6, 7, 8, 16 slabs take 484, 475, 476,
-// 474, 488, 493 us).
-static int pipe_slabs(const pdg_context *ctx, long *planes_per_slab) {
+// Number of slabs (1: no pipelining) and planes per slab.  A slab costs about 4 us;
+// what does not overlap is a slab's share of the time T of the stages beside the
+// longest one: 4 n + T / n is least at n = sqrt(T / 4 us).  A result that the kernel
+// stores into host memory leaves the copy in and half of the kernel, about one per
+// MB under the root (64^3 Q2, 57 MB: 4, 5, 6, 7, 8, 16 slabs take 484, 475, 476, 474,
+// 488, 493 us).  One that is copied out into pinned memory leaves the copy in and the
+// copy out or the kernel, 2.5 per MB under the root (1000^2 Q2, 72 MB: 4, 6, 8, 10, 12,
+// 16 slabs 724, 663, 640, 615, 609, 642 us; 400^2 Q4, 32 MB: 4, 5, 7, 10, 16 slabs 379,
+// 370, 342, 335, 389; 256 x 200 Q2, 3.7 MB: 1, 2, 3, 4, 8 slabs 96, 78, 73, 71, 85).
+// Copies of pageable memory hardly overlap, and each slab costs more: one per MB
+// under the root there too (256 x 200 Q2: 1, 2, 3 slabs 101, 133, 150 us).
+static int pipe_slabs(const pdg_context *ctx, bool copied_out, long *planes_per_slab) {
   const long planes = ctx->cfg.cells[ctx->dim - 1];
-  long s = std::min(ctx->ncell / kMinSlabCells,
-                    (long)std::sqrt(sizeof(double) * (double)ctx->ndof / 1e6));
+  const double mb = sizeof(double) * (double)ctx->ndof / 1e6;
+  long s = std::min(ctx->ncell / kMinSlabCells, (long)std::sqrt(copied_out ? 2.5 * mb : mb));
   if (s > kMaxSlabs) s = kMaxSlabs;
   if (s > planes) s = planes;
   if (s < 2) return 1;
@@ -1801,11 +1816,22 @@ static double *mapped_host(const double *p, size_t n) {
   return (double *)mapped_range(m, n * sizeof(double));
 }
 
+// the address under which the kernel may store into the host vector y, or null
+static double *store_target(const pdg_context *ctx, double *y) {
+  // k_apply_p stores runs of whole cells; the other kernels' stores of 32 to 200
+  // contiguous bytes are too short for the link (128^3 Q1 2045 against 985 us with
+  // copies, 32^3 Q4 398 against 347 us, 512^2 Q2 422 against 233 us)
+  const bool runs = ctx->N == 3 && apply_i_usable(ctx) && !ctx->f64_pair &&
+                    !general_coefficients(ctx) && !convection_on(ctx);
+  return runs ? mapped_host(y, ctx->ndof) : nullptr;
+}
+
 // y = (acc ? y : 0) + alpha J x + add with x and/or y in host memory;
-// xdev/ydev: the device copies (staging buffers for host vectors)
+// xdev/ydev: the device copies (staging buffers for host vectors), ydev = ymap: the
+// kernel stores into y itself
 static int apply_pipelined(pdg_context *ctx, const double *x, double *y, const double *xdev,
-                           double *ydev, bool hx, bool hy, const double *add, double alpha,
-                           int acc, int transpose, int nslab, long pps) {
+                           double *ydev, bool hx, bool hy, double *ymap, const double *add,
+                           double alpha, int acc, int transpose, int nslab, long pps) {
   PDG_TRY(pipe_ready(ctx));
   PDG_TRY(prepare_apply64(ctx, transpose));
   const long plane = ctx->ncell / ctx->cfg.cells[ctx->dim - 1];
@@ -1819,13 +1845,6 @@ static int apply_pipelined(pdg_context *ctx, const double *x, double *y, const d
   PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->pipe_d2h, ev_start, 0));
   PDG_CUDA_TRY(cudaStreamWaitEvent(ctx->pipe_k2, ev_start, 0));
   cudaStream_t const ctx_stream = ctx->stream;
-  // k_apply_p stores runs of whole cells; the other kernels' stores of 32 to 200
-  // contiguous bytes are too short for the link (128^3 Q1 2045 against 985 us with
-  // copies, 32^3 Q4 398 against 347 us, 512^2 Q2 422 against 233 us)
-  const bool runs = ctx->N == 3 && apply_i_usable(ctx) && !ctx->f64_pair &&
-                    !general_coefficients(ctx) && !convection_on(ctx);
-  double *const ymap = hy && !acc && runs ? mapped_host(y, ctx->ndof) : nullptr;
-  if (ymap) ydev = ymap;
   auto range = [&](int s, long *c0, long *c1) {
     *c0 = s * pps * plane;
     *c1 = std::min(ctx->ncell, (s + 1) * pps * plane);
@@ -1883,11 +1902,17 @@ static int apply_entry(pdg_context *ctx, const double *x, double *y, double alph
   const bool hx = !is_device_ptr(x), hy = !is_device_ptr(y);
   if (hx || hy) PDG_TRY(ensure_stage(ctx));
   long pps = 0;
-  const int nslab = (hx || hy) ? pipe_slabs(ctx, &pps) : 1;
+  int nslab = (hx || hy) ? pipe_slabs(ctx, true, &pps) : 1;   // the most it may be
   if (nslab > 1 && !ctx->use_matrix && !ctx->ops32 && ctx->nl_deg == 0 &&
-      ctx->basis != PDG_BASIS_LEGENDRE)
-    return apply_pipelined(ctx, x, y, hx ? ctx->stage_a : x, hy ? ctx->stage_b : y, hx, hy,
-                           with_r0 ? ctx->r0 : nullptr, alpha, acc, transpose, nslab, pps);
+      ctx->basis != PDG_BASIS_LEGENDRE) {
+    double *const ymap = hy && !acc ? store_target(ctx, y) : nullptr;
+    const bool copied_out = hy && !ymap && is_pinned(y) && (!hx || is_pinned(x));
+    if (!copied_out) nslab = pipe_slabs(ctx, false, &pps);
+    if (nslab > 1)
+      return apply_pipelined(ctx, x, y, hx ? ctx->stage_a : x,
+                             ymap ? ymap : hy ? ctx->stage_b : y, hx, hy, ymap,
+                             with_r0 ? ctx->r0 : nullptr, alpha, acc, transpose, nslab, pps);
+  }
   Staged<double> sx, sy;
   PDG_TRY(stage_in<double>(ctx, x, ctx->ndof, ctx->stage_a, true, &sx));
   PDG_TRY(stage_in<double>(ctx, y, ctx->ndof, ctx->stage_b, acc != 0, &sy));
