@@ -61,12 +61,7 @@ struct PCfg {
   static constexpr int OUTE = -61 + SHX + SHM + SHO;
 };
 
-// v * c for a small integer constant
-template <int c>
-__device__ __forceinline__ long long times(long long v) {
-  return v * c;
-}
-// a run-time one: two 32-bit products
+// v * c for a small integer: two 32-bit products
 __device__ __forceinline__ long long times(long long v, int c) {
   return (long long)((unsigned long long)v * (unsigned long long)(long long)c);
 }
