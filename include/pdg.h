@@ -43,7 +43,8 @@ enum {
   PDG_EUNSUPPORTED = 6,    /* configuration not compiled in / not supported */
   PDG_EOUTFLOW = 7,        /* outflow boundary on inflow (convectiondiffusiondg.hh:802-806) */
   PDG_ENONFINITE = 8,      /* NaN/Inf defect */
-  PDG_ETIMEOUT = 9,        /* a bounded device wait ran out */
+  PDG_ETIMEOUT = 9,        /* a bounded device wait ran out: in this call or in an
+                              asynchronous one since the last that waited */
   PDG_ELINESEARCH = 10     /* Newton line search failed (LineSearchError,
                               solver/linesearch.hh:134-154) */
 };
