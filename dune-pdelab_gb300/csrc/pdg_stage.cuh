@@ -2,13 +2,18 @@
 //
 // A run of source elements [g0, g0 + count) lands at dst[ph + i], ph = g0 mod
 // the elements of 16 bytes, so that source and destination share their 16-byte
-// phase (dst is 16-byte aligned and has room for whole 16-byte chunks).  Runs
-// inside [0, lim) of an aligned source are one bulk copy by thread 0, completing
-// on `bar` (per-thread copies of all runs cost the FP32 operator of
-// pdg_cell32.cu about 900 of its 3800 instructions per warp); runs that
-// straddle an end are copied element-wise with zeros outside, runs outside are
-// left out (an absent neighbour's values are not used).  All threads call it,
-// then wait().
+// phase (dst is 16-byte aligned and has room for whole 16-byte chunks).  Of an aligned
+// source the part inside [0, lim) is one bulk copy of whole chunks by thread 0,
+// completing on `bar` (per-thread copies of all runs cost the FP32 operator of
+// pdg_cell32.cu about 900 of its 3800 instructions per warp), and at most one chunk's
+// rest element-wise.  What lies outside is left as it is: an absent neighbour's values
+// and those of inactive cells are not used.  All threads call it, then wait().
+//
+// Runs that straddle an end go the same way: copied element-wise they are tens of
+// loads one after another, and the blocks at the ends of a grid of a few thousand
+// cells are its last ones (9x10x11 Q2, device time: FP32 block Jacobi 6.0 us that way,
+// 3.7 this, FP32 operator 7.8 and 5.2, FP64 operator 10.6 and 8.7; asynchronous copies
+// of the rest: 3.3, 5.0, 8.8, but 64^3 Q2 FP64 159 instead of 158 us).
 #pragma once
 
 #include "pdg_tma.cuh"
@@ -28,20 +33,28 @@ struct Stager {
     const long ga = g0 - ph;
     const int len = (ph + count + E - 1) & ~(E - 1);
     if (ga + len <= 0 || ga >= lim) return dst + ph;
-    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && ga >= 0 && ga + len <= lim) {
-      if (threadIdx.x == 0) {
-        // every copy is announced before it is issued; the phase completes
-        // with the arrival in wait()
-        mbar_announce_tx(bar, (unsigned)sizeof(V) * len);
-        bulk_load(smem_u32(dst), src + ga, (unsigned)sizeof(V) * len, bar);
-      }
-    } else {
-      for (int c = threadIdx.x; c < len; c += T) {
-        const long g = ga + c;
-        dst[c] = (g >= 0 && g < lim) ? src[g] : V(0);
-      }
+    const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+    if (aligned && ga >= 0 && ga + len <= lim) {
+      bulk(dst, src + ga, len);
+      return dst + ph;
     }
+    // the part inside [0, lim); ga is a multiple of E
+    const int b = ga < 0 ? (int)-ga : 0, e = lim - ga < len ? (int)(lim - ga) : len;
+    int c = b;
+    if (aligned) {
+      c = e & ~(E - 1);
+      if (c > b) bulk(dst + b, src + ga + b, c - b);
+      else c = b;
+    }
+    for (c += threadIdx.x; c < e; c += T) dst[c] = src[ga + c];
     return dst + ph;
+  }
+  // every copy is announced before it is issued; the phase completes with the
+  // arrival in wait()
+  __device__ __forceinline__ void bulk(V *dst, const V *src, int n) {
+    if (threadIdx.x != 0) return;
+    mbar_announce_tx(bar, (unsigned)sizeof(V) * n);
+    bulk_load(smem_u32(dst), src, (unsigned)sizeof(V) * n, bar);
   }
   // false: the copies did not arrive within the poll limit.  They may still be
   // in flight then, and a block must not leave its shared memory to the next one

@@ -56,7 +56,52 @@ MAIN = r"""
 #include "pdg_stage.cuh"
 alignas(16) static double src[64], dst[64];
 static unsigned long long bar;
-int main(int, char **argv) {
+// every run of a vector of 61 values, by T threads one after another: the values
+// inside arrive, nothing is read or written outside
+template <int T, typename V>
+static int runs() {
+  constexpr int E = 16 / (int)sizeof(V), kLim = 61, kMax = 40;
+  alignas(16) static V x[kLim + 2 * E], to[kMax + 4 * E];
+  lands_at = 1;
+  for (int shift = 0; shift < 2; shift++)          // aligned source or not
+    for (int g0 = -kMax - 3; g0 < kLim + 3; g0++)
+      for (int count = 1; count <= kMax - E; count += 3) {
+        for (int i = 0; i < kLim + 2 * E; i++) x[i] = V(-5);
+        const V *src = x + E + shift;
+        for (int i = 0; i < kLim; i++) x[E + shift + i] = V(i + 1);
+        for (V &v : to) v = V(-7);
+        V *run = nullptr;
+        arrived = false;
+        polls = 0;
+        for (threadIdx.x = T; threadIdx.x-- > 0;) {
+          pdg::Stager<T, V> st(&bar);
+          run = st.run(to + E, src, g0, kLim, count);
+        }
+        threadIdx.x = 0;
+        for (int i = 0; i < queued; i++) {
+          const V *s = (const V *)queue[i].src;
+          if ((uintptr_t)s % 16 || (uintptr_t)queue[i].dst % 16 || queue[i].n % 16 || s < src ||
+              s + queue[i].n / sizeof(V) > src + kLim)
+            return 1;
+        }
+        pdg::Stager<T, V> st(&bar);
+        if (!st.wait() || queued) return 2;
+        for (int i = 0; i < count; i++)
+          if (g0 + i >= 0 && g0 + i < kLim && run[i] != V(g0 + i + 1)) return 3;
+        const V *end = run + count + E - 1;      // whole chunks
+        for (V &v : to)
+          if ((&v < to + E || &v >= end) && v != V(-7)) return 4;
+        for (V &v : to)
+          if (v == V(-5)) return 5;
+      }
+  return 0;
+}
+int main(int argc, char **argv) {
+  if (argc < 2) {
+    const int bad = runs<4, float>() + 10 * runs<2, double>();
+    std::printf("%d\n", bad);
+    return bad;
+  }
   lands_at = std::atol(argv[1]);
   for (int i = 0; i < 64; i++) src[i] = i + 1;
   pdg::Stager<1, double> st(&bar);
@@ -95,3 +140,8 @@ def test_nothing_in_flight_after_a_wait(exe, lands_at, ok):
     r = subprocess.run([exe, str(lands_at)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
     assert [int(v) for v in r.stdout.split()] == [ok, 0, 0]
+
+
+def test_runs_that_straddle_the_ends(exe):
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
