@@ -29,8 +29,9 @@
 // 64^3 Q2 (7.1 M DOF): k_apply_i 204 us, this one 179 as first written, 153
 // with the record prefetched to the L2 cache, no FP64 and 96 registers, 145 with
 // the loops rolled, 161 with the last masses in two halves and the cells' signs
-// taken out (57 MB in, 57 MB out and 123 MB of records need 35 us).  What is
-// left is the integer work (issue slots 58 %, ALU 55 %, IMAD 52 % busy) at 18
+// taken out (57 MB in, 57 MB out and 123 MB of records need 35 us).  Accumulating
+// (y += J x) 162 us, 185 with loads and stores of y one value at a time.  What is
+// left is the integer work (issue slots 58 %, ALU 57 %, IMAD 50 % busy) at 18
 // warps per SM; 15 warps without any spill take 173 us.
 #include <cmath>
 
@@ -494,13 +495,23 @@ __global__ void __launch_bounds__(PCfg::THREADS, 6)
     if (a.dot_part)
       for (long g = g0 + threadIdx.x; g < g1; g += C::THREADS) part += a.x[g] * Os[g];
   } else {
-    for (long g = g0 + threadIdx.x; g < g1; g += C::THREADS) {
-      double v = a.alpha * Os[g];
-      if (a.accumulate) v += a.y[g];
-      if (a.add) v += a.add[g];
-      if (a.dot_part) part += a.x[g] * v;
-      a.y[g] = v;
-    }
+    // all loads of a thread before its first store, and no FP64 operation (64 cycles
+    // for a warp) that is not needed
+    constexpr int U = T * NB / C::THREADS;
+    static_assert(U * C::THREADS == T * NB, "one pass writes a group");
+    const long gt = g0 + threadIdx.x;
+    const auto each = [&](auto f) {
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (gt + u * C::THREADS < g1) f(u, gt + u * C::THREADS);
+    };
+    double v[U];
+    each([&](int u, long g) { v[u] = Os[g]; });
+    if (a.alpha != 1.0) each([&](int u, long) { v[u] *= a.alpha; });
+    if (a.accumulate) each([&](int u, long g) { v[u] += a.y[g]; });
+    if (a.add) each([&](int u, long g) { v[u] += a.add[g]; });
+    if (a.dot_part) each([&](int u, long g) { part += a.x[g] * v[u]; });
+    each([&](int u, long g) { a.y[g] = v[u]; });
   }
   if (a.dot_part)
     reduce_tail_grouped<C::THREADS>(a.dot_part, a.dot_max_blocks, a.dot_cnt,

@@ -124,11 +124,22 @@ __device__ __forceinline__ void cell_line(const C32Tab<N> &tb, float k, const fl
 }
 
 // write-back of a run staged in shared memory: element f(O[i], index), by the
-// threads i0, i0 + T, ..
+// threads i0, i0 + T, ..  f may load from y, so stores wait for the loads of nine
+// elements at a time instead of one (y += J x, 64^3 Q2: 56 -> 33 us, 5x4x3 Q2 13.6 ->
+// 6.6 us on the device)
 template <int T, class F>
 __device__ __forceinline__ void write_run(const float *O, float *y, long g0, int count, int i0,
                                           F f) {
-  for (int i = i0; i < count; i += T) y[g0 + i] = f(O[i], g0 + i);
+  constexpr int U = 9;
+  for (int b = i0; b < count; b += U * T) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (b + u * T < count) v[u] = f(O[b + u * T], g0 + b + u * T);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (b + u * T < count) y[g0 + b + u * T] = v[u];
+  }
 }
 // The same unchanged: O has the 16-byte phase of y + g0 (y aligned), whole
 // 16-byte chunks are one bulk store by thread i0 = 0, the ends go one by one.
