@@ -249,7 +249,7 @@ __device__ __noinline__ double apply_cells_fp64(const OpParams<double> &p,
 // the four the register count alone gives, 156 with the results put together on
 // the integer pipe, 163 with s2 in finer units.  Degree 2 has its own kernel
 // (k_apply_p); the exchanges through shared memory, 12 loads and stores per value
-// there, are what it avoids (204 -> 161 us at 64^3 Q2).  At degrees 3 and 4 a plane per thread is 16 or
+// there, are what it avoids (204 -> 160 us at 64^3 Q2).  At degrees 3 and 4 a plane per thread is 16 or
 // 25 values with 96-bit sums, which does not fit the registers.
 template <int N>
 __global__ void __launch_bounds__(ICfg<N>::THREADS, N == 5 ? 5 : N == 4 ? 12 : 6)

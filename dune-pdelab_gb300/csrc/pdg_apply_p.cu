@@ -28,7 +28,7 @@
 //
 // 64^3 Q2 (7.1 M DOF): k_apply_i 204 us, this one 179 as first written, 153
 // with the record prefetched to the L2 cache, no FP64 and 96 registers, 145 with
-// the loops rolled, 161 with the last masses in two halves and the cells' signs
+// the loops rolled, 160 with the last masses in two halves and the cells' signs
 // taken out (57 MB in, 57 MB out and 123 MB of records need 35 us).  Accumulating
 // (y += J x) 162 us, 185 with loads and stores of y one value at a time.  What is
 // left is the integer work (issue slots 58 %, ALU 57 %, IMAD 50 % busy) at 18
