@@ -1,5 +1,5 @@
 // pdg_hostmap.h -- whether a kernel may store straight into a host vector
-// (host code only, no CUDA: what the driver says about the address comes in).
+// (host code only: what CUDA says about the address comes in).
 #pragma once
 
 #include <cstddef>
